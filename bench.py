@@ -333,14 +333,16 @@ def run_ours(args):
             import torch.distributed as dist
             dist.barrier()
 
-    def tracer(prec, tally_mode=0):
+    def tracer(prec, tally_mode=0, plain=False):
+        # plain: the plain kernel, every ray against every surface (a pinned launch knob keeps
+        # the culled kernel out; the autotuner still chooses the shape)
         t = Tracer(precision=prec, key1=w.key1, device=local, rays_per_thread=args.rays_per_thread,
-                   tally_mode=tally_mode)
+                   tally_mode=tally_mode, table_mode=1 if plain else 0)
         t.set_scene(sc)
         return t, torch.cuda.ExternalStream(t.stream_handle, device=dev)
 
     # -- headline kernel: scene resident, per-step device time ------------
-    t, stream = tracer(headline, args.tally_mode)
+    t, stream = tracer(headline, args.tally_mode, plain=headline != PREC_MIXED)
     head_bv = plain_bv
     # launch shape (plain kernels) or kernel choice (mixed: small-scene vs batched) for these budgets
     t.trace_async(rays, head_bv)
@@ -423,7 +425,7 @@ def run_ours(args):
     # -- the plain kernel (reference method, bit-exact) on the same rays -----
     plain = None
     if headline != PREC_EXACT and not args.no_plain:
-        tp, sp = tracer(PREC_EXACT)
+        tp, sp = tracer(PREC_EXACT, plain=True)
         tp.trace_async(rays, plain_bv)  # the workload's budgets, which the autotuner then tunes for
         tp.read_results(None, None)
         plain_cfg = tp.autotune(plain_bv)  # the plain kernel at its best launch shape
@@ -436,7 +438,7 @@ def run_ours(args):
     # reference's native_* functions): no longer bit-exact, same method
     plain_fast = None
     if headline != PREC_FAST and not args.no_plain:
-        tp, sp = tracer(PREC_FAST)
+        tp, sp = tracer(PREC_FAST, plain=True)
         tp.trace_async(rays, plain_bv)
         tp.read_results(None, None)
         fast_cfg = tp.autotune(plain_bv)
@@ -597,7 +599,7 @@ def run_sweep(args):
     p_ms = {PREC_EXACT: 0.0, PREC_FAST: 0.0}
     for sc, r in zip(sub_scenes, sub_rays):
         for prec in p_ms:
-            with Tracer(precision=prec, device=local) as tp:
+            with Tracer(precision=prec, device=local, table_mode=1) as tp:  # the plain kernel
                 tp.set_scene(sc)
                 tp.trace(r)  # the budgets the autotuner tunes for
                 tp.autotune()

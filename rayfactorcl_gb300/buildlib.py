@@ -3,7 +3,7 @@
 Each CUDA translation unit is compiled for sm_103a only
 (``-gencode arch=compute_103a,code=sm_103a``), in parallel, then linked with
 the static CUDA runtime so the library needs nothing but the driver.
-``rf_kern_exact.cu`` is compiled with ``-fmad=false`` so that products and sums
+``rf_kern_exact.cu``, ``rf_culled_exact.cu`` and ``rf_culled_f64.cu`` are compiled with ``-fmad=false`` so that products and sums
 written separately in the source keep separate roundings (bit-exact mode).
 """
 from __future__ import annotations
@@ -28,12 +28,16 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = {
     "rf_kern_exact.cu": ["-fmad=false"],
     "rf_kern_fast.cu": [],
+    "rf_culled_exact.cu": ["-fmad=false"],
+    "rf_culled_f64.cu": ["-fmad=false"],
+    "rf_culled_fast.cu": [],
     "rf_kern_batched.cu": [],
     "rf_kern_post.cu": [],
     "rf_capi.cu": [],
+    "rf_bounds.cu": [],
     "rf_noalloc.cu": [],
 }
-HEADERS = ["rf_internal.h", "rf_device.cuh", "rf_trace_kernels.cuh", "rf_batched.cuh", "rf_mixed_small.cuh"]
+HEADERS = ["rf_internal.h", "rf_device.cuh", "rf_trace_kernels.cuh", "rf_batched.cuh", "rf_mixed_small.cuh", "rf_culled.cuh"]
 
 
 def nvcc() -> str:

@@ -104,6 +104,11 @@ struct rf_ctx {
     float eps = 1e-3f;  // the scene's self-hit threshold (cfg.eps, or scaled when negative)
     std::vector<rf_primitive> prims;
     DevBuf d_tab, d_emit, d_bvtab, d_bvinfo;
+    std::vector<rf_bounding_volume> bvs;
+    int cull = 0;   // the culled kernel's tables: 0 not made yet, 1 in d_cull, -1 of no use for this scene
+    DevBuf d_cull;  // hit records (n), then float4: spheres (n), cone words (2 n), ring slack (n), bounding
+                    // surfaces' spheres (nbv)
+    bool tuning = false;  // rf_autotune is timing the plain kernel's launch shapes
 
     // trace state
     DevBuf d_hits, d_seg, d_rays, d_F, d_rec, d_err, d_misc;
@@ -217,6 +222,23 @@ cudaError_t launch_arith(int arith, const LaunchCfg &lc, const TraceParams &p, c
     }
 }
 
+cudaError_t launch_culled_arith(int arith, const TraceParams &p, bool bv, bool rec, int sms, cudaStream_t st)
+{
+    switch (arith) {
+    case RF_PREC_EXACT: return launch_culled<MExact>(p, bv, rec, sms, st);
+    case RF_PREC_FP64: return launch_culled<MF64>(p, bv, rec, sms, st);
+    default: return launch_culled<MFast>(p, bv, rec, sms, st);
+    }
+}
+
+// Philox draws of per-emitter ray counts (4 rays each).
+int64_t total_draws(const int64_t *count, int n)
+{
+    int64_t d = 0;
+    for (int e = 0; e < n; ++e) d += (count[e] + 3) >> 2;
+    return d;
+}
+
 rf_status check_budgets(rf_ctx *c, const int64_t *rays, int n)
 {
     for (int e = 0; e < n; ++e) {
@@ -252,12 +274,76 @@ struct Plan {
     LaunchCfg lc;
     bool hist = false;
     bool stage = true;
+    int chunk_draws = 0;  // > 0: the culled kernel, with chunks of this many draws
+    int64_t chunk_gids() const { return chunk_draws > 0 ? chunk_draws : (int64_t)lc.block * lc.gpt; }
 };
 
+// The culled kernel (rf_culled.cuh) takes a trace when the scene's bounds leave
+// enough out, unless the caller pinned a launch shape of the plain kernel or the
+// autotuner is timing those.  Culled against plain, measured on scenes of the
+// benchmark's type mix, ms:
+//   surfaces: at 1e7 rays (FP64: 1e6)  EXACT 16: 0.41 / 0.60, 64: 0.71 / 1.88, 400: 3.2 / 9.9;
+//     FAST 16: 0.34 / 0.33, 24: 0.38 / 0.47, 64: 0.62 / 1.11; FP64 16: 0.89 / 2.10
+//     -> from 16 surfaces on, FAST from 24;
+//   rays: the sort's fixed cost, EXACT at 1e5 rays  64 surfaces: 0.065 / 0.056, 201: 0.15 / 0.19;
+//     at 3e5 rays 24: 0.044 / 0.040, 64: 0.071 / 0.085, FAST 64: 0.060 / 0.060, at 1e6 rays
+//     0.099 / 0.140 -> from 4e5 rays (FAST 1e6) or 128 surfaces (FAST 256) on, in FP64
+//     always (64 surfaces, 1e5 rays: 0.58 / 1.01);
+//   a few hundred rays per emitter leave most threads of a plain chunk idle: 1e4 rays,
+//     64 surfaces EXACT 0.033 / 0.056, FAST 0.029 / 0.032.
+// The tables are made for the first trace that takes this kernel (about 40 us at 64
+// surfaces), not in rf_set_scene, where a scene traced otherwise would pay for them.
+bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
+{
+    const rf_config &f = c->cfg;
+    if (f.precision == RF_PREC_MIXED || c->tuning || f.block_size || f.rays_per_thread || f.tally_mode || f.table_mode ||
+        f.test_order)
+        return false;
+    if (bv && (c->n > kBatchTile || c->nbv > kBatchMaxBV)) return false;
+    const int n = c->n;
+    const int64_t rays = 4 * draws;
+    if (f.precision == RF_PREC_FP64) return n >= 16;
+    if (f.precision == RF_PREC_FAST) return n >= 256 || (n >= 24 && rays >= 1000000) || (n >= 64 && rays <= 200 * n);
+    return n >= 128 || (n >= 16 && rays >= 400000) || (n >= 24 && rays <= 400 * n);
+}
+
+rf_status ensure_culled(rf_ctx *c)
+{
+    const size_t n = c->n, words = 8 * n + c->nbv;  // float4
+    std::vector<float4> buf(words);
+    HitRec *tab = reinterpret_cast<HitRec *>(buf.data());
+    for (size_t i = 0; i < n; ++i)
+        tab[i] = make_hitrec(c->prims[i].invm, c->prims[i].type, c->prims[i].util1, c->prims[i].util2);
+    float4 *q = buf.data() + 4 * n;
+    const bool ok = cull_tables(c->prims.data(), c->n, c->bvs.data(), c->nbv, c->cfg.split_stacks == 0, tab, q, q + n,
+                                q + 3 * n, q + 4 * n);
+    if (ok) {
+        RF_CUDA(c, cudaStreamSynchronize(c->stream));
+        RF_CUDA(c, c->d_cull.ensure(words * sizeof(float4)));
+        RF_CUDA(c, cudaMemcpyAsync(c->d_cull.p, buf.data(), words * sizeof(float4), cudaMemcpyHostToDevice, c->stream));
+        RF_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
+    c->cull = ok ? 1 : -1;
+    return RF_OK;
+}
+
+// Draws per chunk of the culled kernel: about four chunks per SM, so that the last
+// ones end together, within what a block's shared memory holds and what its
+// threads need (64 surfaces EXACT, ms at 1024 / 2048 / 4096 / 8192 draws: 1e8 rays
+// 8.2 / 7.0 / 6.3 / 5.9, 1e7 rays 0.86 / 0.76 / 0.71 / 0.73, 1e6 rays 0.127 / 0.124 /
+// 0.21 / 0.33: larger chunks sort into more similar packets).
+int culled_chunk(const rf_ctx *c, int64_t draws)
+{
+    const int64_t want = (draws / (4 * (int64_t)c->sms) + 255) / 256 * 256;
+    const int64_t least = c->cfg.precision == RF_PREC_FP64 ? 512 : 1024;  // one draw per thread
+    return (int)std::max(least, std::min<int64_t>(kBatchChunkDraws, want));
+}
+
 // Launch shape for the single-scene kernels.
-Plan make_plan(rf_ctx *c, bool bv, bool rec)
+Plan make_plan(const rf_ctx *c, bool bv, bool rec, int64_t draws)
 {
     Plan pl;
+    if (c->cull > 0 && culled_pays(c, bv, draws)) pl.chunk_draws = culled_chunk(c, draws);
     pl.lc.bv = bv;
     pl.lc.rec = rec;
     pl.lc.block = c->block > 0 ? c->block : (c->cfg.block_size > 0 ? c->cfg.block_size : kBlock);
@@ -298,7 +384,12 @@ rf_status run_trace(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
                     int32_t *d_rec, int64_t rec_base, bool zero_hits)
 {
     const int n = c->n;
-    if (zero_hits) RF_CUDA(c, cudaMemsetAsync(c->d_hits.p, 0, (size_t)n * n * 8, c->stream));
+    // the culled kernel's work queue follows the tallies
+    unsigned long long *queue = c->d_hits.as<unsigned long long>() + (size_t)n * n;
+    if (zero_hits)
+        RF_CUDA(c, cudaMemsetAsync(c->d_hits.p, 0, (size_t)n * n * 8 + 8, c->stream));
+    else if (pl.chunk_draws > 0)
+        RF_CUDA(c, cudaMemsetAsync(queue, 0, 8, c->stream));
     c->last_launches = 0;
     c->timed = false;
     if (seg.empty() || total_chunks == 0) return RF_OK;
@@ -325,6 +416,22 @@ rf_status run_trace(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
     p.use_smem_hist = pl.hist ? 1 : 0;
 
     const int arith = arith_of(c);
+    if (pl.chunk_draws > 0) {
+        p.queue = queue;
+        p.tab = c->d_cull.as<HitRec>();
+        p.bsph = c->d_cull.as<float4>() + 4 * (size_t)n;
+        p.cquad = p.bsph + n;
+        p.cstack = p.bsph + 3 * (size_t)n;
+        p.bvsph = p.bsph + 4 * (size_t)n;
+        p.chunk_draws = pl.chunk_draws;
+        p.use_smem_hist = n <= kBatchTile ? 1 : 0;
+        RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+        RF_CUDA(c, launch_culled_arith(arith, p, pl.lc.bv, pl.lc.rec, c->sms, c->stream));
+        RF_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+        c->last_launches = 1;
+        c->timed = true;
+        return RF_OK;
+    }
     int bps = blocks_per_sm(arith, pl.lc);
     if (bps <= 0) bps = 1;
     const int64_t wave = (int64_t)c->sms * bps;
@@ -1205,7 +1312,7 @@ void rf_destroy(rf_ctx *c)
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (DevBuf *b : {&c->d_tab, &c->d_emit, &c->d_bvtab, &c->d_bvinfo, &c->d_hits, &c->d_seg,
-                      &c->d_rays, &c->d_F, &c->d_rec, &c->d_err, &c->d_misc, &c->b_tab, &c->b_emit,
+                      &c->d_rays, &c->d_F, &c->d_rec, &c->d_cull, &c->d_err, &c->d_misc, &c->b_tab, &c->b_emit,
                       &c->b_bsph, &c->b_scenes, &c->b_hits, &c->b_rows, &c->b_counters, &c->b_patch,
                       &c->b_chain, &c->b_plane, &c->b_cone, &c->b_maskrows, &c->b_maskoff, &c->b_mask, &c->b_frame, &c->b_bvtab,
                       &c->b_bvinfo, &c->b_bvsph})
@@ -1257,7 +1364,7 @@ rf_status rf_set_scene(rf_ctx *c, const rf_primitive *prims, int32_t n, const rf
     RF_CUDA(c, c->d_emit.ensure(sizeof(rf_primitive) * n));
     RF_CUDA(c, c->d_bvtab.ensure(sizeof(HitRec) * bvtab.size()));
     RF_CUDA(c, c->d_bvinfo.ensure(sizeof(int4) * bvinfo.size()));
-    RF_CUDA(c, c->d_hits.ensure((size_t)n * n * 8));
+    RF_CUDA(c, c->d_hits.ensure((size_t)n * n * 8 + 8));
     RF_CUDA(c, cudaMemcpyAsync(c->d_tab.p, tab.data(), sizeof(HitRec) * n, cudaMemcpyHostToDevice, c->stream));
     RF_CUDA(c, cudaMemcpyAsync(c->d_emit.p, prims, sizeof(rf_primitive) * n, cudaMemcpyHostToDevice, c->stream));
     RF_CUDA(c, cudaMemcpyAsync(c->d_bvtab.p, bvtab.data(), sizeof(HitRec) * bvtab.size(),
@@ -1266,6 +1373,8 @@ rf_status rf_set_scene(rf_ctx *c, const rf_primitive *prims, int32_t n, const rf
                                cudaMemcpyHostToDevice, c->stream));
     RF_CUDA(c, cudaStreamSynchronize(c->stream));
     c->prims.assign(prims, prims + n);
+    c->bvs.assign(bvs, bvs + nbv);
+    c->cull = 0;
     c->n = n;
     c->nbv = nbv;
     c->have_results = false;
@@ -1358,11 +1467,12 @@ rf_status rf_trace_async(rf_ctx *c, const int64_t *rays, int32_t use_bv)
         c->have_results = true;
         return RF_OK;
     }
-    Plan pl = make_plan(c, use_bv != 0, false);
-    const int64_t chunk_gids = (int64_t)pl.lc.block * pl.lc.gpt;
+    const int64_t draws = total_draws(rays, c->n);
+    if (c->cull == 0 && culled_pays(c, use_bv != 0, draws) && (s = ensure_culled(c)) != RF_OK) return s;
+    Plan pl = make_plan(c, use_bv != 0, false, draws);
     std::vector<Segment> seg;
     int64_t chunks = 0;
-    for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, 0, rays[e], chunk_gids, chunks);
+    for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, 0, rays[e], pl.chunk_gids(), chunks);
     if ((s = run_trace(c, seg, chunks, pl, nullptr, 0, true)) != RF_OK) return s;
     c->have_results = true;
     return RF_OK;
@@ -1391,8 +1501,10 @@ rf_status rf_trace_range(rf_ctx *c, const int64_t *first_ray, const int64_t *cou
     std::vector<Segment> seg;
     int64_t chunks = 0;
     const bool mixed = c->cfg.precision == RF_PREC_MIXED;
-    Plan pl = make_plan(c, use_bv != 0, false);
-    const int64_t chunk_gids = mixed ? mixed_chunk_draws(c, false, use_bv != 0) : (int64_t)pl.lc.block * pl.lc.gpt;
+    const int64_t draws = total_draws(count, c->n);
+    if (c->cull == 0 && culled_pays(c, use_bv != 0, draws) && (s = ensure_culled(c)) != RF_OK) return s;
+    Plan pl = make_plan(c, use_bv != 0, false, draws);
+    const int64_t chunk_gids = mixed ? mixed_chunk_draws(c, false, use_bv != 0) : pl.chunk_gids();
     for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, first_ray[e], count[e], chunk_gids, chunks);
     if (!accumulate) c->last_rays.assign(c->n, 0);
     for (int e = 0; e < c->n; ++e) c->last_rays[e] += count[e];
@@ -1515,10 +1627,11 @@ rf_status rf_trace_rays(rf_ctx *c, int32_t emitter, int64_t first_ray, int64_t n
         if ((s = run_mixed(c, seg, chunks, true, c->d_rec.as<int32_t>(), first_ray, false, use_bv != 0)) != RF_OK)
             return s;
     } else {
-        Plan pl = make_plan(c, use_bv != 0, true);
-        const int64_t chunk_gids = (int64_t)pl.lc.block * pl.lc.gpt;
+        const int64_t draws = (n_rays + 3) / 4;
+        if (c->cull == 0 && culled_pays(c, use_bv != 0, draws) && (s = ensure_culled(c)) != RF_OK) return s;
+        Plan pl = make_plan(c, use_bv != 0, true, draws);
         std::vector<Segment> seg;
-        const int64_t chunks = plan_segments(seg, emitter, 0, first_ray, n_rays, chunk_gids, 0);
+        const int64_t chunks = plan_segments(seg, emitter, 0, first_ray, n_rays, pl.chunk_gids(), 0);
         if ((s = run_trace(c, seg, chunks, pl, c->d_rec.as<int32_t>(), first_ray, false)) != RF_OK) return s;
     }
     RF_CUDA(c, cudaMemcpyAsync(out, c->d_rec.p, (size_t)n_rays * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -2142,6 +2255,11 @@ rf_status rf_autotune(rf_ctx *c, int32_t use_bv, const char *cache_path)
     const bool wide = !bv && c->cfg.precision != RF_PREC_FP64;
     double best_ms = 1e300;
     const TuneChoice saved{c->block, c->gpt, c->hist, c->stage, c->order};
+    struct Tuning {  // the trials are the plain kernel's
+        rf_ctx *c;
+        explicit Tuning(rf_ctx *x) : c(x) { c->tuning = true; }
+        ~Tuning() { c->tuning = false; }
+    } tuning(c);
     for (int block : {128, 256})
         for (int gpt : {1, 2}) {
             if (gpt == 2 && !wide) continue;

@@ -1,0 +1,653 @@
+// rf_culled.cuh -- nearest hits of one scene in the plain kernels' arithmetic
+// (MExact, MFast, MF64), with the surfaces a ray cannot hit left out.
+//
+// The plain kernel (rf_trace_kernels.cuh) tests every ray against every surface,
+// RayFactorGPU.cl:445-472.  Here a block sorts a chunk of one emitter's rays by
+// direction and emission patch, its warps take packets of 32 similar rays, and a
+// packet tests, in index order, the surfaces whose bounding sphere one of its
+// rays reaches, each with the plain kernel's own arithmetic.  A surface is left
+// out only when its test, rounding included, could not return a hit, so every
+// ray gets the plain kernel's nearest hit bit for bit, whatever packet it is in:
+//
+// * rf_capi.cu (cull_tables) bounds the points where a test can place a hit: the
+//   object-space shape grown by the test's rounding (for quadrics the
+//   cancellation in B^2 - AC, about 32 ulps of the largest squared object-space
+//   coordinate of the scene), as a world sphere grown again by this file's own
+//   FP32 rounding.  The bound of a cone fails for rays whose direction makes its
+//   A = c^T N c vanish; `band` lets those through (a frustum's sphere carries the
+//   sign bit in its radius as the mark).
+// * A ray with a non-finite or vanishing component is tested against everything,
+//   with the rest of its packet.
+// * Consecutive cylinders with one linear part that tile a longer cylinder (a
+//   furnace wall of rings) are first intersected as one, in FP32: the roots, with
+//   error bounds, name the one or two rings that a ring's own test could accept,
+//   and only those are tested, each lane its own.  Concentric annuli in one plane
+//   whose radii meet share one plane hit, exactly: the same operations give the
+//   same radius, and a binary search finds the member.
+//
+// What bounds it: FP32 issue, like the batched mixed-precision kernel whose
+// structure it shares; in MF64 the FP64 pipe.  64 surfaces, EXACT, 1e8 rays: 5.9 ms
+// (plain 18.2), of which draws, keys and sort 0.6, emission and packet bounds 1.3,
+// the spheres 2.2 (11 candidates per packet) and the tests 1.7 (5.3 per packet, of
+// which 2.4 find a hit for some ray; the plain kernel makes 64 per ray).  The
+// furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.15 ms EXACT
+// (plain 7.9), 1.0 FAST (5.7); 1e6 rays in FP64 2.2 (35.4).
+#pragma once
+
+#include "rf_trace_kernels.cuh"
+#include "rf_batched.cuh"
+
+namespace rf {
+
+// Shared memory of a block: arrays sized by the launch's chunk (cd draws), the
+// surfaces kept resident (nres, 0: read through L1), the histogram row (nhist,
+// 0: global tallies) and the bounding surfaces (nbv).
+struct CulledLayout {
+    int cnt, perm, unif, tab, bs, bvtab, bvinfo, bvbs, hist, bytes;
+    __host__ __device__ CulledLayout(int cd, int nres, int nhist, int nbv)
+    {
+        cnt = 0;
+        perm = cnt + kCells * 4;
+        unif = perm + cd * 8;
+        tab = unif + cd * 12;
+        bs = tab + nres * (int)sizeof(HitRec);
+        bvtab = bs + nres * 16;
+        bvinfo = bvtab + nbv * (int)sizeof(HitRec);
+        bvbs = bvinfo + nbv * 16;
+        hist = bvbs + nbv * 16;
+        bytes = hist + nhist * 4;
+    }
+};
+
+__device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz)
+{
+    return fmaf(ax, bx, fmaf(ay, by, az * bz));
+}
+
+__device__ __forceinline__ Ray<float> to_f32(const Ray<float> &r) { return r; }
+__device__ __forceinline__ Ray<float> to_f32(const Ray<double> &r)
+{
+    return Ray<float>{(float)r.sx, (float)r.sy, (float)r.sz, (float)r.cx, (float)r.cy, (float)r.cz};
+}
+
+__device__ __forceinline__ bool planar(int type) { return type == RF_DISC || type == RF_ANNULUS || type == RF_RECTANGLE; }
+
+// Sort key of a ray from its uniforms alone: an approximate direction (hardware
+// sin/cos, reciprocals) in the 256 octahedral cells above the 4 x 4 cell of the
+// two surface parameters.  Any key is correct; similar rays should share one.
+// f: a planar emitter's rotation (rows), set up once per emitter.
+__device__ __forceinline__ int quick_key(const rf_primitive &e, const float4 *f, const float r[4])
+{
+    float so, co;
+    MFast::sincos(r[2] * k2PiF, so, co);
+    const float st = MFast::sqrt(r[3]);
+    const float ox = st * co, oy = st * so, oz = MFast::sqrt(1.0f - r[3]);
+    float cx, cy, cz;
+    if (planar(e.type)) {
+        cx = dot3(f[0].x, f[0].y, f[0].z, ox, oy, oz);
+        cy = dot3(f[1].x, f[1].y, f[1].z, ox, oy, oz);
+        cz = dot3(f[2].x, f[2].y, f[2].z, ox, oy, oz);
+    } else {
+        float px, py, pz = 0.0f;
+        MFast::sincos((e.type == RF_CYLINDER ? r[0] : r[1]) * k2PiF, py, px);
+        if (e.type == RF_FRUSTUM) {
+            pz = 1.0f - e.util1;
+        } else if (e.type == RF_SPHERE) {
+            pz = fmaf(2.0f, r[0], -1.0f);
+            const float rho = MFast::sqrt(fmaf(-pz, pz, 1.0f));
+            px *= rho;
+            py *= rho;
+        }
+        float nx = dot3(e.invm[0], e.invm[4], e.invm[8], px, py, pz);
+        float ny = dot3(e.invm[1], e.invm[5], e.invm[9], px, py, pz);
+        float nz = dot3(e.invm[2], e.invm[6], e.invm[10], px, py, pz);
+        const float il = MFast::rsqrt(dot3(nx, ny, nz, nx, ny, nz)) * e.util2;
+        nx *= il;
+        ny *= il;
+        nz *= il;
+        const float d = MFast::rcp(fmaxf(1.0f + nz, 1e-6f));
+        const float k = d * fmaf(ny, ox, -nx * oy);
+        cx = fmaf(nz, ox, fmaf(ny, k, nx * oz));
+        cy = fmaf(nz, oy, fmaf(-nx, k, ny * oz));
+        cz = fmaf(nz, oz, -fmaf(nx, ox, ny * oy));
+    }
+    return (direction_cell(cx, cy, cz) << 4) | (min(3, (int)(r[0] * 4.0f)) << 2) | min(3, (int)(r[1] * 4.0f));
+}
+
+// Rotation rows of alignRayDirection (RayFactorGPU.cl:87-97) for a planar
+// emitter's normal, to the accuracy a sort key needs.
+__device__ __forceinline__ void quick_frame(const rf_primitive &e, float4 *f)
+{
+    float x = e.invm[8], y = e.invm[9], z = e.invm[10];
+    const float il = MFast::rsqrt(dot3(x, y, z, x, y, z));
+    x *= il;
+    y *= il;
+    z *= il;
+    const float d = MFast::rcp(fmaxf(1.0f + z, 1e-6f));
+    f[0] = make_float4(fmaf(d * y, y, z), -d * x * y, x, 0.0f);
+    f[1] = make_float4(-d * x * y, fmaf(d * x, x, z), y, 0.0f);
+    f[2] = make_float4(-x, -y, z, 0.0f);
+}
+
+// As ray_may_hit and packet_bounds / packet_may_hit of the batched kernel, with
+// every product and sum fused explicitly (two of the three translation units
+// are compiled with -fmad=false); |b.w| is the squared radius.
+__device__ __forceinline__ bool reaches(const Ray<float> &r, float idd, const float4 b)
+{
+    const float ox = b.x - r.sx, oy = b.y - r.sy, oz = b.z - r.sz;
+    const float oc2 = dot3(ox, oy, oz, ox, oy, oz);
+    const float bb = fmaxf(dot3(ox, oy, oz, r.cx, r.cy, r.cz), 0.0f);
+    return fmaf(-bb * bb, idd, oc2) <= fabsf(b.w);
+}
+
+__device__ __forceinline__ Packet bounds_of(const Ray<float> &r, float idd)
+{
+    Packet pk;
+    pk.ox = 0.5f * (warp_min(r.sx) + warp_max(r.sx));
+    pk.oy = 0.5f * (warp_min(r.sy) + warp_max(r.sy));
+    pk.oz = 0.5f * (warp_min(r.sz) + warp_max(r.sz));
+    const float dx = r.sx - pk.ox, dy = r.sy - pk.oy, dz = r.sz - pk.oz;
+    pk.rho = fmaf(MFast::sqrt(warp_max(dot3(dx, dy, dz, dx, dy, dz))), 1.0001f, 1e-30f);
+    const float il = MFast::sqrt(idd);
+    const float nx = r.cx * il, ny = r.cy * il, nz = r.cz * il;
+    const float ax = 0.5f * (warp_min(nx) + warp_max(nx));
+    const float ay = 0.5f * (warp_min(ny) + warp_max(ny));
+    const float az = 0.5f * (warp_min(nz) + warp_max(nz));
+    const float al2 = dot3(ax, ay, az, ax, ay, az);
+    const bool ok = al2 > 1e-6f;
+    const float ial = ok ? MFast::rsqrt(al2) : 0.0f;
+    pk.ax = ax * ial;
+    pk.ay = ay * ial;
+    pk.az = az * ial;
+    const float c = warp_min(dot3(nx, ny, nz, pk.ax, pk.ay, pk.az)) - 1e-4f;  // for rounding
+    pk.cull = ok && c > 0.0f;
+    pk.cos_t = c;
+    pk.sin_t = MFast::sqrt(fmaxf(0.0f, fmaf(-c, c, 1.0f))) * 1.0001f;
+    return pk;
+}
+
+__device__ __forceinline__ bool packet_reaches(const Packet &pk, const float4 b)
+{
+    const float vx = b.x - pk.ox, vy = b.y - pk.oy, vz = b.z - pk.oz;
+    const float L2 = dot3(vx, vy, vz, vx, vy, vz);
+    const float R = fmaf(MFast::sqrt(fabsf(b.w)), 1.0001f, pk.rho);
+    const float R2 = R * R;
+    const float va = dot3(vx, vy, vz, pk.ax, pk.ay, pk.az);
+    return !(L2 > R2) || va >= fmaf(pk.cos_t, MFast::sqrt(L2 - R2), -pk.sin_t * R);
+}
+
+// c^T N c of a cone's A for direction c, N in q0.xyz (diagonal) and q1.xyz
+// (yz, xz, xy, doubled).
+__device__ __forceinline__ float cone_A(const float4 q0, const float4 q1, float x, float y, float z)
+{
+    return fmaf(x, fmaf(q0.x, x, q1.z * y), fmaf(y, fmaf(q0.y, y, q1.x * z), z * fmaf(q0.z, z, q1.y * x)));
+}
+
+// A ray along which the frustum's A nearly vanishes (its roots then carry
+// unbounded rounding): q0.w is the threshold for a unit direction.
+__device__ __forceinline__ bool band(const float4 *quad, int j, const Ray<float> &r, float cc)
+{
+    const float4 q0 = __ldg(quad + 2 * j), q1 = __ldg(quad + 2 * j + 1);
+    return !(fabsf(cone_A(q0, q1, r.cx, r.cy, r.cz)) > q0.w * cc);
+}
+
+// The same for some direction of the packet's cone.  With c = a cos f + e sin f (a
+// the axis, e square to it, f up to the half-angle), c^T N c differs from
+// a^T N a cos^2 f by at most 2 sin f cos f |(N a) square to a| + sin^2 f |N|; q1.w = |N|.
+__device__ __forceinline__ bool packet_band(const float4 *quad, int j, const Packet &pk)
+{
+    const float4 q0 = __ldg(quad + 2 * j), q1 = __ldg(quad + 2 * j + 1);
+    const float nx = fmaf(q0.x, pk.ax, 0.5f * fmaf(q1.z, pk.ay, q1.y * pk.az));
+    const float ny = fmaf(q0.y, pk.ay, 0.5f * fmaf(q1.z, pk.ax, q1.x * pk.az));
+    const float nz = fmaf(q0.z, pk.az, 0.5f * fmaf(q1.y, pk.ax, q1.x * pk.ay));
+    const float A = dot3(nx, ny, nz, pk.ax, pk.ay, pk.az);
+    const float side = MFast::sqrt(fmaxf(0.0f, fmaf(-A, A, dot3(nx, ny, nz, nx, ny, nz))) + 1e-6f * q1.w * q1.w);
+    const float c2 = pk.cos_t * pk.cos_t;
+    return !(fabsf(A) * c2 > fmaf(2.0f * pk.sin_t, side, fmaf(pk.sin_t * pk.sin_t, q1.w, q0.w)));
+}
+
+// Nearest hit among the rings [a, a + m) of a cylinder stack: the tests of the
+// rings that the stack's own roots leave possible, each lane its own, with the
+// plain kernel's arithmetic.  In the first ring's frame every point that a ring's
+// test can accept has |x^2 + y^2 - 1| <= mg.x and z in its ring to within mg.y
+// (rf_bounds.cu: ring_stack), so t lies between (B -+ sqrt(D + A mg.x)) / A and
+// (B -+ sqrt(D - A mg.x)) / A; mg.z / sqrt(A) covers the rounding of these roots.
+// Such an interval names one or two rings; NaN and overflow widen it to all.
+template <class M>
+__device__ __forceinline__ void ring_hits(const HitRec *tab, bool resident, int a, int m, const float4 mg,
+                                          const Ray<typename M::T> &ray, const Ray<float> &w, typename M::T eps,
+                                          bool odd, typename M::T &tb, int &bi)
+{
+    using T = typename M::T;
+    int k1 = 0, e1 = m - 1, k2 = 0, e2 = -1;
+    if (!odd) {
+        const HitRec h = resident ? tab[a] : load_rec(tab, a);
+        const Ray<float> o = xfrm_ray<MFast>(h, w);
+        const float A = fmaf(o.cx, o.cx, o.cy * o.cy);
+        const float B = -fmaf(o.sx, o.cx, o.sy * o.cy);
+        const float wz = fmaf(o.sx, o.cy, -o.sy * o.cx);
+        const float D = fmaf(-wz, wz, A);
+        const float dk = A * mg.x;
+        const float ra = MFast::rcp(A), isa = MFast::rsqrt(A);
+        const float hi = MFast::sqrt(fmaxf(D + dk, 0.0f)), lo = MFast::sqrt(fmaxf(D - dk, 0.0f));
+        const float te = mg.z * isa, zs = fmaf(fabsf(o.cz), te, mg.y);
+        const float t1a = (B - hi) * ra, t1b = (B - lo) * ra, t2a = (B + lo) * ra, t2b = (B + hi) * ra;
+        const float z1a = fmaf(o.cz, t1a, o.sz), z1b = fmaf(o.cz, t1b, o.sz);
+        const float z2a = fmaf(o.cz, t2a, o.sz), z2b = fmaf(o.cz, t2b, o.sz);
+        const float feps = (float)eps, ftb = (float)tb, last = (float)(m - 1);
+        k1 = (int)fmaxf(0.0f, floorf(fminf(z1a, z1b) - zs));
+        e1 = (int)fminf(last, floorf(fmaxf(z1a, z1b) + zs));
+        k2 = (int)fmaxf(0.0f, floorf(fminf(z2a, z2b) - zs));
+        e2 = (int)fminf(last, floorf(fmaxf(z2a, z2b) + zs));
+        const float s1 = fmaf(8e-6f, fabsf(t1a) + fabsf(t1b), te), s2 = fmaf(8e-6f, fabsf(t2a) + fabsf(t2b), te);
+        const bool miss = D + dk < 0.0f;
+        if (miss || t1b + s1 < feps || t1a - s1 > ftb) e1 = -1;  // behind the threshold, or farther than a hit found
+        if (miss || t2b + s2 < feps || t2a - s2 > ftb) e2 = -1;
+        if (!(A > 0.0f) || !(te < 1e30f)) {
+            k1 = 0;
+            e1 = m - 1;
+            e2 = -1;
+        }
+    }
+    bool second = false;
+    for (;;) {
+        if (k1 > e1 && !second) {
+            k1 = k2;
+            e1 = e2;
+            second = true;
+        }
+        const bool have = k1 <= e1;
+        if (!__any_sync(0xffffffffu, have)) break;
+        if (have) {
+            const int j = a + k1;
+            const HitRec h = resident ? tab[j] : load_rec(tab, j);
+            const T t = cylinder_hit<M>(h, ray, eps);
+            if (t < tb || (t == tb && j < bi)) {  // the rings do not come in index order
+                tb = t;
+                bi = j;
+            }
+            ++k1;
+        }
+    }
+}
+
+// Nearest hit among the annuli [a, a + m) of a plate: one plane, one radius.
+template <class M>
+__device__ __forceinline__ void plate_hits(const HitRec &h, const HitRec *tab, bool resident, int a, int m,
+                                           const Ray<typename M::T> &w, typename M::T eps, typename M::T &tb, int &bi)
+{
+    using T = typename M::T;  // annulus_hit's operations
+    const Ray<T> o = xfrm_ray<M>(h, w);
+    const T th = -o.sz * M::rcp(o.cz);
+    const T hx = o.sx + o.cx * th;
+    const T hy = o.sy + o.cy * th;
+    const T e = M::fma(hx, hx, hy * hy);
+    auto util2 = [&](int k) { return T(resident ? tab[a + k].aux.z : __ldg(&tab[a + k].aux.z)); };
+    int base = 0, len = m;  // lowest k with util2_k >= e (uniform trip count)
+    while (len > 1) {
+        const int half = len >> 1;
+        base = util2(base + half - 1) < e ? base + half : base;
+        len -= half;
+    }
+    const T lo = T(resident ? tab[a].aux.y : __ldg(&tab[a].aux.y));
+    if (e >= lo && e <= util2(base) && th > eps && th < tb) {
+        tb = th;
+        bi = a + base;
+    }
+}
+
+// BV: runBVGPU's walk (RayFactorGPU.cl:530-626) over at most kBatchMaxBV
+// bounding surfaces; RESIDENT: the surfaces stay in shared memory (n <=
+// kBatchTile; always so with BV); REC: write hit indices instead of tallying.
+template <class M, int THREADS, bool BV, bool REC, bool RESIDENT>
+__global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
+{
+    using T = typename M::T;
+    constexpr int kPer = kCells / THREADS;                 // buckets per thread of the scan
+    constexpr int kMaxG = kChunkDraws / THREADS;           // draws per thread of the largest chunk
+    static_assert(THREADS % 32 == 0 && kPer % 4 == 0, "scan shape");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ rf_primitive s_emit;
+    __shared__ float4 s_frame[3];
+    __shared__ int s_wsum[THREADS / 32];
+    __shared__ int64_t s_chunk;
+    __shared__ int s_next, s_nvalid;
+
+    const int n = p.n, cd = p.chunk_draws;
+    const bool hist = !REC && p.use_smem_hist;
+    const CulledLayout lay(cd, RESIDENT ? n : 0, hist ? n : 0, BV ? p.nbv : 0);
+    int *cnt = reinterpret_cast<int *>(smem_raw + lay.cnt);
+    uint16_t *perm = reinterpret_cast<uint16_t *>(smem_raw + lay.perm);
+    uint32_t *unif = reinterpret_cast<uint32_t *>(smem_raw + lay.unif);
+    HitRec *s_tab = reinterpret_cast<HitRec *>(smem_raw + lay.tab);
+    float4 *s_bs = reinterpret_cast<float4 *>(smem_raw + lay.bs);
+    HitRec *s_bvtab = reinterpret_cast<HitRec *>(smem_raw + lay.bvtab);
+    int4 *s_bvinfo = reinterpret_cast<int4 *>(smem_raw + lay.bvinfo);
+    float4 *s_bvbs = reinterpret_cast<float4 *>(smem_raw + lay.bvbs);
+    int *s_hist = reinterpret_cast<int *>(smem_raw + lay.hist);
+    const HitRec *tab = RESIDENT ? s_tab : p.tab;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool sc = (p.compat & RF_COMPAT_SPHERE) != 0;
+    const T eps = T(p.eps);
+
+    if (RESIDENT) {
+        for (int i = tid; i < 4 * n; i += THREADS)
+            reinterpret_cast<float4 *>(s_tab)[i] = __ldg(reinterpret_cast<const float4 *>(p.tab) + i);
+        for (int i = tid; i < n; i += THREADS) s_bs[i] = __ldg(p.bsph + i);
+    }
+    if (BV) {
+        for (int i = tid; i < 4 * p.nbv; i += THREADS)
+            reinterpret_cast<float4 *>(s_bvtab)[i] = __ldg(reinterpret_cast<const float4 *>(p.bvtab) + i);
+        for (int i = tid; i < p.nbv; i += THREADS) {
+            s_bvinfo[i] = __ldg(p.bvinfo + i);
+            s_bvbs[i] = __ldg(p.bvsph + i);
+        }
+    }
+    if (hist)
+        for (int i = tid; i < n; i += THREADS) s_hist[i] = 0;
+
+    int emitter = -1;
+    int row_chunks = 0;  // chunks in the shared-memory row since its last flush
+    auto flush = [&]() {
+        __syncthreads();
+        if (hist && emitter >= 0) {
+            unsigned long long *row = p.hits + (int64_t)emitter * n;
+            for (int i = tid; i < n; i += THREADS) {
+                const int v = s_hist[i];
+                if (v) {
+                    atomicAdd(row + i, (unsigned long long)v);
+                    s_hist[i] = 0;
+                }
+            }
+        }
+        __syncthreads();
+    };
+
+    for (;;) {
+        if (tid == 0) s_chunk = (int64_t)atomicAdd(p.queue, 1ull);
+        __syncthreads();
+        const int64_t c = s_chunk;
+        if (c >= p.total_chunks) break;  // block-uniform
+        const Segment sg = p.seg[find_segment(p.seg, p.nseg, c)];
+        if (sg.emitter != emitter || ++row_chunks >= 32768) {  // (32-bit bins: at most 32768 hits per chunk)
+            flush();
+            row_chunks = 0;
+            if (sg.emitter != emitter) {
+                if (tid < (int)(sizeof(rf_primitive) / 4))
+                    reinterpret_cast<float *>(&s_emit)[tid] = reinterpret_cast<const float *>(p.emit + sg.emitter)[tid];
+                if (tid == 32 % THREADS) quick_frame(p.emit[sg.emitter], s_frame);
+                emitter = sg.emitter;
+            }
+        }
+        for (int i = tid; i < kCells; i += THREADS) cnt[i] = 0;
+        if (tid == 0) s_next = 0;
+        __syncthreads();
+        const int64_t gid0 = (sg.ray_begin >> 2) + (c - sg.chunk_begin) * (int64_t)cd;
+        const uint32_t sid = (p.compat & RF_COMPAT_STREAMS) ? 0u : p.scene_id;
+
+        // 1. uniforms and sort keys; a ray's key waits in perm[] until the sort
+#pragma unroll 1
+        for (int d = tid; d < cd; d += THREADS) {
+            const int64_t gid = gid0 + d;
+            uint2 kk = make_uint2(kCells | (kCells << 16), kCells | (kCells << 16));  // no valid ray
+            if (gid * 4 + 3 >= sg.ray_begin && gid * 4 < sg.ray_end) {
+                const uint4 u = stream_bits(p.compat, p.key1, sid, sg.emitter, gid);
+                pack_uniforms(u, unif[d], unif[cd + d], unif[2 * cd + d]);
+                const float uf[4] = {u01(u.x), u01(u.y), u01(u.z), u01(u.w)};
+                int key4[4];
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    float r[4];
+                    rotate_uniforms(uf, v, r);
+                    const int64_t rid = gid * 4 + v;
+                    const bool valid = rid >= sg.ray_begin && rid < sg.ray_end;
+                    key4[v] = valid ? quick_key(s_emit, s_frame, r) : kCells;
+                    if (valid) atomicAdd(&cnt[key4[v]], 1);
+                }
+                kk = make_uint2((uint32_t)key4[0] | ((uint32_t)key4[1] << 16),
+                                (uint32_t)key4[2] | ((uint32_t)key4[3] << 16));
+            }
+            *reinterpret_cast<uint2 *>(&perm[4 * d]) = kk;
+        }
+        __syncthreads();
+        uint2 mykeys[kMaxG];
+#pragma unroll
+        for (int g = 0; g < kMaxG; ++g)
+            if (g * THREADS + tid < cd) mykeys[g] = *reinterpret_cast<const uint2 *>(&perm[4 * (g * THREADS + tid)]);
+        // 2. counting sort: exclusive scan of the bucket sizes, kPer per thread
+        {
+            int sum = 0;
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) sum += cnt[kPer * tid + q];
+            int incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) s_wsum[warp] = incl;
+            __syncthreads();
+            if (warp == 0) {
+                const int x = lane < THREADS / 32 ? s_wsum[lane] : 0;
+                int xi = x;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, xi, o);
+                    if (lane >= o) xi += t;
+                }
+                if (lane < THREADS / 32) s_wsum[lane] = xi - x;
+                if (lane == 31) s_nvalid = xi;
+            }
+            __syncthreads();
+            int run = s_wsum[warp] + incl - sum;
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) {
+                const int v = cnt[kPer * tid + q];
+                cnt[kPer * tid + q] = run;
+                run += v;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int g = 0; g < kMaxG; ++g) {
+            const int d = g * THREADS + tid;
+            if (d < cd) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const uint32_t w = (v < 2) ? mykeys[g].x : mykeys[g].y;
+                    const int key = (int)((w >> (16 * (v & 1))) & 0xffffu);
+                    if (key < kCells) perm[atomicAdd(&cnt[key], 1)] = (uint16_t)(4 * d + v);
+                }
+            }
+        }
+        __syncthreads();
+
+        // 3. packets of 32 sorted rays
+        const int n_valid = s_nvalid;
+        const int n_packets = (n_valid + 31) >> 5;
+        for (;;) {
+            int k = 0;
+            if (lane == 0) k = atomicAdd(&s_next, 1);
+            k = __shfl_sync(0xffffffffu, k, 0);
+            if (k >= n_packets) break;  // warp-uniform
+            const int pos = k * 32 + lane;
+            const bool valid = pos < n_valid;
+            const int l = perm[valid ? pos : k * 32];  // (an idle lane repeats the packet's first ray)
+            Ray<T> ray;
+            {
+                const int d = l >> 2, v = l & 3;
+                float uf[4], r[4];
+                unpack_uniforms(unif[d], unif[cd + d], unif[2 * cd + d], uf);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int q = (i + v + 1) & 3;
+                    r[i] = q == 0 ? uf[0] : (q == 1 ? uf[1] : (q == 2 ? uf[2] : uf[3]));
+                }
+                ray = emit_ray<M>(s_emit, r);
+            }
+            const Ray<float> rf = to_f32(ray);
+            const float cc = dot3(rf.cx, rf.cy, rf.cz, rf.cx, rf.cy, rf.cz);
+            // a ray the bounds do not speak for: its packet tests everything
+            const bool odd = __any_sync(0xffffffffu, !(fabsf(rf.sx) + fabsf(rf.sy) + fabsf(rf.sz) < 1e15f) ||
+                                                         !(cc > 1e-6f && cc < 1e6f));
+            const float idd = MFast::rcp(cc);
+            Packet pk = bounds_of(rf, idd);
+            pk.cull = pk.cull && !odd;
+
+            // candidate words of the 1024 surfaces from j0 on, lane w holding word w: by
+            // sphere (cmask), and frusta in whose band some ray of the packet lies (bmask)
+            unsigned cmask = 0u, bmask = 0u;
+            auto candidates = [&](int j0) {
+                const int nwords = min(32, (n - j0 + 31) >> 5);
+#pragma unroll 1
+                for (int w = 0; w < nwords; ++w) {
+                    const int jw = j0 + (w << 5), js = jw + lane;
+                    bool cand = false, banded = false;
+                    if (js < n) {
+                        const float4 b = RESIDENT ? s_bs[js] : __ldg(p.bsph + js);
+                        cand = b.w != 0.0f && (!pk.cull || packet_reaches(pk, b));
+                        if (b.w < 0.0f) banded = pk.cull && packet_band(p.cquad, js, pk);
+                    }
+                    const unsigned cm = __ballot_sync(0xffffffffu, cand);
+                    unsigned bm = __ballot_sync(0xffffffffu, banded);
+                    for (unsigned todo = bm; todo; todo &= todo - 1) {  // warp-uniform
+                        const int b_ = __ffs(todo) - 1;
+                        if (!__any_sync(0xffffffffu, band(p.cquad, jw + b_, rf, cc))) bm &= ~(1u << b_);
+                    }
+                    if (lane == w) {
+                        cmask = cm;
+                        bmask = bm;
+                    }
+                }
+            };
+            // can the lane's ray be hit by surface j (a packet's sphere candidate)
+            auto gate = [&](int j) {
+                return odd || reaches(rf, idd, RESIDENT ? s_bs[j] : __ldg(p.bsph + j));
+            };
+            auto test = [&](int j, T &tb, int &bi) {  // every lane, the same j
+                const HitRec h = RESIDENT ? s_tab[j] : load_rec(p.tab, j);
+                const int type = __float_as_int(h.aux.x);
+                const unsigned m = (unsigned)__float_as_int(h.aux.w);
+                if (m) {  // the first of a stack of m surfaces: one search for all of them
+                    if (type == RF_ANNULUS)
+                        plate_hits<M>(h, tab, RESIDENT, j, (int)m, ray, eps, tb, bi);
+                    else
+                        ring_hits<M>(tab, RESIDENT, j, (int)m, __ldg(p.cstack + j), ray, rf, eps, odd, tb, bi);
+                } else {
+                    const T t = hit_any<M>(type, h, ray, eps, sc, M::inf());
+                    if (t < tb) {
+                        tb = t;
+                        bi = j;
+                    }
+                }
+            };
+            // nearest hit among the candidates of [lo, hi) within the words of j0, in index order
+            auto search = [&](int j0, int lo, int hi, T &tb, int &bi) {
+#pragma unroll 1
+                for (int w = (lo - j0) >> 5; w < 32 && j0 + (w << 5) < hi; ++w) {
+                    const int jw = j0 + (w << 5);
+                    const unsigned bm = __shfl_sync(0xffffffffu, bmask, w);
+                    unsigned cm = (__shfl_sync(0xffffffffu, cmask, w) | bm) & keep_from(lo - jw);
+                    if (hi < jw + 32) cm &= (1u << (hi - jw)) - 1u;
+                    while (cm) {  // the same in every lane; two spheres per pass (independent chains)
+                        const int ba_ = __ffs(cm) - 1;
+                        cm &= cm - 1;
+                        const int bb_ = cm ? __ffs(cm) - 1 : ba_;
+                        const bool two = cm != 0u;
+                        cm &= cm - 1;  // 0 stays 0
+                        const int ja = jw + ba_, jb = jw + bb_;
+                        const bool ma = gate(ja), mb = gate(jb);
+                        unsigned go = (__any_sync(0xffffffffu, ma) || ((bm >> ba_) & 1u)) ? 1u : 0u;
+                        if (two && (__any_sync(0xffffffffu, mb) || ((bm >> bb_) & 1u))) go |= 2u;
+#pragma unroll 1
+                        for (; go; go &= go - 1) test((go & 1u) ? ja : jb, tb, bi);
+                    }
+                }
+            };
+
+            int bi = -1;
+            if constexpr (BV) {  // RayFactorGPU.cl:580-619, the children's hit found when a lane needs it
+                candidates(0);  // n <= kBatchTile
+                T tbest = M::inf();
+                int bvi = -1, obj = -1, nb = -1;  // nb: children's nearest hit of the current winner bvi
+                for (int w = 0; w < p.nbv; ++w) {
+                    const bool may = odd || reaches(rf, idd, s_bvbs[w]);
+                    if (!__any_sync(0xffffffffu, may)) continue;
+                    const HitRec hb = s_bvtab[w];
+                    const T t = hit_any<M>(__float_as_int(hb.aux.x), hb, ray, eps, sc, M::inf());
+                    const bool nearer = t < tbest;
+                    if (!__any_sync(0xffffffffu, nearer)) continue;
+                    const int4 info = s_bvinfo[w];
+                    T tn = M::inf();
+                    int nw = -1;
+                    search(0, info.y, info.z, tn, nw);
+                    if (nearer) {
+                        if (info.x == 1) {  // counts only if a child is hit
+                            obj = nw;
+                            if (nw != -1) {
+                                tbest = t;
+                                bvi = w;
+                                nb = nw;
+                            }
+                        } else {
+                            tbest = t;
+                            bvi = w;
+                            nb = nw;
+                            if (!(p.compat & RF_COMPAT_BV_STALE)) obj = -1;
+                        }
+                    }
+                }
+                bi = (bvi != -1 && obj == -1) ? nb : obj;
+            } else {
+                T tb = M::inf();
+#pragma unroll 1
+                for (int j0 = 0; j0 < n; j0 += 1024) {
+                    candidates(j0);
+                    search(j0, j0, min(n, j0 + 1024), tb, bi);
+                }
+            }
+            if (REC) {
+                if (valid) p.rec[gid0 * 4 + l - p.rec_base] = bi;
+            } else if (hist) {
+                warp_tally(s_hist, valid ? bi : -1);
+            } else {
+                warp_tally_global(p.hits + (int64_t)emitter * n, valid ? bi : -1);
+            }
+        }
+        __syncthreads();
+    }
+    if (!REC) flush();
+}
+
+template <class M, bool BV, bool REC, bool RES>
+static cudaError_t launch_culled_k(const TraceParams &p, int sms, cudaStream_t st)
+{
+    // one block per SM: 1024 threads of 64 registers, in FP64 512 of 128 (two blocks of
+    // 512 or four of 256 threads with shorter chunks sort into less similar packets:
+    // 64 surfaces EXACT, 1e8 rays, 5.9 / 6.4 / 7.6 ms)
+    constexpr int THREADS = M::kF64 ? 512 : 1024;
+    auto k = culled_kernel<M, THREADS, BV, REC, RES>;
+    const int smem = CulledLayout(p.chunk_draws, RES ? p.n : 0, !REC && p.use_smem_hist ? p.n : 0, BV ? p.nbv : 0).bytes;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int grid = (int)max((int64_t)1, min((int64_t)sms, p.total_chunks));
+    k<<<grid, THREADS, smem, st>>>(p);
+    return cudaGetLastError();
+}
+
+template <class M>
+cudaError_t launch_culled(const TraceParams &p, bool bv, bool rec, int sms, cudaStream_t st)
+{
+    const bool res = p.n <= kBatchTile;
+    if (p.chunk_draws <= 0 || p.chunk_draws > kChunkDraws || p.chunk_draws % 4 ||
+        (bv && (!res || p.nbv <= 0 || p.nbv > kBatchMaxBV)) || (p.use_smem_hist && p.n > kBatchHist))
+        return cudaErrorInvalidValue;
+    if (bv)
+        return rec ? launch_culled_k<M, true, true, true>(p, sms, st) : launch_culled_k<M, true, false, true>(p, sms, st);
+    if (res)
+        return rec ? launch_culled_k<M, false, true, true>(p, sms, st) : launch_culled_k<M, false, false, true>(p, sms, st);
+    return rec ? launch_culled_k<M, false, true, false>(p, sms, st) : launch_culled_k<M, false, false, false>(p, sms, st);
+}
+
+}  // namespace rf

@@ -1,0 +1,7 @@
+// rf_culled_fast.cu -- the culled kernel with the FP32 hardware approximations; default
+// contraction like rf_kern_fast.cu.
+#include "rf_culled.cuh"
+
+namespace rf {
+template cudaError_t launch_culled<MFast>(const TraceParams &, bool, bool, int, cudaStream_t);
+}  // namespace rf

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 #include "rayfactor_gb300.h"
@@ -68,6 +69,9 @@ struct TraceParams {
     const uint32_t *cmask;          // batched kernel: cell masks of all rows that have them
     const int64_t *mask_off;        // per global row (prim_off + emitter): first mask word, -1 = none
     const float4 *bvsph;            // mixed kernels: bounding sphere of each bounding surface (as bsph)
+    const float4 *cquad;            // culled kernel: two words per surface, a frustum's A and its threshold
+    const float4 *cstack;           // culled kernel: per surface, slack of its ring stack
+    int32_t chunk_draws;            // culled kernel: draws of a chunk
 };
 
 // Cell masks of the batched kernel (build_masks_kernel): one bit per surface for
@@ -115,6 +119,19 @@ struct LaunchCfg {
 // Implemented once per arithmetic policy (rf_kern_exact.cu, rf_kern_fast.cu).
 template <class M> cudaError_t launch_trace(const LaunchCfg &cfg, const TraceParams &p, cudaStream_t st);
 template <class M> int trace_blocks_per_sm(const LaunchCfg &cfg);
+
+// The plain kernels' results with the surfaces that a ray cannot hit left out
+// (rf_culled.cuh; one translation unit per policy).
+template <class M> cudaError_t launch_culled(const TraceParams &p, bool bv, bool rec, int sms, cudaStream_t st);
+
+// The culled kernel's tables of one scene (rf_bounds.cu): sph (n), a ball around
+// the points a surface can return as hits (squared radius in w, infinite when there
+// is no bound, negative for a frustum, whose bound holds outside its band, 0 for a
+// stack's later members); quad (2 n), slack (n, ring stacks), bvsph (nbv); a stack's
+// size goes into its first member's tab[].aux.w.
+// False when the bounds leave too little out.  stacks: look for ring stacks.
+bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs, int nbv, bool stacks, HitRec *tab,
+                 float4 *sph, float4 *quad, float4 *slack, float4 *bvsph);
 
 // Batched mixed-precision persistent kernel (rf_kern_batched.cu); count: also
 // collect the work counters (TraceParams::work); stacks: some scene's tables
