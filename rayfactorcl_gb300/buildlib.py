@@ -35,6 +35,7 @@ UNITS = {
     "rf_kern_post.cu": [],
     "rf_capi.cu": [],
     "rf_bounds.cu": [],
+    "rf_masks.cu": [],
     "rf_noalloc.cu": [],
 }
 HEADERS = ["rf_internal.h", "rf_device.cuh", "rf_trace_kernels.cuh", "rf_batched.cuh", "rf_mixed_small.cuh", "rf_culled.cuh"]

@@ -1206,75 +1206,4 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
     if (COUNT && tid < 8 && p.work && S.work[tid]) atomicAdd(p.work + tid, S.work[tid]);
 }
 
-// ---------------------------------------------------------------------------
-// Cell masks.  For a row (scene, emitter) and each of the kCells sort keys,
-// bit j of the key's mask says whether any ray of that emitter whose key it is
-// can reach surface j: origins in the parameter patch's ball (MaskInputs::patch,
-// 16 per emitter), directions in the direction cell's cone (cone[2*cell],
-// axis and cos in xyzw, sin in the next entry's x), surfaces covered by up to
-// kChainMax spheres (chain; radius < 0 ends the list) and, for planar surfaces,
-// the plane (plane.xyz unit normal, w = normal . point; w NaN: not planar), which
-// no ray crosses when the whole ball lies on one side and every direction of the
-// cone points away from it.  A ray from a ball B(c, rho) with a direction within
-// theta of axis a comes within R of a point C only if angle(C - c, a) <=
-// theta + asin((R + rho) / |C - c|).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ bool cell_reaches(float4 ball, float4 axis_cos, float sin_t, float4 sph)
-{
-    const float vx = sph.x - ball.x, vy = sph.y - ball.y, vz = sph.z - ball.z;
-    const float L2 = vx * vx + vy * vy + vz * vz;
-    const float R = (sph.w + ball.w) * 1.0001f + 1e-5f * sqrtf(L2) + 1e-7f;
-    if (L2 <= R * R) return true;
-    const float va = vx * axis_cos.x + vy * axis_cos.y + vz * axis_cos.z;
-    return va >= axis_cos.w * sqrtf(L2 - R * R) - sin_t * R;
-}
-
-__device__ __forceinline__ bool plane_separates(float4 ball, float4 axis_cos, float sin_t, float4 pl)
-{
-    if (!(pl.w == pl.w)) return false;  // not planar
-    const float h = pl.x * ball.x + pl.y * ball.y + pl.z * ball.z - pl.w;
-    const float na = pl.x * axis_cos.x + pl.y * axis_cos.y + pl.z * axis_cos.z;
-    const float margin = ball.w * 1e-4f + 1e-6f * (fabsf(pl.w) + ball.w) + 1e-7f;
-    if (h > ball.w + margin) return na >= sin_t + 1e-4f;     // every ray moves away on the + side
-    if (h < -(ball.w + margin)) return -na >= sin_t + 1e-4f; // ... or on the - side
-    return false;
-}
-
-static __global__ void __launch_bounds__(256) build_masks_kernel(MaskInputs in, uint32_t *out)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= in.total_words) return;
-    int lo = 0, hi = in.nrows - 1;  // the row holding word t (rows sorted by off)
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (in.rows[mid].off <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    const MaskRow row = in.rows[lo];
-    const SceneInfo si = in.scenes[row.scene];
-    const int nwords = (si.n + 31) >> 5;
-    const int64_t local = t - row.off;
-    const int cell = (int)(local / nwords), w = (int)(local % nwords);
-    const float4 ball = in.patch[(int64_t)(si.prim_off + row.emitter) * 16 + (cell & 15)];
-    const float4 ac = in.cone[2 * (cell >> 4)];
-    const float sin_t = in.cone[2 * (cell >> 4) + 1].x;
-    uint32_t bits = 0u;
-    for (int b = 0; b < 32; ++b) {
-        const int j = 32 * w + b;
-        if (j >= si.n) break;
-        const int gj = si.prim_off + j;
-        bool ok = false;
-        for (int k = 0; k < kChainMax && !ok; ++k) {
-            const float4 sph = in.chain[(int64_t)gj * kChainMax + k];
-            if (sph.w < 0.0f) break;
-            ok = cell_reaches(ball, ac, sin_t, sph);
-        }
-        const float4 pl = in.plane[gj];
-        if (ok && plane_separates(ball, ac, sin_t, pl)) ok = false;
-        if (j == row.emitter && pl.w == pl.w) ok = false;  // a planar emitter cannot hit itself (self_skip)
-        bits |= (ok ? 1u : 0u) << b;
-    }
-    out[t] = bits;
-}
-
 }  // namespace rf

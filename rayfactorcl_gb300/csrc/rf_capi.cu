@@ -126,10 +126,9 @@ struct rf_ctx {
     // batched mixed-precision path: scenes concatenated, re-centred in FP64
     DevBuf b_tab, b_emit, b_bsph, b_scenes, b_hits, b_rows, b_counters;
     // cell masks of the batched kernel and their inputs (built at upload)
-    DevBuf b_patch, b_chain, b_plane, b_cone, b_maskrows, b_maskoff, b_mask, b_frame;
+    DevBuf b_own, b_patch, b_chain, b_plane, b_cone, b_maskrows, b_maskoff, b_mask, b_frame;
     DevBuf b_bvtab, b_bvinfo, b_bvsph;  // the single scene's bounding surfaces, re-centred like its surfaces
     bool b_masks = false;
-    double b_mask_ms = 0.0;     // device time of the last mask build
     std::vector<SceneInfo> b_info;
     int64_t b_hits_total = 0;
     bool b_single = false;      // b_* hold the scene of rf_set_scene
@@ -628,184 +627,6 @@ float scene_eps(float eps, const float4 *bs, int n)
     return (float)(-(double)eps * std::sqrt(dx * dx + dy * dy + dz * dz));
 }
 
-// --- cell-mask inputs (FP64 on the host, in the scene's re-centred frame) ---
-
-// World point of an object-space point under a re-centred record's m.
-void xf_point(const rf_primitive &e, const double o[3], double w[3])
-{
-    for (int k = 0; k < 3; ++k) {
-        const float *r = e.m + 4 * k;
-        w[k] = (double)r[0] * o[0] + (double)r[1] * o[1] + (double)r[2] * o[2] + (double)r[3];
-    }
-}
-
-// Candidate angles of an angular interval for the extremes of sin and cos:
-// its ends and the multiples of pi/2 inside it.
-int angle_candidates(double t0, double t1, double *out)
-{
-    int k = 0;
-    out[k++] = t0;
-    out[k++] = t1;
-    for (int q = 0; q <= 8; ++q) {
-        const double a = q * (M_PI / 2);
-        if (a > t0 && a < t1) out[k++] = a;
-    }
-    return k;
-}
-
-// Object-space box of parameter patch (pi, pj) of an emitter -- the points its
-// rays start from when r[0] in [pi/4, (pi+1)/4) and r[1] in [pj/4, (pj+1)/4)
-// (emission formulas RayFactorGPU.cl:298-443).  Each coordinate is linear in the
-// radius-like parameter for a fixed angle, and the angle's extremes are at the
-// ends of its interval or at multiples of pi/2, so the listed points bound the
-// patch.  Returns false when the formulas give no finite point (a frustum whose
-// top radius is 1).
-bool patch_box(const rf_primitive &e, int pi, int pj, double lo[3], double hi[3])
-{
-    const double a0 = pi / 4.0, a1 = (pi + 1) / 4.0, b0 = pj / 4.0, b1 = (pj + 1) / 4.0;
-    const double u1 = e.util1, u2 = e.util2;
-    double th[16], pts[64][3];
-    int np = 0, nt;
-    auto add = [&](double x, double y, double z) {
-        pts[np][0] = x; pts[np][1] = y; pts[np][2] = z; ++np;
-    };
-    switch (e.type) {
-    case RF_DISC:
-    case RF_ANNULUS: {
-        double r0, r1;
-        if (e.type == RF_DISC) { r0 = std::sqrt(b0); r1 = std::sqrt(b1); }
-        else {
-            r0 = std::sqrt(std::max(0.0, u1 + (u2 - u1) * b0));
-            r1 = std::sqrt(std::max(0.0, u1 + (u2 - u1) * b1));
-        }
-        nt = angle_candidates(2 * M_PI * a0, 2 * M_PI * a1, th);
-        for (int k = 0; k < nt; ++k)
-            for (double r : {r0, r1}) add(r * std::sin(th[k]), r * std::cos(th[k]), 0.0);
-        break;
-    }
-    case RF_RECTANGLE:
-        for (double x : {2 * a0 - 1, 2 * a1 - 1})
-            for (double y : {2 * b0 - 1, 2 * b1 - 1}) add(x, y, 0.0);
-        break;
-    case RF_CYLINDER:
-        nt = angle_candidates(2 * M_PI * a0, 2 * M_PI * a1, th);
-        for (int k = 0; k < nt; ++k)
-            for (double z : {b0, b1}) add(std::cos(th[k]), std::sin(th[k]), z);
-        break;
-    case RF_FRUSTUM: {
-        auto zf = [&](double a) { return (std::sqrt(1.0 - a + a * u1 * u1) - 1.0) / (u1 - 1.0); };
-        const double z0 = zf(a0), z1 = zf(a1);
-        if (!std::isfinite(z0) || !std::isfinite(z1)) return false;
-        nt = angle_candidates(2 * M_PI * b0, 2 * M_PI * b1, th);
-        for (int k = 0; k < nt; ++k)
-            for (double z : {z0, z1}) {
-                const double rho = 1.0 + z * (u1 - 1.0);
-                add(rho * std::cos(th[k]), rho * std::sin(th[k]), z);
-            }
-        break;
-    }
-    case RF_SPHERE: {
-        double zs[3] = {2 * a0 - 1, 2 * a1 - 1, 0.0};
-        const int nz = (zs[0] < 0.0 && zs[1] > 0.0) ? 3 : 2;
-        nt = angle_candidates(2 * M_PI * b0, 2 * M_PI * b1, th);
-        for (int k = 0; k < nt; ++k)
-            for (int q = 0; q < nz; ++q) {
-                const double rho = std::sqrt(std::max(0.0, 1.0 - zs[q] * zs[q]));
-                add(rho * std::cos(th[k]), rho * std::sin(th[k]), zs[q]);
-            }
-        break;
-    }
-    default:
-        return false;
-    }
-    for (int k = 0; k < 3; ++k) { lo[k] = 1e300; hi[k] = -1e300; }
-    for (int q = 0; q < np; ++q)
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = std::min(lo[k], pts[q][k]);
-            hi[k] = std::max(hi[k], pts[q][k]);
-        }
-    return true;
-}
-
-// Ball around the image of an object-space box: the image of the box centre and
-// the farthest image of a corner (the image is a parallelepiped), widened for
-// the FP32 emission's rounding and approximations.
-float4 box_ball(const rf_primitive &e, const double lo[3], const double hi[3])
-{
-    const double oc[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
-    double c[3], rad = 0.0;
-    xf_point(e, oc, c);
-    for (int q = 0; q < 8; ++q) {
-        const double o[3] = {(q & 1) ? hi[0] : lo[0], (q & 2) ? hi[1] : lo[1], (q & 4) ? hi[2] : lo[2]};
-        double w[3];
-        xf_point(e, o, w);
-        rad = std::max(rad, std::sqrt((w[0] - c[0]) * (w[0] - c[0]) + (w[1] - c[1]) * (w[1] - c[1]) +
-                                      (w[2] - c[2]) * (w[2] - c[2])));
-    }
-    const double cn = std::sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
-    return make_float4((float)c[0], (float)c[1], (float)c[2], (float)(rad * (1 + 1e-4) + 1e-5 * (cn + rad) + 1e-7));
-}
-
-// Sixteen parameter-patch balls of an emitter (infinite radius when a patch has
-// no finite bound: every surface is then a candidate).
-void patch_balls(const rf_primitive &e, float4 *out)
-{
-    for (int pi = 0; pi < 4; ++pi)
-        for (int pj = 0; pj < 4; ++pj) {
-            double lo[3], hi[3];
-            out[4 * pi + pj] = patch_box(e, pi, pj, lo, hi) ? box_ball(e, lo, hi)
-                                                            : make_float4(0.f, 0.f, 0.f, INFINITY);
-        }
-}
-
-// Spheres covering a surface: for a cylinder or frustum longer than it is wide,
-// a chain of up to kChainMax spheres along its axis (points A + rho(z) (c0 cos +
-// c1 sin) + Z z of slab [z0, z1] lie within rmax * max rho + |Z| (z1 - z0) / 2 of
-// the slab's axis midpoint, rmax the largest radius of the ellipse spanned by the
-// first two columns); otherwise the bounding sphere `bs` (radius in w).
-int surface_chain(const rf_primitive &e, float4 bs, float4 *out)
-{
-    for (int k = 0; k < kChainMax; ++k) out[k] = make_float4(0.f, 0.f, 0.f, -1.f);
-    out[0] = bs;
-    if (e.type != RF_CYLINDER && e.type != RF_FRUSTUM) return 1;
-    double A[3], Z[3], c0[3], c1[3];
-    for (int k = 0; k < 3; ++k) {
-        A[k] = e.m[4 * k + 3];
-        c0[k] = e.m[4 * k + 0];
-        c1[k] = e.m[4 * k + 1];
-        Z[k] = e.m[4 * k + 2];
-    }
-    const double L = std::sqrt(Z[0] * Z[0] + Z[1] * Z[1] + Z[2] * Z[2]);
-    const double g00 = c0[0] * c0[0] + c0[1] * c0[1] + c0[2] * c0[2];
-    const double g11 = c1[0] * c1[0] + c1[1] * c1[1] + c1[2] * c1[2];
-    const double g01 = c0[0] * c1[0] + c0[1] * c1[1] + c0[2] * c1[2];
-    const double rmax = std::sqrt(0.5 * (g00 + g11 + std::sqrt((g00 - g11) * (g00 - g11) + 4 * g01 * g01)));
-    const double top = e.type == RF_FRUSTUM ? (double)e.util1 : 1.0;
-    const double wide = rmax * std::max(1.0, std::fabs(top));
-    if (!(L > 0.0) || !(wide > 0.0) || !std::isfinite(L + wide)) return 1;
-    const int K = (int)std::min<double>(kChainMax, std::ceil(L / wide));
-    if (K < 2) return 1;
-    for (int k = 0; k < K; ++k) {
-        const double z0 = (double)k / K, z1 = (double)(k + 1) / K, zm = 0.5 * (z0 + z1);
-        const double rho = std::max(std::fabs(1.0 + z0 * (top - 1.0)), std::fabs(1.0 + z1 * (top - 1.0)));
-        const double c[3] = {A[0] + Z[0] * zm, A[1] + Z[1] * zm, A[2] + Z[2] * zm};
-        const double r = rmax * rho + 0.5 * L * (z1 - z0);
-        const double cn = std::sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
-        out[k] = make_float4((float)c[0], (float)c[1], (float)c[2], (float)(r * (1 + 1e-4) + 1e-5 * (cn + r) + 1e-7));
-    }
-    return K;
-}
-
-// Plane of a disc, annulus or rectangle: object z = 0 is row 2 of invm.
-float4 surface_plane(const rf_primitive &e)
-{
-    if (e.type != RF_DISC && e.type != RF_ANNULUS && e.type != RF_RECTANGLE) return make_float4(0.f, 0.f, 0.f, NAN);
-    const double n[3] = {e.invm[8], e.invm[9], e.invm[10]};
-    const double nn = std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-    if (!(nn > 0.0)) return make_float4(0.f, 0.f, 0.f, NAN);
-    return make_float4((float)(n[0] / nn), (float)(n[1] / nn), (float)(n[2] / nn), (float)(-(double)e.invm[11] / nn));
-}
-
 // Unit direction of octahedral-map point (u, v): the inverse of the map that
 // the kernel's direction_cell applies.
 void oct_dir(double u, double v, double d[3])
@@ -927,8 +748,7 @@ rf_status upload_batch(rf_ctx *c, const rf_scene_desc *scenes, int ns, bool with
     if (nprim > (1ll << 31) / 4) return fail(c, RF_ERR_OVERFLOW, "too many surfaces in the batch");
     std::vector<rf_primitive> emit(nprim);
     std::vector<HitRec> tab(nprim);
-    std::vector<float4> bs(nprim), patch((size_t)nprim * 16), chain((size_t)nprim * kChainMax), plane(nprim),
-        frame((size_t)nprim * kEmitFrameWords);
+    std::vector<float4> bs(nprim), own(nprim), frame((size_t)nprim * kEmitFrameWords);
     c->b_info.resize(ns);
     c->b_stacks = 0;
     int64_t off = 0, hoff = 0;
@@ -938,11 +758,8 @@ rf_status upload_batch(rf_ctx *c, const rf_scene_desc *scenes, int ns, bool with
         c->b_info[s].eps = scene_eps(c->cfg.eps, bs.data() + off, n);
         c->b_info[s].pad = 0;
         for (int i = 0; i < n; ++i) {
-            const int64_t g = off + i;
-            patch_balls(emit[g], patch.data() + g * 16);
-            surface_chain(emit[g], bs[g], chain.data() + g * kChainMax);  // the masks: per surface
-            plane[g] = surface_plane(emit[g]);
-            emit_frame(emit[g], frame.data() + g * kEmitFrameWords);
+            own[off + i] = bs[off + i];  // the masks: per surface, not per stack
+            emit_frame(emit[off + i], frame.data() + (off + i) * kEmitFrameWords);
         }
         if (!c->cfg.split_stacks)
             c->b_stacks += mark_stacks(emit.data() + off, n, tab.data() + off, bs.data() + off,
@@ -1003,19 +820,19 @@ rf_status upload_batch(rf_ctx *c, const rf_scene_desc *scenes, int ns, bool with
     RF_CUDA(c, cudaMemcpyAsync(c->b_scenes.p, c->b_info.data(), sizeof(SceneInfo) * ns, cudaMemcpyHostToDevice, c->stream));
 
     c->b_masks = !mrows.empty();
-    c->b_mask_ms = 0.0;
     if (c->b_masks) {
         const std::vector<float4> &cones = direction_cones();
-        RF_CUDA(c, c->b_patch.ensure(sizeof(float4) * patch.size()));
-        RF_CUDA(c, c->b_chain.ensure(sizeof(float4) * chain.size()));
-        RF_CUDA(c, c->b_plane.ensure(sizeof(float4) * plane.size()));
+        RF_CUDA(c, c->b_own.ensure(sizeof(float4) * nprim));
+        RF_CUDA(c, c->b_patch.ensure(sizeof(float4) * nprim * 16));
+        RF_CUDA(c, c->b_chain.ensure(sizeof(float4) * nprim * kChainMax));
+        RF_CUDA(c, c->b_plane.ensure(sizeof(float4) * nprim));
         RF_CUDA(c, c->b_cone.ensure(sizeof(float4) * cones.size()));
         RF_CUDA(c, c->b_maskrows.ensure(sizeof(MaskRow) * mrows.size()));
         RF_CUDA(c, c->b_maskoff.ensure(sizeof(int64_t) * moff.size()));
         RF_CUDA(c, c->b_mask.ensure(sizeof(uint32_t) * (size_t)mwords));
-        RF_CUDA(c, cudaMemcpyAsync(c->b_patch.p, patch.data(), sizeof(float4) * patch.size(), cudaMemcpyHostToDevice, c->stream));
-        RF_CUDA(c, cudaMemcpyAsync(c->b_chain.p, chain.data(), sizeof(float4) * chain.size(), cudaMemcpyHostToDevice, c->stream));
-        RF_CUDA(c, cudaMemcpyAsync(c->b_plane.p, plane.data(), sizeof(float4) * plane.size(), cudaMemcpyHostToDevice, c->stream));
+        RF_CUDA(c, cudaMemcpyAsync(c->b_own.p, own.data(), sizeof(float4) * nprim, cudaMemcpyHostToDevice, c->stream));
+        RF_CUDA(c, launch_mask_inputs(c->b_emit.as<rf_primitive>(), c->b_own.as<float4>(), (int)nprim, c->b_patch.as<float4>(),
+                                      c->b_chain.as<float4>(), c->b_plane.as<float4>(), c->stream));
         RF_CUDA(c, cudaMemcpyAsync(c->b_cone.p, cones.data(), sizeof(float4) * cones.size(), cudaMemcpyHostToDevice, c->stream));
         RF_CUDA(c, cudaMemcpyAsync(c->b_maskrows.p, mrows.data(), sizeof(MaskRow) * mrows.size(), cudaMemcpyHostToDevice, c->stream));
         RF_CUDA(c, cudaMemcpyAsync(c->b_maskoff.p, moff.data(), sizeof(int64_t) * moff.size(), cudaMemcpyHostToDevice, c->stream));
@@ -1028,12 +845,7 @@ rf_status upload_batch(rf_ctx *c, const rf_scene_desc *scenes, int ns, bool with
         in.cone = c->b_cone.as<float4>();
         in.chain = c->b_chain.as<float4>();
         in.plane = c->b_plane.as<float4>();
-        RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
         RF_CUDA(c, launch_build_masks(in, c->b_mask.as<uint32_t>(), c->stream));
-        RF_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-        RF_CUDA(c, cudaStreamSynchronize(c->stream));
-        float ms = 0.f;
-        if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->b_mask_ms = ms;
     }
 
     RF_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1313,7 +1125,7 @@ void rf_destroy(rf_ctx *c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (DevBuf *b : {&c->d_tab, &c->d_emit, &c->d_bvtab, &c->d_bvinfo, &c->d_hits, &c->d_seg,
                       &c->d_rays, &c->d_F, &c->d_rec, &c->d_cull, &c->d_err, &c->d_misc, &c->b_tab, &c->b_emit,
-                      &c->b_bsph, &c->b_scenes, &c->b_hits, &c->b_rows, &c->b_counters, &c->b_patch,
+                      &c->b_bsph, &c->b_scenes, &c->b_hits, &c->b_rows, &c->b_counters, &c->b_own, &c->b_patch,
                       &c->b_chain, &c->b_plane, &c->b_cone, &c->b_maskrows, &c->b_maskoff, &c->b_mask, &c->b_frame, &c->b_bvtab,
                       &c->b_bvinfo, &c->b_bvsph})
         b->release();

@@ -74,7 +74,7 @@ struct TraceParams {
     int32_t chunk_draws;            // culled kernel: draws of a chunk
 };
 
-// Cell masks of the batched kernel (build_masks_kernel): one bit per surface for
+// Cell masks of the batched kernel (rf_masks.cu): one bit per surface for
 // each of kMaskCells sort keys of a row (scene, emitter).
 constexpr int kMaskCells = 4096;
 constexpr int kChainMax = 8;            // bounding spheres per surface in the mask test
@@ -141,6 +141,8 @@ cudaError_t launch_batched(const TraceParams &p, bool rec, bool resident, bool c
 // The same kernel with runBVGPU's bounding-surface semantics (one resident scene).
 cudaError_t launch_batched_bv(const TraceParams &p, bool rec, bool count, bool stacks, int grid, cudaStream_t st);
 int batched_blocks_per_sm(bool rec, bool resident);
+cudaError_t launch_mask_inputs(const rf_primitive *emit, const float4 *sph, int n, float4 *patch, float4 *chain,
+                               float4 *plane, cudaStream_t st);
 cudaError_t launch_build_masks(const MaskInputs &in, uint32_t *out, cudaStream_t st);
 // Mixed-precision kernel for one small scene with the plain kernel's launch shape
 // (rf_kern_fast.cu): gpt Philox draws per thread, block kSmallThreads.

@@ -1,6 +1,6 @@
 // rf_kern_batched.cu -- launchers of the batched mixed-precision persistent
 // kernel (every instantiation: record / resident / counting / bounding-surface /
-// segment-stack variants) and of the cell-mask builder.
+// segment-stack variants).
 #include "rf_trace_kernels.cuh"
 #include "rf_batched.cuh"
 
@@ -76,15 +76,6 @@ int batched_blocks_per_sm(bool rec, bool resident)
 {
     if (rec) return resident ? occ_b<true, true>() : occ_b<true, false>();
     return resident ? occ_b<false, true>() : occ_b<false, false>();
-}
-
-cudaError_t launch_build_masks(const MaskInputs &in, uint32_t *out, cudaStream_t st)
-{
-    if (in.total_words <= 0) return cudaSuccess;
-    const int64_t blocks = (in.total_words + 255) / 256;
-    if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
-    build_masks_kernel<<<(unsigned)blocks, 256, 0, st>>>(in, out);
-    return cudaGetLastError();
 }
 
 int batched_tile() { return kBatchTile; }
