@@ -272,6 +272,32 @@ int ring_stack(const rf_primitive *prims, int n, int i, const std::vector<char> 
 
 }  // namespace
 
+float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, double reach, bool loose_balls)
+{
+    if (loose_balls && e.type == RF_SPHERE) return box;
+    const double M[9] = {e.m[0], e.m[1], e.m[2], e.m[4], e.m[5], e.m[6], e.m[8], e.m[9], e.m[10]};
+    const double t[3] = {e.m[3], e.m[7], e.m[11]};
+    Extent x = extent_of(e.type, e.util1, e.type == RF_ANNULUS ? outer2 : e.util2);
+    if (rings > 1) x.z1 = rings;
+    if (e.type == RF_FRUSTUM) {
+        double L2 = 0.0;
+        for (int k = 0; k < 3; ++k)
+            L2 = std::max(L2, (double)e.invm[4 * k] * e.invm[4 * k] + (double)e.invm[4 * k + 1] * e.invm[4 * k + 1] +
+                                  (double)e.invm[4 * k + 2] * e.invm[4 * k + 2]);
+        const double over = 16.0 * 4096.0 / (1 << 24) * std::sqrt(3.0 * L2) * reach;
+        const double grow = std::fabs((double)e.util1 - 1.0) * over;
+        x.z0 -= over;
+        x.z1 += over;
+        x.r0 += grow;
+        x.r1 += grow;
+    }
+    const Ball b = image_ball(M, t, x);
+    const double cn = std::sqrt(dot(b.c, b.c));
+    const double r = b.r * (1.0 + 1e-5) + 1e-6 * (cn + b.r) + 1e-7;
+    if (!(r < (double)box.w)) return box;
+    return make_float4((float)b.c[0], (float)b.c[1], (float)b.c[2], (float)r);
+}
+
 bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs, int nbv, bool stacks, HitRec *tab,
                  float4 *sph, float4 *quad, float4 *slack, float4 *bvsph)
 {

@@ -460,11 +460,12 @@ rf_status validate_prims(rf_ctx *c, const rf_primitive *prims, int32_t n, int sc
 }
 
 // The kernel's ray/sphere test takes the squared radius, widened by 1 % for
-// directions that are unit only to ~1e-3 and for FP32 rounding.
-float4 widen_sq(float4 b)
+// directions that are unit only to ~1e-3 and for FP32 rounding; slack: the test's own
+// rounding at the scene's distances.
+float4 widen_sq(float4 b, double slack = 0.0)
 {
     const double r = (double)b.w * 1.01 + 1e-6 + 1e-6 * std::sqrt((double)b.x * b.x + (double)b.y * b.y + (double)b.z * b.z);
-    return make_float4(b.x, b.y, b.z, (float)(r * r));
+    return make_float4(b.x, b.y, b.z, (float)(r * r + slack));
 }
 
 // Bounding sphere (centre, radius) of the object-space box [-ext, ext]^2 x [z0, z1]
@@ -529,6 +530,17 @@ void prepare_mixed(const rf_primitive *prims, int n, rf_primitive *emit, HitRec 
     }
 }
 
+// Longest distance between two points of a re-centred scene, and the rounding of a
+// ray/sphere check over it (64 ulps of its square).
+double scene_reach(const float4 *bs, int n)
+{
+    double r = 0.0;
+    for (int i = 0; i < n; ++i)
+        r = std::max(r, std::sqrt((double)bs[i].x * bs[i].x + (double)bs[i].y * bs[i].y + (double)bs[i].z * bs[i].z) + bs[i].w);
+    return 2.0 * r;
+}
+double reach_slack(double reach) { return 64.0 / (1 << 24) * reach * reach; }
+
 // Segment stacks of one scene's mixed tables, runs [a, a + m) of 2 <= m <= 65535
 // consecutive surfaces.  Cylinder stacks (kStackType): the same linear part of m
 // (axes and radii), the same normal sign (util2) and each translation one axis
@@ -542,7 +554,7 @@ void prepare_mixed(const rf_primitive *prims, int n, rf_primitive *emit, HitRec 
 // across an index i with cut[i] set (a bounding surface's children start or end
 // there).  Every member's bounding sphere becomes the stack's.  Returns the
 // number of stacks.
-int mark_stacks(const rf_primitive *e, int n, HitRec *tab, float4 *bs, const std::vector<char> &cut)
+int mark_stacks(const rf_primitive *e, int n, HitRec *tab, float4 *bs, double reach, const std::vector<char> &cut)
 {
     auto cont = [&](int j) { return j < n && !((size_t)j < cut.size() && cut[j]); };
     int nstacks = 0;
@@ -556,7 +568,8 @@ int mark_stacks(const rf_primitive *e, int n, HitRec *tab, float4 *bs, const std
                 ++j;
             const int m = j - i;
             if (m >= 2) {
-                const float4 sph = object_box_sphere(e[i], std::sqrt((double)e[j - 1].util2), 0.0, 0.0);
+                const float4 sph = tight_sphere(e[i], object_box_sphere(e[i], std::sqrt((double)e[j - 1].util2), 0.0, 0.0), 1,
+                                                e[j - 1].util2, reach, false);
                 for (int k = 0; k < m; ++k) {
                     int32_t ti = kPlateType, w = (m << 16) | k;
                     std::memcpy(&tab[i + k].aux.x, &ti, 4);
@@ -593,7 +606,7 @@ int mark_stacks(const rf_primitive *e, int n, HitRec *tab, float4 *bs, const std
             int32_t ti = kStackType;
             std::memcpy(&u.aux.x, &ti, 4);
             u.aux.y = (float)m;
-            const float4 sph = object_box_sphere(e[i], 1.0, 0.0, (double)m);
+            const float4 sph = tight_sphere(e[i], object_box_sphere(e[i], 1.0, 0.0, (double)m), m, 0.f, reach, false);
             for (int k = 0; k < m; ++k) {
                 tab[i + k] = u;
                 const int32_t w = (m << 16) | k;
@@ -716,13 +729,16 @@ void rf::emit_frame(const rf_primitive &e, float4 *f)
 // Mixed-precision tables of one scene as the batched kernel reads them
 // (re-centred transforms, hit records, bounding spheres with squared radius)
 // and the scene's self-hit threshold (eps < 0: relative, as rf_trace forms it).
-int rf::prepare_mixed_tables(const rf_primitive *prims, int n, float eps, rf_primitive *emit, HitRec *tab,
+int rf::prepare_mixed_tables(const rf_primitive *prims, int n, float eps, uint32_t compat, rf_primitive *emit, HitRec *tab,
                              float4 *bs, float *eps_out)
 {
     prepare_mixed(prims, n, emit, tab, bs);
     *eps_out = scene_eps(eps, bs, n);
-    const int nstacks = mark_stacks(emit, n, tab, bs, std::vector<char>());
-    for (int i = 0; i < n; ++i) bs[i] = widen_sq(bs[i]);
+    const double reach = scene_reach(bs, n);
+    for (int i = 0; i < n; ++i)
+        bs[i] = tight_sphere(emit[i], bs[i], 1, emit[i].util2, reach, (compat & RF_COMPAT_SPHERE) != 0);
+    const int nstacks = mark_stacks(emit, n, tab, bs, reach, std::vector<char>());
+    for (int i = 0; i < n; ++i) bs[i] = widen_sq(bs[i], reach_slack(reach));
     return nstacks;
 }
 
@@ -757,12 +773,15 @@ rf_status upload_batch(rf_ctx *c, const rf_scene_desc *scenes, int ns, bool with
         prepare_mixed(scenes[s].prims, n, emit.data() + off, tab.data() + off, bs.data() + off);
         c->b_info[s].eps = scene_eps(c->cfg.eps, bs.data() + off, n);
         c->b_info[s].pad = 0;
+        const double reach = scene_reach(bs.data() + off, n);
         for (int i = 0; i < n; ++i) {
+            bs[off + i] = tight_sphere(emit[off + i], bs[off + i], 1, emit[off + i].util2, reach,
+                                       (c->cfg.compat & RF_COMPAT_SPHERE) != 0);
             own[off + i] = bs[off + i];  // the masks: per surface, not per stack
             emit_frame(emit[off + i], frame.data() + (off + i) * kEmitFrameWords);
         }
         if (!c->cfg.split_stacks)
-            c->b_stacks += mark_stacks(emit.data() + off, n, tab.data() + off, bs.data() + off,
+            c->b_stacks += mark_stacks(emit.data() + off, n, tab.data() + off, bs.data() + off, reach,
                                        s == 0 ? cut0 : std::vector<char>());
         if (s == 0) {
             c->b_test_type.assign(n, 0);
@@ -774,7 +793,7 @@ rf_status upload_batch(rf_ctx *c, const rf_scene_desc *scenes, int ns, bool with
                 c->b_test_type[i] = (ti < kStackType || (w & 0xffff) == 0) ? own : -1;
             }
         }
-        for (int i = 0; i < n; ++i) bs[off + i] = widen_sq(bs[off + i]);
+        for (int i = 0; i < n; ++i) bs[off + i] = widen_sq(bs[off + i], reach_slack(reach));
         c->b_info[s].n = n;
         c->b_info[s].prim_off = (int32_t)off;
         c->b_info[s].hits_off = hoff;
@@ -1577,7 +1596,7 @@ rf_status rf_segment_stacks(const rf_primitive *prims, int32_t n, const rf_bound
         if (bvs[b].objStartIndex >= 0 && bvs[b].objStartIndex <= n) cut[bvs[b].objStartIndex] = 1;
         if (bvs[b].objEndIndex >= 0 && bvs[b].objEndIndex <= n) cut[bvs[b].objEndIndex] = 1;
     }
-    mark_stacks(e.data(), n, tab.data(), bs.data(), cut);
+    mark_stacks(e.data(), n, tab.data(), bs.data(), scene_reach(bs.data(), n), cut);
     int32_t k = 0;
     for (int i = 0; i < n;) {
         int32_t ti, w;

@@ -124,6 +124,15 @@ template <class M> int trace_blocks_per_sm(const LaunchCfg &cfg);
 // (rf_culled.cuh; one translation unit per policy).
 template <class M> cudaError_t launch_culled(const TraceParams &p, bool bv, bool rec, int sms, cudaStream_t st);
 
+// Bounding sphere (centre, radius) of a mixed-precision surface under its record's
+// m, in place of box, the sphere around its object-space box, where that is larger
+// (a round surface's box adds up to sqrt 3): rings > 1: a cylinder stack of that
+// many; outer2: an annulus's, or a plate's, outer radius squared.  A frustum's rims
+// move out by what rounding can shift a root along a ray of length reach where its A
+// has lost the 12 bits that the FP32 test still accepts (kCondA).  loose_balls: keep
+// the box's sphere for spheres (RF_COMPAT_SPHERE's uncorrected discriminant).
+float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, double reach, bool loose_balls);
+
 // The culled kernel's tables of one scene (rf_bounds.cu): sph (n), a ball around
 // the points a surface can return as hits (squared radius in w, infinite when there
 // is no bound, negative for a frustum, whose bound holds outside its band, 0 for a
@@ -176,8 +185,8 @@ void emit_frame(const rf_primitive &e, float4 *out);
 // Host preparation of one scene for the batched kernel (rf_capi.cu); eps_out
 // receives the scene's self-hit threshold for the configured eps; returns the
 // number of segment stacks in the tables.
-int prepare_mixed_tables(const rf_primitive *prims, int n, float eps, rf_primitive *emit, HitRec *tab, float4 *bs,
-                         float *eps_out);
+int prepare_mixed_tables(const rf_primitive *prims, int n, float eps, uint32_t compat, rf_primitive *emit, HitRec *tab,
+                         float4 *bs, float *eps_out);
 
 // FP64 post-processing and probes (rf_kern_post.cu).
 cudaError_t launch_normalise_single(const unsigned long long *hits, const int64_t *rays, int n,
