@@ -7,8 +7,6 @@
 // binomial standard error sqrt(F(1-F)/rays) for the convergence loop.
 #include <algorithm>
 #include <cstdint>
-#include <utility>
-#include <vector>
 #include <cuda_runtime.h>
 
 #include "rf_internal.h"
@@ -177,34 +175,46 @@ __device__ __forceinline__ void atomic_max_double(double *a, double v)
 }
 
 // out2[0] = max_i |sum_j F_ij - 1|; out2[1] = max over pairs with both entries
-// non-zero of |A_i F_ij - A_j F_ji| / max(A_i F_ij, A_j F_ji).
-__global__ void check_F_kernel(const double *F, const double *areas, int n, double *out2)
+// non-zero of |A_i F_ij - A_j F_ji| / max(A_i F_ij, A_j F_ji).  Bound by FP64
+// operations (two a clock on an SM): each pair is looked at once, its ratio compared
+// by cross products and divided only at the end.  A block takes four rows, so that
+// the transposed entries it reads fill their 32-byte sectors.
+constexpr int kCheckRows = 4;
+__global__ void __launch_bounds__(256) check_F_kernel(const double *F, const double *areas, int n, double *out2)
 {
-    const int i = blockIdx.x;
-    double s = 0.0, worst = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double fij = F[(int64_t)i * n + j];
-        s += fij;
-        if (areas) {
-            const double fji = F[(int64_t)j * n + i];
-            const double a = areas[i] * fij, b = areas[j] * fji;
-            if (fij > 0.0 && fji > 0.0) worst = fmax(worst, fabs(a - b) / fmax(a, b));
+    const int r = threadIdx.x % kCheckRows, q = threadIdx.x / kCheckRows, i = blockIdx.x * kCheckRows + r;
+    double s = 0.0, num = 0.0, den = 1.0;
+    if (i < n) {
+        const double ai = areas ? areas[i] : 0.0;
+        for (int j = q; j < n; j += 256 / kCheckRows) {
+            const double fij = F[(int64_t)i * n + j];
+            s += fij;
+            if (areas && j > i && fij > 0.0) {
+                const double fji = F[(int64_t)j * n + i];
+                if (fji > 0.0) {
+                    const double a = ai * fij, b = areas[j] * fji, d = fabs(a - b), m = fmax(a, b);
+                    if (d * den > num * m) {
+                        num = d;
+                        den = m;
+                    }
+                }
+            }
         }
     }
     __shared__ double ss[256], sw[256];
     ss[threadIdx.x] = s;
-    sw[threadIdx.x] = worst;
+    sw[threadIdx.x] = num / den;
     __syncthreads();
-    for (int o = blockDim.x / 2; o; o >>= 1) {
+    for (int o = 128; o >= kCheckRows; o >>= 1) {
         if (threadIdx.x < o) {
             ss[threadIdx.x] += ss[threadIdx.x + o];
             sw[threadIdx.x] = fmax(sw[threadIdx.x], sw[threadIdx.x + o]);
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        atomic_max_double(&out2[0], fabs(ss[0] - 1.0));
-        atomic_max_double(&out2[1], sw[0]);
+    if (threadIdx.x < kCheckRows && i < n) {
+        atomic_max_double(&out2[0], fabs(ss[threadIdx.x] - 1.0));
+        atomic_max_double(&out2[1], sw[threadIdx.x]);
     }
 }
 
@@ -212,7 +222,7 @@ cudaError_t launch_check_F(const double *F, const double *areas, int n, double *
 {
     cudaError_t e = cudaMemsetAsync(out2, 0, 2 * sizeof(double), st);
     if (e != cudaSuccess) return e;
-    check_F_kernel<<<n, 256, 0, st>>>(F, areas, n, out2);
+    check_F_kernel<<<(n + kCheckRows - 1) / kCheckRows, 256, 0, st>>>(F, areas, n, out2);
     return cudaGetLastError();
 }
 
@@ -221,87 +231,195 @@ cudaError_t launch_check_F(const double *F, const double *areas, int n, double *
 // exactly for any symmetric G).  For a closed enclosure the rows must also sum
 // to 1: a symmetric scaling X G X with X = diag(x) keeps the symmetry, and x is
 // found by the symmetric Sinkhorn iteration x_i <- sqrt(x_i A_i / (G x)_i).
-__global__ void symmetrise_kernel(const double *F, const double *A, int n, double *G)
+//
+// One cooperative launch: block b owns a run of consecutive rows, keeps them in
+// shared memory when they fit (RES; n up to about 2000), forms G, iterates and writes
+// the scaled rows.  A round is n^2 FP64 multiply-adds (two a clock on an SM: 0.3 us
+// at n = 412 over the chip) and an exchange of x through L2, without a barrier: an
+// element is published with its round as one 16-byte word, and its readers wait for
+// the round they need.  Two buffers suffice: who publishes round r + 2 has read all of
+// round r + 1, so everyone has read round r.  A row's sum keeps the order of a
+// 256-thread block's tree (partial sums t, t + 256, ...; halves added), a warp holding
+// eight partials per lane; one warp then takes the roots of all rows of the block.
+// n = 412, 56 rounds: 0.22 ms (7400 clocks a round: 2600 row sums, 1700 root and
+// quotient, 3100 exchange), 0.34 for the call; as a launch and a memset per round with a
+// host check every eight, 0.38 ms of kernels and 0.85 for the call.
+struct SmoothState {
+    double final_err;
+    int iters;
+    int gave_up;  // some wait ran out of time
+};
+struct __align__(16) Tagged {
+    double v;
+    unsigned long long round;
+};
+
+__device__ __forceinline__ void publish(Tagged *p, double v, unsigned long long round)
 {
-    const int64_t total = (int64_t)n * n;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(k / n), j = (int)(k % n);
-        const double a = F[k], b = F[(int64_t)j * n + i];
-        const double fa = (a == a) ? a : 0.0, fb = (b == b) ? b : 0.0;  // rows without rays: 0
-        G[k] = 0.5 * (A[i] * fa + A[j] * fb);
-    }
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"(round)
+                 : "memory");
 }
 
-// one block per row: s_i = sum_j G_ij x_j, then x_i <- sqrt(x_i A_i / s_i);
-// err = max_i |x_i s_i / A_i - 1| before the update
-__global__ void sinkhorn_row_kernel(const double *G, const double *A, int n, const double *x_in, double *x_out,
-                                    double *err)
+// The value published for `round` at p; false after about two seconds (2^32 clocks)
+// without it, or when another wait gave up.
+__device__ __forceinline__ bool await(const Tagged *p, unsigned long long round, SmoothState *st, double &v)
 {
-    const int i = blockIdx.x;
-    double s = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) s += G[(int64_t)i * n + j] * x_in[j];
-    __shared__ double sh[256];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const double si = sh[0];
-        if (si > 0.0 && A[i] > 0.0) {
-            x_out[i] = sqrt(x_in[i] * A[i] / si);
-            const double e = fabs(x_in[i] * si / A[i] - 1.0);
-            atomicMax(reinterpret_cast<unsigned long long *>(err), (unsigned long long)__double_as_longlong(e));
-        } else {
-            x_out[i] = x_in[i];  // a surface that sees nothing keeps its row
+    long long bits, t0 = 0;
+    unsigned long long have;
+    for (int spin = 0;; ++spin) {
+        asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                     : "=l"(bits), "=l"(have)
+                     : "l"(p)
+                     : "memory");
+        if (have == round) break;
+        if (spin == 0) t0 = clock64();
+        if ((spin & 63) == 63 &&
+            (*reinterpret_cast<volatile int *>(&st->gave_up) || clock64() - t0 > (1ll << 32))) {
+            *reinterpret_cast<volatile int *>(&st->gave_up) = 1;
+            return false;
         }
     }
+    v = __longlong_as_double(bits);
+    return true;
 }
 
-__global__ void scale_out_kernel(const double *G, const double *A, const double *x, int n, int closed, double *F)
+constexpr int kSmoothThreads = 512;
+constexpr int kSmoothRows = 256;  // row sums of a pass: rows of a block are taken in runs of this many
+
+template <bool RES>
+__global__ void __launch_bounds__(kSmoothThreads, 1)
+    smooth_kernel(const double *F, const double *A, int n, int closed, int max_iter, double tol, double *G, double *xg,
+                  Tagged *xbuf, Tagged *ebuf, double *F_out, SmoothState *st)
 {
-    const int64_t total = (int64_t)n * n;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(k / n), j = (int)(k % n);
-        const double g = closed ? x[i] * G[k] * x[j] : G[k];
-        F[k] = A[i] > 0.0 ? g / A[i] : 0.0;
+    extern __shared__ double s_rows[];  // RES: this block's rows of G, then x
+    __shared__ double s_sum[kSmoothRows];
+    __shared__ double s_err[kSmoothThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kSmoothThreads / 32;
+    const int i0 = (int)((int64_t)n * blockIdx.x / gridDim.x), i1 = (int)((int64_t)n * (blockIdx.x + 1) / gridDim.x);
+    const int rows = i1 - i0;
+    double *g = RES ? s_rows : G + (int64_t)i0 * n;
+    double *x = RES ? s_rows + (int64_t)rows * n : xg + (int64_t)blockIdx.x * n;  // this block's copy of x
+    // rows fastest: the transposed entries of a block are contiguous
+    for (int64_t k = tid; k < (int64_t)rows * n; k += kSmoothThreads) {
+        const int j = (int)(k / rows), i = i0 + (int)(k % rows);
+        const double a = F[(int64_t)i * n + j], b = F[(int64_t)j * n + i];
+        const double fa = (a == a) ? a : 0.0, fb = (b == b) ? b : 0.0;  // rows without rays: 0
+        g[(int64_t)(i - i0) * n + j] = 0.5 * (A[i] * fa + A[j] * fb);
     }
-}
-
-cudaError_t launch_smooth(const double *F, const double *A, int n, int closed, int max_iter, double tol,
-                          double *G, double *x0, double *x1, double *err_dev, double *F_out, int *iters,
-                          double *final_err, cudaStream_t st)
-{
-    const int64_t total = (int64_t)n * n;
-    int grid = (int)std::min<int64_t>(4096, (total + 255) / 256);
-    symmetrise_kernel<<<grid, 256, 0, st>>>(F, A, n, G);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    *iters = 0;
-    *final_err = 0.0;
-    double *xa = x0, *xb = x1;
     if (closed) {
-        std::vector<double> ones(n, 1.0);
-        if ((e = cudaMemcpyAsync(xa, ones.data(), n * sizeof(double), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-            return e;
+        for (int j = tid; j < n; j += kSmoothThreads) x[j] = 1.0;
+        __syncthreads();
         for (int it = 0; it < max_iter; ++it) {
-            if ((e = cudaMemsetAsync(err_dev, 0, sizeof(double), st)) != cudaSuccess) return e;
-            sinkhorn_row_kernel<<<n, 256, 0, st>>>(G, A, n, xa, xb, err_dev);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            std::swap(xa, xb);
-            *iters = it + 1;
-            if ((it & 7) == 7 || it + 1 == max_iter) {
-                double h = 0.0;
-                if ((e = cudaMemcpyAsync(&h, err_dev, sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-                if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-                *final_err = h;
-                if (h <= tol) break;
+            const bool check = (it & 7) == 7 || it + 1 == max_iter;
+            const unsigned long long round = it + 1;
+            Tagged *xb = xbuf + (int64_t)(it & 1) * n, *eb = ebuf + (int64_t)((it >> 3) & 1) * n;
+            for (int r0 = 0; r0 < rows; r0 += kSmoothRows) {
+                const int cnt = min(kSmoothRows, rows - r0);
+                for (int r = warp; r < cnt; r += nwarps) {
+                    const double *gr = g + (int64_t)(r0 + r) * n;
+                    double p[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                    for (int b = lane; b < n; b += 256)  // eight independent loads and chains
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            if (b + 32 * k < n) p[k] += gr[b + 32 * k] * x[b + 32 * k];
+#pragma unroll
+                    for (int h = 4; h; h >>= 1)
+#pragma unroll
+                        for (int k = 0; k < h; ++k) p[k] += p[k + h];
+                    double s = p[0];
+#pragma unroll
+                    for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+                    if (lane == 0) s_sum[r] = s;
+                }
+                __syncthreads();
+                for (int r = tid; r < cnt; r += kSmoothThreads) {
+                    const int i = i0 + r0 + r;
+                    const double s = s_sum[r], xi = x[i], a = A[i];
+                    double xn = xi, e = 0.0;  // a surface that sees nothing keeps its row
+                    if (s > 0.0 && a > 0.0) {
+                        xn = sqrt(xi * a / s);
+                        if (check) e = fabs(xi * s / a - 1.0);
+                    }
+                    publish(xb + i, xn, round);
+                    if (check) publish(eb + i, e, round);
+                }
+                if (r0 + kSmoothRows < rows) __syncthreads();
+            }
+            __syncthreads();  // every row's sum is formed: x may change
+            bool ok = true;
+            double worst = 0.0;
+            for (int j = tid; j < n && ok; j += kSmoothThreads) {
+                double v = 0.0;
+                ok = await(xb + j, round, st, v);
+                x[j] = v;
+                if (check && ok) {
+                    ok = await(eb + j, round, st, v);
+                    worst = fmax(worst, v);
+                }
+            }
+            if (check) {
+#pragma unroll
+                for (int o = 16; o; o >>= 1) worst = fmax(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+                if (lane == 0) s_err[warp] = worst;
+            }
+            if (__syncthreads_or(!ok)) return;
+            if (check) {
+                double e = 0.0;
+#pragma unroll
+                for (int k = 0; k < nwarps; ++k) e = fmax(e, s_err[k]);
+                if (blockIdx.x == 0 && tid == 0) {
+                    st->iters = it + 1;
+                    st->final_err = e;
+                }
+                if (e <= tol) break;  // the same in every block
             }
         }
     }
-    scale_out_kernel<<<grid, 256, 0, st>>>(G, A, xa, n, closed, F_out);
-    return cudaGetLastError();
+    __syncthreads();
+    for (int64_t k = tid; k < (int64_t)rows * n; k += kSmoothThreads) {
+        const int r = (int)(k / n), j = (int)(k % n), i = i0 + r;
+        const double v = g[k];
+        F_out[(int64_t)i * n + j] = A[i] > 0.0 ? (closed ? x[i] * v * x[j] : v) / A[i] : 0.0;
+    }
+}
+
+// Workspace in bytes: two 16-byte-tagged buffers of x and of the errors, the state,
+// and, where a block's rows do not fit shared memory, G and the blocks' copies of x.
+static bool smooth_resident(int n, int grid)
+{
+    const size_t rows = (n + grid - 1) / grid;
+    return (rows + 1) * n * sizeof(double) <= 216 * 1024;
+}
+size_t smooth_bytes(int n, int sms)
+{
+    const int grid = std::min(n, sms);
+    const size_t tagged = 4 * (size_t)n * sizeof(Tagged) + 64;
+    return tagged + (smooth_resident(n, grid) ? 0 : ((size_t)n + grid) * n * sizeof(double));
+}
+
+cudaError_t launch_smooth(const double *F, const double *A, int n, int closed, int max_iter, double tol, void *work,
+                          double *F_out, int sms, int *iters, double *final_err, bool *gave_up, cudaStream_t st)
+{
+    const int grid = std::min(n, sms);
+    const bool resident = smooth_resident(n, grid);
+    Tagged *xbuf = static_cast<Tagged *>(work), *ebuf = xbuf + 2 * (size_t)n;
+    SmoothState *ds = reinterpret_cast<SmoothState *>(ebuf + 2 * (size_t)n);
+    double *G = reinterpret_cast<double *>(ds) + 8, *xg = G + (size_t)n * n;
+    cudaError_t e = cudaMemsetAsync(work, 0, 4 * (size_t)n * sizeof(Tagged) + 64, st);  // no round published
+    if (e != cudaSuccess) return e;
+    const size_t rows = (n + grid - 1) / grid, smem = resident ? (rows + 1) * n * sizeof(double) : 0;
+    const void *k = resident ? (const void *)smooth_kernel<true> : (const void *)smooth_kernel<false>;
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    void *args[] = {&F, &A, &n, &closed, &max_iter, &tol, &G, &xg, &xbuf, &ebuf, &F_out, &ds};
+    if ((e = cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kSmoothThreads), args, smem, st)) != cudaSuccess) return e;
+    SmoothState h{};
+    if ((e = cudaMemcpyAsync(&h, ds, sizeof h, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+    *iters = h.iters;
+    *final_err = h.final_err;
+    *gave_up = h.gave_up != 0;
+    return cudaSuccess;
 }
 
 // Eight independent FMA chains per thread: the FP32 issue roofline.
