@@ -31,6 +31,7 @@ UNITS = {
     "rf_culled_exact.cu": ["-fmad=false"],
     "rf_culled_f64.cu": ["-fmad=false"],
     "rf_culled_fast.cu": [],
+    "rf_culled_mixed.cu": [],
     "rf_kern_batched.cu": [],
     "rf_kern_post.cu": [],
     "rf_capi.cu": [],

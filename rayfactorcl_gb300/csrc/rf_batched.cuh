@@ -78,9 +78,6 @@ struct BatchSmem {
     int hist[kBatchHist];
     rf_primitive emit;
     float4 frame[kFrameWords];
-    HitRec bvtab[kBatchMaxBV];          // bounding surfaces (runBVGPU semantics)
-    int4 bvinfo[kBatchMaxBV];           // (settings, first child, end of children, 0)
-    float4 bvbs[kBatchMaxBV];           // their bounding spheres, squared widened radius in w
     int64_t chunk;
     unsigned long long bar;             // mbarrier of the bulk copies of the scene tables
     int next_packet;
@@ -661,14 +658,11 @@ __device__ __forceinline__ int resolve_brute(int bi, bool deferred, int lo, int 
 // The bounding-surface walk of runBVGPU (RayFactorGPU.cl:580-619) for one ray:
 // surfaces w = 0..nbv-1 in order, each tested in mixed precision (FP64 when
 // ill-conditioned); find(lo, hi) is the ray's nearest hit among the children
-// [lo, hi) (findObject, :445-472).  bvbs: the surfaces' bounding spheres.  A ray
-// needs its children's hit only when w is nearer than its best so far, so find()
-// runs only then: WARP (find() is
-// warp-wide, every lane here): when that holds in some lane of the warp, in
-// every lane, so the warp-wide steps stay in step; else per lane.  stale:
-// RF_COMPAT_BV_STALE, where a plain bounding surface that becomes the nearest
-// keeps the child found under an earlier one (:596-619).
-template <bool WARP, class Find>
+// [lo, hi) (findObject, :445-472), looked for only when w is nearer than the best so
+// far.  bvbs: the surfaces' bounding spheres.  stale: RF_COMPAT_BV_STALE, where a
+// plain bounding surface that becomes the nearest keeps the child found under an
+// earlier one (:596-619).
+template <class Find>
 __device__ __forceinline__ int bv_select(const HitRec *bvtab, const int4 *bvinfo, const float4 *bvbs, int nbv,
                                          const Ray<float> &ray, float eps, bool sc, bool stale, Find find)
 {
@@ -676,28 +670,22 @@ __device__ __forceinline__ int bv_select(const HitRec *bvtab, const int4 *bvinfo
     int bvi = -1, obj = -1, nb = -1;  // nb: children's nearest hit of the current winner bvi
     const float idd = MFast::rcp(ray.cx * ray.cx + ray.cy * ray.cy + ray.cz * ray.cz);
     for (int w = 0; w < nbv; ++w) {
-        // a ray that cannot reach w's bounding sphere misses w (t = inf: nothing changes);
-        // the warp skips w when that holds in every lane
-        const bool may = ray_may_hit(ray, idd, bvbs[w]);
-        if (WARP ? !__any_sync(0xffffffffu, may) : !may) continue;
+        if (!ray_may_hit(ray, idd, bvbs[w])) continue;  // misses w
         const HitRec hb = bvtab[w];
         bool defer = false;
         float t = hit_mixed(__float_as_int(hb.aux.x), hb, ray, eps, sc, defer);
         if (defer) t = hit_f64(hb, ray, eps, sc);
+        if (!(t < tbest)) continue;
         const int4 info = bvinfo[w];
-        const bool nearer = t < tbest;
-        const bool run = WARP ? __any_sync(0xffffffffu, nearer) : nearer;
-        const int nw = run ? find(info.y, info.z) : -1;  // used only when nearer
-        if (nearer) {
-            if (info.x == 1) {  // test the children at once; the surface counts only if one is hit
-                obj = nw;
-                if (nw != -1) { tbest = t; bvi = w; nb = nw; }
-            } else {
-                tbest = t;
-                bvi = w;
-                nb = nw;
-                if (!stale) obj = -1;
-            }
+        const int nw = find(info.y, info.z);
+        if (info.x == 1) {  // test the children at once; the surface counts only if one is hit
+            obj = nw;
+            if (nw != -1) { tbest = t; bvi = w; nb = nw; }
+        } else {
+            tbest = t;
+            bvi = w;
+            nb = nw;
+            if (!stale) obj = -1;
         }
     }
     if (bvi != -1 && obj == -1) obj = nb;  // the winner's children
@@ -707,11 +695,9 @@ __device__ __forceinline__ int bv_select(const HitRec *bvtab, const int4 *bvinfo
 // RESIDENT: every scene of the launch fits the shared-memory tables
 // (n <= kBatchTile); otherwise surfaces are read through L1.  COUNT: also count
 // the tests by surface type, the candidates and the packets (p.work); the
-// counters cost a few per cent, so timed runs leave them out.  BV: one resident
-// scene with bounding surfaces (p.bvtab, p.bvinfo, p.nbv <= kBatchMaxBV) traced
-// with runBVGPU's semantics (bv_select).  STK: some scene has segment stacks
-// (kStackType records); the candidate loops then test a stack once.
-template <bool REC, bool RESIDENT, bool COUNT, bool BV, bool STK>
+// counters cost a few per cent, so timed runs leave them out.  STK: some scene
+// has segment stacks (kStackType records); the candidate loops then test a stack once.
+template <bool REC, bool RESIDENT, bool COUNT, bool STK>
 __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TraceParams p)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -796,14 +782,6 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
                     }
                     staged = true;
                 }
-                if (BV) {
-                    for (int i = tid; i < 4 * p.nbv; i += blockDim.x)
-                        reinterpret_cast<float4 *>(S.bvtab)[i] = __ldg(reinterpret_cast<const float4 *>(p.bvtab) + i);
-                    for (int i = tid; i < p.nbv; i += blockDim.x) {
-                        S.bvinfo[i] = __ldg(p.bvinfo + i);
-                        S.bvbs[i] = __ldg(p.bvsph + i);
-                    }
-                }
                 cur_scene = sg.scene;
             }
             if (tid < (int)(sizeof(rf_primitive) / 4))
@@ -850,31 +828,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
                     const int64_t rid = gid * 4 + v;
                     const bool valid = rid >= sg.ray_begin && rid < sg.ray_end;
                     int bi = -1;
-                    if (valid && BV) {
-                        float r[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) r[i] = uf[(i + v + 1) & 3];
-                        const Ray<float> ray = emit_mixed(S.emit, S.frame, r);
-                        auto find = [&](int lo, int hi) {  // every child of [lo, hi), index order
-                            float tr = MFast::inf();
-                            int br = -1;
-                            bool dr = false;
-                            for (int j = lo; j < hi; ++j) {
-                                if (j == skip) continue;
-                                const HitRec h = S.tab[j];
-                                const int type = __float_as_int(h.aux.x);
-                                bool defer = false;
-                                int idx;
-                                const float t = test_mixed<STK>(type, h, j, S.tab, true, ray, eps, sc, defer, idx);
-                                if (t < tr) { tr = t; br = idx; }
-                                dr |= defer;
-                                if (STK && is_stack(type)) j = stack_end(h, j) - 1;
-                            }
-                            return resolve_brute<STK>(br, dr, lo, hi, true, S.tab, gtab, ray, eps, sc, skip, nref);
-                        };
-                        bi = bv_select<false>(S.bvtab, S.bvinfo, S.bvbs, p.nbv, ray, eps, sc,
-                                              (p.compat & RF_COMPAT_BV_STALE) != 0, find);
-                    } else if (valid) {
+                    if (valid) {
                         float r[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) r[i] = uf[(i + v + 1) & 3];
@@ -1035,71 +989,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
                 const Ray<float> ray = emit_mixed(S.emit, S.frame, r);
                 const float idd = MFast::rcp(ray.cx * ray.cx + ray.cy * ray.cy + ray.cz * ray.cz);
                 const uint32_t *mcell = mrow ? mrow + (int64_t)ray_key(ray, r) * nwords_all : nullptr;
-                if constexpr (BV) {
-                    // runBVGPU: the nearest child in each bounding surface's range with the
-                    // packet's culled candidate loop restricted to the range, then the walk
-                    const int skip = self_skip(S.emit, cur_emitter);
-                    if (COUNT && lane == 0) S.wcount[warp][7] += 1;
-                    unsigned cmask = 0u;  // without masks: lane w holds candidate word w (n <= kBatchTile)
-                    if (!mcell) {
-                        const Packet pk = packet_bounds(ray, idd);
-#pragma unroll 1
-                        for (int w = 0; w < nwords_all; ++w) {
-                            const int js = (w << 5) + lane;
-                            const bool cand = js < si.n && packet_may_hit(pk, S.bs[js]);
-                            const unsigned cm = __ballot_sync(0xffffffffu, cand);
-                            if (lane == w) cmask = cm;
-                        }
-                    }
-                    auto find = [&](int lo, int hi) {  // warp-wide: every lane, same lo and hi
-                        float tr = MFast::inf();
-                        int br = -1, dr = -1, nd = 0, skip_to = lo;
-#pragma unroll 1
-                        for (int w = lo >> 5; lo < hi && w <= (hi - 1) >> 5; ++w) {
-                            const int jw = w << 5;
-                            unsigned cm = mcell ? __reduce_or_sync(0xffffffffu, __ldg(mcell + w))
-                                                : __shfl_sync(0xffffffffu, cmask, w);
-                            cm &= keep_from((STK ? skip_to : lo) - jw);  // lo, and stacks tested in an earlier word
-                            if (hi < jw + 32) cm &= (1u << (hi - jw)) - 1u;
-                            if (skip >= jw && skip < jw + 32) cm &= ~(1u << (skip - jw));
-                            while (cm) {
-                                const int j = jw + __ffs(cm) - 1;
-                                cm &= cm - 1;
-                                if (COUNT && lane == 0) S.wcount[warp][6] += 1;  // candidates checked
-                                if (!__any_sync(0xffffffffu, ray_may_hit(ray, idd, S.bs[j]))) continue;
-                                const HitRec h = S.tab[j];
-                                const int type = __float_as_int(h.aux.x);
-                                if (COUNT) tcount += lane == stat_type(type) ? nvalid : 0;
-                                bool defer = false;
-                                int idx = j;
-                                unsigned nb = 0u;
-                                const float t = STK ? hit_hot(type, h, j, S.tab, true, ray, eps, sc, defer, idx, jw, cm,
-                                                              skip_to, hi, nb)
-                                                    : hit_mixed(type, h, ray, eps, sc, defer);
-                                if (t < tr) { tr = t; br = idx; }
-                                nd += defer;
-                                dr = defer ? j : dr;
-                            }
-                        }
-                        // as below: nearest among the children the lane's own gate admits
-                        bool again = valid && nd > 1;
-                        if (valid && nd == 1) {
-                            int dq;
-                            const float t = test_f64<STK>(S.tab[dr], dr, ray, eps, sc, dq);
-                            if (t < tr || (t == tr && br >= 0 && dq < br)) { tr = t; br = dq; }
-                            ++nref;
-                            again = !own_gate(mcell, dr, ray, idd, S.bs[dr]);
-                        }
-                        if (valid && !again && br >= 0) again = !own_gate(mcell, br, ray, idd, S.bs[br]);
-                        if (again) {
-                            br = retrace_f64<STK>(lo, hi, true, S.tab, gtab, S.bs, gbs, mcell, true, ray, idd, eps, sc, skip,
-                                             nref);
-                        }
-                        return br;
-                    };
-                    bi = bv_select<true>(S.bvtab, S.bvinfo, S.bvbs, p.nbv, ray, eps, sc, (p.compat & RF_COMPAT_BV_STALE) != 0,
-                                         find);
-                } else {
+                {
                     float tb = MFast::inf();
                     int dj = -1, ndef = 0;  // deferred FP64 tests of this lane: the last one, and how many
                     if (COUNT && lane == 0) S.wcount[warp][7] += 1;

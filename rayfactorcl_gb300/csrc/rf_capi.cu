@@ -926,7 +926,7 @@ int batched_grid(rf_ctx *c, bool rec)
 
 // One persistent launch over host-planned segments.
 rf_status run_batched(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec,
-                      int32_t *d_rec, int64_t rec_base, bool zero_hits, bool bv = false)
+                      int32_t *d_rec, int64_t rec_base, bool zero_hits, bool bv = false, int chunk_draws = 0)
 {
     c->last_small = false;
     c->last_launches = 0;
@@ -943,12 +943,16 @@ rf_status run_batched(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_
     p.rec_base = rec_base;
     const int grid = (int)std::min<int64_t>(batched_grid(c, rec), total_chunks);
     RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    if (bv) {
+    if (chunk_draws > 0) {  // the culled kernel
         p.bvtab = c->b_bvtab.as<HitRec>();
         p.bvinfo = c->b_bvinfo.as<int4>();
         p.bvsph = c->b_bvsph.as<float4>();
         p.nbv = c->nbv;
-        RF_CUDA(c, launch_batched_bv(p, rec, c->cfg.work_counts != 0, c->b_stacks > 0, grid, c->stream));
+        p.n = c->n;
+        p.eps = c->b_info[0].eps;
+        p.chunk_draws = chunk_draws;
+        p.use_smem_hist = 1;
+        RF_CUDA(c, launch_mixed_culled(p, bv, rec, c->cfg.work_counts != 0, grid, c->stream));
     } else {
         RF_CUDA(c, launch_batched(p, rec, batch_resident(c), c->cfg.work_counts != 0, c->b_stacks > 0, grid,
                                   c->stream));
@@ -970,22 +974,37 @@ bool use_small(const rf_ctx *c)
     return c->n <= kSmallDefaultMax;
 }
 
-int small_gpt(const rf_ctx *c, bool rec)
+// The small-scene kernel for this trace (with bounding surfaces by size alone).
+bool small_trace(const rf_ctx *c, bool bv)
 {
-    if (rec) return 1;
+    return bv ? c->b_single && c->n <= kSmallDefaultMax : use_small(c);
+}
+
+int small_gpt(const rf_ctx *c, bool rec, bool bv = false)
+{
+    if (rec || bv) return 1;
     if (c->gpt > 0) return c->gpt == 2 ? 2 : 1;
     return c->cfg.rays_per_thread == 8 ? 2 : 1;
 }
 
-int64_t mixed_chunk_draws(const rf_ctx *c, bool rec, bool bv)
+// Single scenes that the culled kernel traces in MIXED precision: with bounding
+// surfaces, and with segment stacks, whose members it need not look at.
+bool mixed_culled(const rf_ctx *c, bool bv)
 {
-    return !bv && use_small(c) ? (int64_t)kSmallThreads * small_gpt(c, rec) : (int64_t)kBatchChunkDraws;
+    return !small_trace(c, bv) && (bv || (c->b_stacks > 0 && c->n <= kBatchTile));
+}
+
+// Draws per chunk of a MIXED trace of so many draws.
+int64_t mixed_chunk_draws(const rf_ctx *c, bool rec, bool bv, int64_t draws)
+{
+    if (mixed_culled(c, bv)) return culled_chunk(c, draws);
+    return small_trace(c, bv) ? (int64_t)kSmallThreads * small_gpt(c, rec, bv) : (int64_t)kBatchChunkDraws;
 }
 
 // One launch of the small-scene kernel over host-planned segments (chunks of
 // kSmallThreads * gpt draws) of the scene held in the batch tables.
 rf_status run_small(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec, int32_t *d_rec,
-                    int64_t rec_base, bool zero_hits)
+                    int64_t rec_base, bool zero_hits, bool bv)
 {
     c->last_launches = 0;
     c->timed = false;
@@ -1016,12 +1035,20 @@ rf_status run_small(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
     p.total_chunks = total_chunks;
     p.rec = d_rec;
     p.rec_base = rec_base;
-    const int gpt = small_gpt(c, rec);
-    int bps = mixed_small_blocks_per_sm(gpt, rec);
+    const int gpt = small_gpt(c, rec, bv);
+    int bps = bv ? 4 : mixed_small_blocks_per_sm(gpt, rec);
     if (bps <= 0) bps = 1;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sms * bps, total_chunks));
     RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    RF_CUDA(c, launch_mixed_small(p, gpt, rec, grid, c->stream));
+    if (bv) {
+        p.bvtab = c->b_bvtab.as<HitRec>();
+        p.bvinfo = c->b_bvinfo.as<int4>();
+        p.bvsph = c->b_bvsph.as<float4>();
+        p.nbv = c->nbv;
+        RF_CUDA(c, launch_mixed_small_bv(p, rec, grid, c->stream));
+    } else {
+        RF_CUDA(c, launch_mixed_small(p, gpt, rec, grid, c->stream));
+    }
     RF_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     c->last_launches = 1;
     c->timed = true;
@@ -1031,10 +1058,10 @@ rf_status run_small(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
 // A MIXED trace of the single scene: small-scene or batched kernel; with its
 // bounding surfaces (runBVGPU semantics), the batched kernel's BV variant.
 rf_status run_mixed(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec, int32_t *d_rec,
-                    int64_t rec_base, bool zero_hits, bool bv)
+                    int64_t rec_base, bool zero_hits, bool bv, int64_t chunk_draws)
 {
-    if (bv) return run_batched(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, true);
-    if (use_small(c)) return run_small(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits);
+    if (mixed_culled(c, bv)) return run_batched(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, bv, (int)chunk_draws);
+    if (small_trace(c, bv)) return run_small(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, bv);
     return run_batched(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits);
 }
 
@@ -1292,9 +1319,9 @@ rf_status rf_trace_async(rf_ctx *c, const int64_t *rays, int32_t use_bv)
         if (!c->b_single) return fail(c, RF_ERR_STATE, "scene not prepared for the mixed kernel");
         std::vector<Segment> seg;
         int64_t chunks = 0;
-        const int64_t cg = mixed_chunk_draws(c, false, use_bv != 0);
+        const int64_t cg = mixed_chunk_draws(c, false, use_bv != 0, total_draws(rays, c->n));
         for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, 0, rays[e], cg, chunks);
-        if ((s = run_mixed(c, seg, chunks, false, nullptr, 0, true, use_bv != 0)) != RF_OK) return s;
+        if ((s = run_mixed(c, seg, chunks, false, nullptr, 0, true, use_bv != 0, cg)) != RF_OK) return s;
         c->have_results = true;
         return RF_OK;
     }
@@ -1335,14 +1362,14 @@ rf_status rf_trace_range(rf_ctx *c, const int64_t *first_ray, const int64_t *cou
     const int64_t draws = total_draws(count, c->n);
     if (c->cull == 0 && culled_pays(c, use_bv != 0, draws) && (s = ensure_culled(c)) != RF_OK) return s;
     Plan pl = make_plan(c, use_bv != 0, false, draws);
-    const int64_t chunk_gids = mixed ? mixed_chunk_draws(c, false, use_bv != 0) : pl.chunk_gids();
+    const int64_t chunk_gids = mixed ? mixed_chunk_draws(c, false, use_bv != 0, draws) : pl.chunk_gids();
     for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, first_ray[e], count[e], chunk_gids, chunks);
     if (!accumulate) c->last_rays.assign(c->n, 0);
     for (int e = 0; e < c->n; ++e) c->last_rays[e] += count[e];
     c->have_results = false;
     if (mixed) {
         if (!c->b_single) return fail(c, RF_ERR_STATE, "scene not prepared for the mixed kernel");
-        s = run_mixed(c, seg, chunks, false, nullptr, 0, !accumulate, use_bv != 0);
+        s = run_mixed(c, seg, chunks, false, nullptr, 0, !accumulate, use_bv != 0, chunk_gids);
     } else {
         s = run_trace(c, seg, chunks, pl, nullptr, 0, !accumulate);
     }
@@ -1453,9 +1480,9 @@ rf_status rf_trace_rays(rf_ctx *c, int32_t emitter, int64_t first_ray, int64_t n
     if (c->cfg.precision == RF_PREC_MIXED) {
         if (use_bv && (s = check_mixed_bv(c)) != RF_OK) return s;
         std::vector<Segment> seg;
-        const int64_t chunks =
-            plan_segments(seg, emitter, 0, first_ray, n_rays, mixed_chunk_draws(c, true, use_bv != 0), 0);
-        if ((s = run_mixed(c, seg, chunks, true, c->d_rec.as<int32_t>(), first_ray, false, use_bv != 0)) != RF_OK)
+        const int64_t cg = mixed_chunk_draws(c, true, use_bv != 0, (n_rays + 3) / 4);
+        const int64_t chunks = plan_segments(seg, emitter, 0, first_ray, n_rays, cg, 0);
+        if ((s = run_mixed(c, seg, chunks, true, c->d_rec.as<int32_t>(), first_ray, false, use_bv != 0, cg)) != RF_OK)
             return s;
     } else {
         const int64_t draws = (n_rays + 3) / 4;

@@ -28,10 +28,13 @@
 // What bounds it: FP32 issue, like the batched mixed-precision kernel whose
 // structure it shares; in MF64 the FP64 pipe.  64 surfaces, EXACT, 1e8 rays: 5.9 ms
 // (plain 18.2), of which draws, keys and sort 0.6, emission and packet bounds 1.3,
-// the spheres 2.2 (11 candidates per packet) and the tests 1.7 (5.3 per packet, of
+// the spheres 2.2 (9 candidates per packet) and the tests 1.7 (5.3 per packet, of
 // which 2.4 find a hit for some ray; the plain kernel makes 64 per ray).  The
-// furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.15 ms EXACT
-// (plain 7.9), 1.0 FAST (5.7); 1e6 rays in FP64 2.2 (35.4).
+// furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.10 ms EXACT
+// (plain 7.9), 0.84 FAST (5.7); 1e6 rays in FP64 2.3 (35.4).  In mixed precision, 5e7
+// rays: 2.55 ms with bounding surfaces (3.36 as a variant of the batched kernel, which
+// spilled 600 bytes a thread), 1.99 without (2.30); the reference's furnace model,
+// 2e7 rays, 0.96 (1.65).
 #pragma once
 
 #include "rf_trace_kernels.cuh"
@@ -41,9 +44,11 @@ namespace rf {
 
 // Shared memory of a block: arrays sized by the launch's chunk (cd draws), the
 // surfaces kept resident (nres, 0: read through L1), the histogram row (nhist,
-// 0: global tallies) and the bounding surfaces (nbv).
+// 0: global tallies) and the bounding surfaces (nbv).  live: the surfaces that can be
+// candidates, in index order (a stack's first member stands for all), with bs in the
+// same order: a furnace's 252 surfaces are 35.
 struct CulledLayout {
-    int cnt, perm, unif, tab, bs, bvtab, bvinfo, bvbs, hist, bytes;
+    int cnt, perm, unif, tab, bs, bvtab, bvinfo, bvbs, hist, live, bytes;
     __host__ __device__ CulledLayout(int cd, int nres, int nhist, int nbv)
     {
         cnt = 0;
@@ -55,7 +60,8 @@ struct CulledLayout {
         bvinfo = bvtab + nbv * (int)sizeof(HitRec);
         bvbs = bvinfo + nbv * 16;
         hist = bvbs + nbv * 16;
-        bytes = hist + nhist * 4;
+        live = hist + nhist * 4;
+        bytes = live + (nres * 2 + 15) / 16 * 16;
     }
 };
 
@@ -296,22 +302,61 @@ __device__ __forceinline__ void plate_hits(const HitRec &h, const HitRec *tab, b
     }
 }
 
+// The mixed-precision arithmetic (emit_mixed, test_mixed with FP64 for an
+// ill-conditioned quadric at once) over the mixed tables; used for scenes with
+// bounding surfaces.
+struct MMixed : MFast {};
+template <class M> constexpr bool kIsMixed = false;
+template <> constexpr bool kIsMixed<MMixed> = true;
+
+// FP64 evaluation of surface j's deferred test (record in shared or global memory):
+// t and, in y, the bits of the surface hit.  By value, so that the hot loop's ray and
+// record stay in registers.
+static __device__ __noinline__ float2 deferred_f64(const HitRec *rec, int j, Ray<float> w, float eps, bool sc)
+{
+    const HitRec h = *rec;
+    int idx;
+    const float t = test_f64<true>(h, j, w, eps, sc, idx);
+    return make_float2(t, __int_as_float(idx));
+}
+
+// A bounding surface's test, out of line: one call or two per packet, and a second
+// inlined set of the six tests overflows the instruction cache.
+template <class M>
+static __device__ __noinline__ typename M::T shell_hit(const HitRec *rec, Ray<typename M::T> w, typename M::T eps,
+                                                       bool sc)
+{
+    const HitRec h = *rec;
+    const int type = __float_as_int(h.aux.x);
+    if constexpr (kIsMixed<M>) {
+        bool defer = false;
+        float t = hit_mixed(type, h, w, eps, sc, defer);
+        if (defer) t = hit_f64(h, w, eps, sc);
+        return t;
+    } else {
+        return hit_any<M>(type, h, w, eps, sc, M::inf());
+    }
+}
+
 // BV: runBVGPU's walk (RayFactorGPU.cl:530-626) over at most kBatchMaxBV
 // bounding surfaces; RESIDENT: the surfaces stay in shared memory (n <=
-// kBatchTile; always so with BV); REC: write hit indices instead of tallying.
-template <class M, int THREADS, bool BV, bool REC, bool RESIDENT>
+// kBatchTile; always so with BV); REC: write hit indices instead of tallying;
+// COUNT: also the work counters (p.work: tests by type, candidates, packets).
+template <class M, int THREADS, bool BV, bool REC, bool RESIDENT, bool COUNT>
 __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
 {
     using T = typename M::T;
+    constexpr bool kMixed = kIsMixed<M>;
     constexpr int kPer = kCells / THREADS;                 // buckets per thread of the scan
     constexpr int kMaxG = kChunkDraws / THREADS;           // draws per thread of the largest chunk
     static_assert(THREADS % 32 == 0 && kPer % 4 == 0, "scan shape");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ rf_primitive s_emit;
     __shared__ float4 s_frame[3];
+    __shared__ float4 s_mframe[kMixed ? kFrameWords : 1];  // mixed: the planar emitter's FP64 frame
     __shared__ int s_wsum[THREADS / 32];
     __shared__ int64_t s_chunk;
-    __shared__ int s_next, s_nvalid;
+    __shared__ int s_next, s_nvalid, s_nlive;
 
     const int n = p.n, cd = p.chunk_draws;
     const bool hist = !REC && p.use_smem_hist;
@@ -325,6 +370,7 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
     int4 *s_bvinfo = reinterpret_cast<int4 *>(smem_raw + lay.bvinfo);
     float4 *s_bvbs = reinterpret_cast<float4 *>(smem_raw + lay.bvbs);
     int *s_hist = reinterpret_cast<int *>(smem_raw + lay.hist);
+    uint16_t *s_live = reinterpret_cast<uint16_t *>(smem_raw + lay.live);
     const HitRec *tab = RESIDENT ? s_tab : p.tab;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -334,13 +380,45 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
     if (RESIDENT) {
         for (int i = tid; i < 4 * n; i += THREADS)
             reinterpret_cast<float4 *>(s_tab)[i] = __ldg(reinterpret_cast<const float4 *>(p.tab) + i);
-        for (int i = tid; i < n; i += THREADS) s_bs[i] = __ldg(p.bsph + i);
+        if (warp == 0) {
+            int m = 0;
+            for (int i0 = 0; i0 < n; i0 += 32) {
+                const int i = i0 + lane;
+                float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (i < n) {
+                    b = __ldg(p.bsph + i);
+                    if (kMixed) {  // (the plain arithmetics' tables have w = 0 for a stack's later members)
+                        const float4 aux = __ldg(&p.tab[i].aux);
+                        if (is_stack(__float_as_int(aux.x)) && (__float_as_int(aux.w) & 0xffff)) b.w = 0.0f;
+                    }
+                }
+                const unsigned on = __ballot_sync(0xffffffffu, b.w != 0.0f);
+                if (b.w != 0.0f) {
+                    const int k = m + __popc(on & ((1u << lane) - 1u));
+                    s_live[k] = (uint16_t)i;
+                    s_bs[k] = b;
+                }
+                m += __popc(on);
+            }
+            if (lane == 0) s_nlive = m;
+        }
+        __syncthreads();
     }
+    const int nc = RESIDENT ? s_nlive : n;  // candidate positions
+    auto surface = [&](int q) { return RESIDENT ? (int)s_live[q] : q; };
     if (BV) {
         for (int i = tid; i < 4 * p.nbv; i += THREADS)
             reinterpret_cast<float4 *>(s_bvtab)[i] = __ldg(reinterpret_cast<const float4 *>(p.bvtab) + i);
         for (int i = tid; i < p.nbv; i += THREADS) {
-            s_bvinfo[i] = __ldg(p.bvinfo + i);
+            int4 info = __ldg(p.bvinfo + i);  // children as positions
+            int lo = 0, hi = 0;
+            for (int q = 0; q < nc; ++q) {
+                lo += s_live[q] < info.y;
+                hi += s_live[q] < info.z;
+            }
+            info.y = lo;
+            info.z = hi;
+            s_bvinfo[i] = info;
             s_bvbs[i] = __ldg(p.bvsph + i);
         }
     }
@@ -348,6 +426,9 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
         for (int i = tid; i < n; i += THREADS) s_hist[i] = 0;
 
     int emitter = -1;
+    int skip = -1;       // mixed: a planar emitter, which its own rays cannot hit
+    int nref = 0;        // mixed: FP64 evaluations
+    uint32_t tcount = 0; // COUNT: lane t < 6 tests of type t, lane 6 candidates, lane 7 packets (this chunk)
     int row_chunks = 0;  // chunks in the shared-memory row since its last flush
     auto flush = [&]() {
         __syncthreads();
@@ -377,7 +458,9 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                 if (tid < (int)(sizeof(rf_primitive) / 4))
                     reinterpret_cast<float *>(&s_emit)[tid] = reinterpret_cast<const float *>(p.emit + sg.emitter)[tid];
                 if (tid == 32 % THREADS) quick_frame(p.emit[sg.emitter], s_frame);
+                if (kMixed && tid < kFrameWords) s_mframe[tid] = p.frame[(int64_t)sg.emitter * kFrameWords + tid];
                 emitter = sg.emitter;
+                if (kMixed) skip = planar(p.emit[emitter].type) ? emitter : -1;
             }
         }
         for (int i = tid; i < kCells; i += THREADS) cnt[i] = 0;
@@ -484,8 +567,13 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                     const int q = (i + v + 1) & 3;
                     r[i] = q == 0 ? uf[0] : (q == 1 ? uf[1] : (q == 2 ? uf[2] : uf[3]));
                 }
-                ray = emit_ray<M>(s_emit, r);
+                if constexpr (kMixed)
+                    ray = emit_mixed(s_emit, s_mframe, r);
+                else
+                    ray = emit_ray<M>(s_emit, r);
             }
+            const int nvalid = COUNT ? __popc(__ballot_sync(0xffffffffu, valid)) : 0;  // every lane
+            if (COUNT && lane == 7) ++tcount;
             const Ray<float> rf = to_f32(ray);
             const float cc = dot3(rf.cx, rf.cy, rf.cz, rf.cx, rf.cy, rf.cz);
             // a ray the bounds do not speak for: its packet tests everything
@@ -495,25 +583,26 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
             Packet pk = bounds_of(rf, idd);
             pk.cull = pk.cull && !odd;
 
-            // candidate words of the 1024 surfaces from j0 on, lane w holding word w: by
+            // candidate words of the 1024 positions from q0 on, lane w holding word w: by
             // sphere (cmask), and frusta in whose band some ray of the packet lies (bmask)
             unsigned cmask = 0u, bmask = 0u;
-            auto candidates = [&](int j0) {
-                const int nwords = min(32, (n - j0 + 31) >> 5);
+            auto candidates = [&](int q0) {
+                const int nwords = min(32, (nc - q0 + 31) >> 5);
 #pragma unroll 1
                 for (int w = 0; w < nwords; ++w) {
-                    const int jw = j0 + (w << 5), js = jw + lane;
+                    const int qw = q0 + (w << 5), q = qw + lane;
                     bool cand = false, banded = false;
-                    if (js < n) {
-                        const float4 b = RESIDENT ? s_bs[js] : __ldg(p.bsph + js);
-                        cand = b.w != 0.0f && (!pk.cull || packet_reaches(pk, b));
-                        if (b.w < 0.0f) banded = pk.cull && packet_band(p.cquad, js, pk);
+                    if (q < nc) {
+                        const float4 b = RESIDENT ? s_bs[q] : __ldg(p.bsph + q);
+                        cand = (RESIDENT || b.w != 0.0f) && (!pk.cull || packet_reaches(pk, b));
+                        if (kMixed) cand = cand && surface(q) != skip;
+                        if (!kMixed && b.w < 0.0f) banded = pk.cull && packet_band(p.cquad, surface(q), pk);
                     }
                     const unsigned cm = __ballot_sync(0xffffffffu, cand);
-                    unsigned bm = __ballot_sync(0xffffffffu, banded);
+                    unsigned bm = kMixed ? 0u : __ballot_sync(0xffffffffu, banded);
                     for (unsigned todo = bm; todo; todo &= todo - 1) {  // warp-uniform
                         const int b_ = __ffs(todo) - 1;
-                        if (!__any_sync(0xffffffffu, band(p.cquad, jw + b_, rf, cc))) bm &= ~(1u << b_);
+                        if (!__any_sync(0xffffffffu, band(p.cquad, surface(qw + b_), rf, cc))) bm &= ~(1u << b_);
                     }
                     if (lane == w) {
                         cmask = cm;
@@ -521,13 +610,30 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                     }
                 }
             };
-            // can the lane's ray be hit by surface j (a packet's sphere candidate)
-            auto gate = [&](int j) {
-                return odd || reaches(rf, idd, RESIDENT ? s_bs[j] : __ldg(p.bsph + j));
+            // can the lane's ray be hit by the surface at q (a packet's sphere candidate)
+            auto gate = [&](int q) {
+                return odd || reaches(rf, idd, RESIDENT ? s_bs[q] : __ldg(p.bsph + q));
             };
             auto test = [&](int j, T &tb, int &bi) {  // every lane, the same j
                 const HitRec h = RESIDENT ? s_tab[j] : load_rec(p.tab, j);
                 const int type = __float_as_int(h.aux.x);
+                if (COUNT) tcount += lane == (kMixed ? stat_type(type) : type) ? nvalid : 0;
+                if constexpr (kMixed) {
+                    bool defer = false;
+                    int idx;
+                    float t = test_mixed<true>(type, h, j, tab, RESIDENT, ray, eps, sc, defer, idx);
+                    if (__any_sync(0xffffffffu, defer) && defer) {
+                        const float2 q = deferred_f64(tab + j, j, ray, eps, sc);
+                        t = q.x;
+                        idx = __float_as_int(q.y);
+                        nref += valid;
+                    }
+                    if (t < tb) {
+                        tb = t;
+                        bi = idx;
+                    }
+                    return;
+                }
                 const unsigned m = (unsigned)__float_as_int(h.aux.w);
                 if (m) {  // the first of a stack of m surfaces: one search for all of them
                     if (type == RF_ANNULUS)
@@ -542,26 +648,26 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                     }
                 }
             };
-            // nearest hit among the candidates of [lo, hi) within the words of j0, in index order
-            auto search = [&](int j0, int lo, int hi, T &tb, int &bi) {
+            // nearest hit among the candidates of positions [lo, hi) within the words of q0, in index order
+            auto search = [&](int q0, int lo, int hi, T &tb, int &bi) {
 #pragma unroll 1
-                for (int w = (lo - j0) >> 5; w < 32 && j0 + (w << 5) < hi; ++w) {
-                    const int jw = j0 + (w << 5);
-                    const unsigned bm = __shfl_sync(0xffffffffu, bmask, w);
-                    unsigned cm = (__shfl_sync(0xffffffffu, cmask, w) | bm) & keep_from(lo - jw);
-                    if (hi < jw + 32) cm &= (1u << (hi - jw)) - 1u;
+                for (int w = (lo - q0) >> 5; w < 32 && q0 + (w << 5) < hi; ++w) {
+                    const int qw = q0 + (w << 5);
+                    const unsigned bm = kMixed ? 0u : __shfl_sync(0xffffffffu, bmask, w);
+                    unsigned cm = (__shfl_sync(0xffffffffu, cmask, w) | bm) & keep_from(lo - qw);
+                    if (hi < qw + 32) cm &= (1u << (hi - qw)) - 1u;
                     while (cm) {  // the same in every lane; two spheres per pass (independent chains)
                         const int ba_ = __ffs(cm) - 1;
                         cm &= cm - 1;
                         const int bb_ = cm ? __ffs(cm) - 1 : ba_;
                         const bool two = cm != 0u;
+                        if (COUNT && lane == 6) tcount += two ? 2 : 1;
                         cm &= cm - 1;  // 0 stays 0
-                        const int ja = jw + ba_, jb = jw + bb_;
-                        const bool ma = gate(ja), mb = gate(jb);
+                        const bool ma = gate(qw + ba_), mb = gate(qw + bb_);
                         unsigned go = (__any_sync(0xffffffffu, ma) || ((bm >> ba_) & 1u)) ? 1u : 0u;
                         if (two && (__any_sync(0xffffffffu, mb) || ((bm >> bb_) & 1u))) go |= 2u;
 #pragma unroll 1
-                        for (; go; go &= go - 1) test((go & 1u) ? ja : jb, tb, bi);
+                        for (; go; go &= go - 1) test(surface(qw + ((go & 1u) ? ba_ : bb_)), tb, bi);
                     }
                 }
             };
@@ -574,8 +680,11 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                 for (int w = 0; w < p.nbv; ++w) {
                     const bool may = odd || reaches(rf, idd, s_bvbs[w]);
                     if (!__any_sync(0xffffffffu, may)) continue;
-                    const HitRec hb = s_bvtab[w];
-                    const T t = hit_any<M>(__float_as_int(hb.aux.x), hb, ray, eps, sc, M::inf());
+                    T t;
+                    if constexpr (M::kF64)  // (registers to spare, and no code to share it with)
+                        t = hit_any<M>(__float_as_int(s_bvtab[w].aux.x), s_bvtab[w], ray, eps, sc, M::inf());
+                    else
+                        t = shell_hit<M>(s_bvtab + w, ray, eps, sc);
                     const bool nearer = t < tbest;
                     if (!__any_sync(0xffffffffu, nearer)) continue;
                     const int4 info = s_bvinfo[w];
@@ -602,9 +711,9 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
             } else {
                 T tb = M::inf();
 #pragma unroll 1
-                for (int j0 = 0; j0 < n; j0 += 1024) {
-                    candidates(j0);
-                    search(j0, j0, min(n, j0 + 1024), tb, bi);
+                for (int q0 = 0; q0 < nc; q0 += 1024) {
+                    candidates(q0);
+                    search(q0, q0, min(nc, q0 + 1024), tb, bi);
                 }
             }
             if (REC) {
@@ -615,37 +724,49 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                 warp_tally_global(p.hits + (int64_t)emitter * n, valid ? bi : -1);
             }
         }
+        if (COUNT) {
+            if (lane < 8 && tcount) atomicAdd(p.work + lane, (unsigned long long)tcount);
+            tcount = 0;
+        }
         __syncthreads();
     }
     if (!REC) flush();
+    if (kMixed) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) nref += __shfl_xor_sync(0xffffffffu, nref, o);
+        if (lane == 0 && nref) atomicAdd(p.refined, (unsigned long long)nref);
+    }
 }
 
-template <class M, bool BV, bool REC, bool RES>
-static cudaError_t launch_culled_k(const TraceParams &p, int sms, cudaStream_t st)
+template <class M, bool BV, bool REC, bool RES, bool COUNT = false>
+static cudaError_t launch_culled_k(const TraceParams &p, int blocks, cudaStream_t st)
 {
     // one block per SM: 1024 threads of 64 registers, in FP64 512 of 128 (two blocks of
     // 512 or four of 256 threads with shorter chunks sort into less similar packets:
     // 64 surfaces EXACT, 1e8 rays, 5.9 / 6.4 / 7.6 ms)
     constexpr int THREADS = M::kF64 ? 512 : 1024;
-    auto k = culled_kernel<M, THREADS, BV, REC, RES>;
+    auto k = culled_kernel<M, THREADS, BV, REC, RES, COUNT>;
     const int smem = CulledLayout(p.chunk_draws, RES ? p.n : 0, !REC && p.use_smem_hist ? p.n : 0, BV ? p.nbv : 0).bytes;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const int grid = (int)max((int64_t)1, min((int64_t)sms, p.total_chunks));
+    const int grid = (int)max((int64_t)1, min((int64_t)blocks, p.total_chunks));
     k<<<grid, THREADS, smem, st>>>(p);
     return cudaGetLastError();
+}
+
+static bool culled_fits(const TraceParams &p, bool bv)
+{
+    return p.chunk_draws > 0 && p.chunk_draws <= kChunkDraws && p.chunk_draws % 4 == 0 &&
+           (!bv || (p.n <= kBatchTile && p.nbv > 0 && p.nbv <= kBatchMaxBV)) && (!p.use_smem_hist || p.n <= kBatchHist);
 }
 
 template <class M>
 cudaError_t launch_culled(const TraceParams &p, bool bv, bool rec, int sms, cudaStream_t st)
 {
-    const bool res = p.n <= kBatchTile;
-    if (p.chunk_draws <= 0 || p.chunk_draws > kChunkDraws || p.chunk_draws % 4 ||
-        (bv && (!res || p.nbv <= 0 || p.nbv > kBatchMaxBV)) || (p.use_smem_hist && p.n > kBatchHist))
-        return cudaErrorInvalidValue;
+    if (!culled_fits(p, bv)) return cudaErrorInvalidValue;
     if (bv)
         return rec ? launch_culled_k<M, true, true, true>(p, sms, st) : launch_culled_k<M, true, false, true>(p, sms, st);
-    if (res)
+    if (p.n <= kBatchTile)
         return rec ? launch_culled_k<M, false, true, true>(p, sms, st) : launch_culled_k<M, false, false, true>(p, sms, st);
     return rec ? launch_culled_k<M, false, true, false>(p, sms, st) : launch_culled_k<M, false, false, false>(p, sms, st);
 }

@@ -147,8 +147,9 @@ bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs
 // have segment stacks (kStackType).
 cudaError_t launch_batched(const TraceParams &p, bool rec, bool resident, bool count, bool stacks, int grid,
                            cudaStream_t st);
-// The same kernel with runBVGPU's bounding-surface semantics (one resident scene).
-cudaError_t launch_batched_bv(const TraceParams &p, bool rec, bool count, bool stacks, int grid, cudaStream_t st);
+// Mixed precision through the culled kernel (rf_culled_mixed.cu), one resident scene:
+// bounding surfaces (runBVGPU's walk), or segment stacks; at most `blocks` blocks.
+cudaError_t launch_mixed_culled(const TraceParams &p, bool bv, bool rec, bool count, int blocks, cudaStream_t st);
 int batched_blocks_per_sm(bool rec, bool resident);
 cudaError_t launch_mask_inputs(const rf_primitive *emit, const float4 *sph, int n, float4 *patch, float4 *chain,
                                float4 *plane, cudaStream_t st);
@@ -159,6 +160,8 @@ constexpr int kSmallMax = 64;       // surfaces of the largest scene it takes
 constexpr int kSmallThreads = 256;
 cudaError_t launch_mixed_small(const TraceParams &p, int gpt, bool rec, int grid, cudaStream_t st);
 int mixed_small_blocks_per_sm(int gpt, bool rec);
+// The same with bounding surfaces (runBVGPU's walk), 4 rays per thread; 4 blocks fit an SM.
+cudaError_t launch_mixed_small_bv(const TraceParams &p, bool rec, int grid, cudaStream_t st);
 size_t batched_smem_bytes();
 int batched_tile();  // scenes with at most this many surfaces use the resident kernel
 constexpr int kBatchTile = 512;  // surfaces the resident kernel keeps in shared memory

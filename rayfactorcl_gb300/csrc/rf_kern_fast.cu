@@ -24,6 +24,16 @@ cudaError_t launch_mixed_small(const TraceParams &p, int gpt, bool rec, int grid
     return gpt == 2 ? launch_s<2, false>(p, grid, st) : launch_s<1, false>(p, grid, st);
 }
 
+cudaError_t launch_mixed_small_bv(const TraceParams &p, bool rec, int grid, cudaStream_t st)
+{
+    if (p.n <= 0 || p.n > kSmallMax || p.nbv <= 0 || p.nbv > kBatchMaxBV) return cudaErrorInvalidValue;
+    if (rec)
+        mixed_small_bv_kernel<true><<<grid, kSmallThreads, 0, st>>>(p);
+    else
+        mixed_small_bv_kernel<false><<<grid, kSmallThreads, 0, st>>>(p);
+    return cudaGetLastError();
+}
+
 // Resident blocks per SM, queried once per process (every GPU of a run is the same part).
 template <int GPT, bool REC>
 static int occ_s()
