@@ -117,7 +117,7 @@ def load() -> ctypes.CDLL:
 
 
 def ptr(a: np.ndarray | None):
-    return None if a is None else a.ctypes.data_as(ctypes.c_void_p)
+    return None if a is None else ctypes.c_void_p(a.__array_interface__["data"][0])
 
 
 def check(status: int, ctx=None):

@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <fstream>
+#include <initializer_list>
 #include <limits>
 #include <map>
 #include <mutex>
@@ -111,14 +112,16 @@ struct rf_ctx {
     bool tuning = false;  // rf_autotune is timing the plain kernel's launch shapes
 
     // trace state
-    DevBuf d_hits, d_seg, d_rays, d_F, d_rec, d_err, d_misc;
-    PinBuf h_seg, h_rays, h_misc;
+    DevBuf d_hits, d_seg, d_F, d_rec, d_err, d_misc;
+    PinBuf h_seg, h_rays, h_out;
     std::vector<Segment> seg_cache;  // the plan in d_seg when seg_valid
     bool seg_valid = false;
     std::vector<int64_t> last_rays;
     bool have_results = false;
     int last_launches = 0;
     bool timed = false;
+    LaunchCfg occ_of;  // the launch shape that occ was asked for (the query costs more than a launch)
+    int occ = 0;
 
     // launch choices (0 / -1 = default); set by rf_config or rf_autotune
     int block = 0, gpt = 0, hist = -1, stage = -1, order = -1;  // order 1: one ray at a time
@@ -359,6 +362,33 @@ Plan make_plan(const rf_ctx *c, bool bv, bool rec, int64_t draws)
     return pl;
 }
 
+// Device arrays to the caller's memory.  On this machine a copy to pageable memory is
+// direct and fast (60 GB/s) when its pages exist, but each 64 KB that was allocated and
+// never written costs a page fault from the GPU, about 50 us (3.4 ms for 4 MB of fresh
+// tallies): the host writes to every page first.  Returns with the stream idle.
+struct OutCopy {
+    void *dst;
+    const void *src;
+    size_t bytes;
+};
+
+void touch(void *dst, size_t bytes)
+{
+    volatile char *p = static_cast<char *>(dst);
+    for (size_t i = 0; i < bytes; i += 4096) p[i] = 0;
+    if (bytes) p[bytes - 1] = 0;
+}
+
+rf_status copy_out(rf_ctx *c, std::initializer_list<OutCopy> list)
+{
+    for (const OutCopy &o : list)
+        if (o.dst) touch(o.dst, o.bytes);
+    for (const OutCopy &o : list)
+        if (o.dst) RF_CUDA(c, cudaMemcpyAsync(o.dst, o.src, o.bytes, cudaMemcpyDeviceToHost, c->stream));
+    RF_CUDA(c, cudaStreamSynchronize(c->stream));
+    return RF_OK;
+}
+
 // Put a launch's segment plan in d_seg, unless it is the plan already there (a trace
 // repeated with the same budgets): then nothing is copied and nothing waits, so the
 // host can queue the next launch while the GPU runs the previous one.  Otherwise the
@@ -431,9 +461,13 @@ rf_status run_trace(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
         c->timed = true;
         return RF_OK;
     }
-    int bps = blocks_per_sm(arith, pl.lc);
-    if (bps <= 0) bps = 1;
-    const int64_t wave = (int64_t)c->sms * bps;
+    const LaunchCfg &q = c->occ_of, &l = pl.lc;
+    if (c->occ <= 0 || q.block != l.block || q.gpt != l.gpt || q.smem != l.smem || q.bv != l.bv || q.rec != l.rec ||
+        q.stage != l.stage || q.serial != l.serial) {
+        c->occ = std::max(1, blocks_per_sm(arith, l));
+        c->occ_of = l;
+    }
+    const int64_t wave = (int64_t)c->sms * c->occ;
     pl.lc.grid = (int)std::max<int64_t>(1, std::min<int64_t>(wave, total_chunks));
     RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     RF_CUDA(c, launch_arith(arith, pl.lc, p, c->stream));
@@ -1170,14 +1204,14 @@ void rf_destroy(rf_ctx *c)
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (DevBuf *b : {&c->d_tab, &c->d_emit, &c->d_bvtab, &c->d_bvinfo, &c->d_hits, &c->d_seg,
-                      &c->d_rays, &c->d_F, &c->d_rec, &c->d_cull, &c->d_err, &c->d_misc, &c->b_tab, &c->b_emit,
+                      &c->d_F, &c->d_rec, &c->d_cull, &c->d_err, &c->d_misc, &c->b_tab, &c->b_emit,
                       &c->b_bsph, &c->b_scenes, &c->b_hits, &c->b_rows, &c->b_counters, &c->b_own, &c->b_patch,
                       &c->b_chain, &c->b_plane, &c->b_cone, &c->b_maskrows, &c->b_maskoff, &c->b_mask, &c->b_frame, &c->b_bvtab,
                       &c->b_bvinfo, &c->b_bvsph})
         b->release();
     c->h_seg.release();
     c->h_rays.release();
-    c->h_misc.release();
+    c->h_out.release();
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1407,32 +1441,38 @@ rf_status rf_read_results(rf_ctx *c, uint64_t *hits_out, double *F_out)
     const size_t nn = (size_t)n * n;
     const unsigned long long *hits_dev = c->cfg.precision == RF_PREC_MIXED ? c->b_hits.as<unsigned long long>()
                                                                            : c->d_hits.as<unsigned long long>();
-    if (F_out) {
-        RF_CUDA(c, c->d_rays.ensure(n * sizeof(int64_t)));
+    const bool mixed = c->cfg.precision == RF_PREC_MIXED;
+    const BatchCounters *bc = mixed ? c->b_counters.as<BatchCounters>() : nullptr;
+    // (the previous call that used these buffers waited for the stream)
+    RF_CUDA(c, c->h_rays.ensure(n * sizeof(int64_t)));
+    std::memcpy(c->h_rays.p, c->last_rays.data(), n * sizeof(int64_t));
+    // up to 64 KB a matrix, the kernel writes the results to pinned memory (n = 3: 31 us a
+    // trace against 66 with the copies); beyond, they are copied
+    const bool pinned = nn * 8 <= 64 * 1024;
+    const size_t head = 256, part = pinned ? nn * 8 : 0;
+    RF_CUDA(c, c->h_out.ensure(head + 2 * part));
+    FinishHead *fh = c->h_out.as<FinishHead>();
+    unsigned long long *ph = hits_out && pinned ? reinterpret_cast<unsigned long long *>(c->h_out.as<char>() + head) : nullptr;
+    double *pF = F_out && pinned ? reinterpret_cast<double *>(c->h_out.as<char>() + head + part) : nullptr;
+    RF_CUDA(c, launch_finish(hits_dev, c->h_rays.as<int64_t>(), n, ph, pF, c->d_err.as<int32_t>(),
+                             mixed ? &bc->refined : nullptr, mixed ? bc->work : nullptr, fh, c->stream));
+    if (!pinned && F_out) {
         RF_CUDA(c, c->d_F.ensure(nn * sizeof(double)));
-        RF_CUDA(c, c->h_rays.ensure(n * sizeof(int64_t)));
+        RF_CUDA(c, launch_normalise_single(hits_dev, c->h_rays.as<int64_t>(), n, c->d_F.as<double>(), c->stream));
+    }
+    if (pinned) {
         RF_CUDA(c, cudaStreamSynchronize(c->stream));
-        std::memcpy(c->h_rays.p, c->last_rays.data(), n * sizeof(int64_t));
-        RF_CUDA(c, cudaMemcpyAsync(c->d_rays.p, c->h_rays.p, n * sizeof(int64_t), cudaMemcpyHostToDevice,
-                                   c->stream));
-        RF_CUDA(c, launch_normalise_single(hits_dev, c->d_rays.as<int64_t>(), n, c->d_F.as<double>(),
-                                           c->stream));
-        RF_CUDA(c, cudaMemcpyAsync(F_out, c->d_F.p, nn * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        if (hits_out) std::memcpy(hits_out, ph, nn * 8);
+        if (F_out) std::memcpy(F_out, pF, nn * 8);
+    } else if ((s = copy_out(c, {{F_out, c->d_F.p, nn * sizeof(double)}, {hits_out, hits_dev, nn * 8}})) != RF_OK) {
+        return s;
     }
-    if (hits_out) RF_CUDA(c, cudaMemcpyAsync(hits_out, hits_dev, nn * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (c->cfg.precision == RF_PREC_MIXED)
-    {
-        RF_CUDA(c, cudaMemcpyAsync(&c->last_refined, &c->b_counters.as<BatchCounters>()->refined,
-                                   sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-        RF_CUDA(c, cudaMemcpyAsync(c->last_work, c->b_counters.as<BatchCounters>()->work,
-                                   sizeof c->last_work, cudaMemcpyDeviceToHost, c->stream));
+    if (mixed) {
+        c->last_refined = fh->refined;
+        std::copy(std::begin(fh->work), std::end(fh->work), std::begin(c->last_work));
+        if (c->last_small) std::copy(std::begin(c->small_work), std::end(c->small_work), std::begin(c->last_work));
     }
-    RF_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (c->cfg.precision == RF_PREC_MIXED && c->last_small)
-        std::copy(std::begin(c->small_work), std::end(c->small_work), std::begin(c->last_work));
-    int32_t err = 0;
-    RF_CUDA(c, cudaMemcpy(&err, c->d_err.p, 4, cudaMemcpyDeviceToHost));
-    if (err) return fail(c, RF_ERR_TIMEOUT, "device reported error %d", err);
+    if (fh->err) return fail(c, RF_ERR_TIMEOUT, "device reported error %d", fh->err);
     return RF_OK;
 }
 
@@ -1492,8 +1532,7 @@ rf_status rf_trace_rays(rf_ctx *c, int32_t emitter, int64_t first_ray, int64_t n
         const int64_t chunks = plan_segments(seg, emitter, 0, first_ray, n_rays, pl.chunk_gids(), 0);
         if ((s = run_trace(c, seg, chunks, pl, c->d_rec.as<int32_t>(), first_ray, false)) != RF_OK) return s;
     }
-    RF_CUDA(c, cudaMemcpyAsync(out, c->d_rec.p, (size_t)n_rays * 4, cudaMemcpyDeviceToHost, c->stream));
-    RF_CUDA(c, cudaStreamSynchronize(c->stream));
+    if ((s = copy_out(c, {{out, c->d_rec.p, (size_t)n_rays * 4}})) != RF_OK) return s;
     c->have_results = false;  // the tallies were not produced by this call
     return RF_OK;
 }
@@ -1733,9 +1772,8 @@ rf_status rf_smooth_F(rf_ctx *c, const double *F, const double *areas, int32_t n
     cudaError_t e = launch_smooth(c->d_F.as<double>(), d_A, n, closed ? 1 : 0, 2000, 1e-13, c->d_misc.p, d_out,
                                   c->sms, &it, &err, &gave_up, c->stream);
     if (e == cudaSuccess && gave_up) return fail(c, RF_ERR_TIMEOUT, "smoothing: the grid's blocks did not meet");
-    if (e == cudaSuccess) e = cudaMemcpyAsync(F_out, d_out, nn * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "smoothing");
+    if (rf_status st = copy_out(c, {{F_out, d_out, nn * sizeof(double)}}); st != RF_OK) return st;
     if (iterations) *iterations = it;
     if (residual) *residual = err;
     return RF_OK;
@@ -1813,14 +1851,10 @@ rf_status rf_trace_batch(rf_ctx *c, const rf_scene_desc *scenes, int32_t n_scene
     RF_CUDA(c, launch_converge_step(c->b_hits.as<unsigned long long>(), d_rows + nrows, d_rows, 
                                     reinterpret_cast<int32_t *>(d_rows + 2 * nrows), nrows,
                                     c->d_F.as<double>(), 0.0, d_rows + 3 * nrows, 0, &bc->flags[0], c->stream));
-    if (hits_out)
-        RF_CUDA(c, cudaMemcpyAsync(hits_out, c->b_hits.p, (size_t)c->b_hits_total * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (F_out)
-        RF_CUDA(c, cudaMemcpyAsync(F_out, c->d_F.p, (size_t)c->b_hits_total * 8, cudaMemcpyDeviceToHost, c->stream));
-    RF_CUDA(c, cudaMemcpyAsync(&c->last_refined, &bc->refined, 8, cudaMemcpyDeviceToHost, c->stream));
-    RF_CUDA(c, cudaMemcpyAsync(c->last_work, bc->work, sizeof c->last_work, cudaMemcpyDeviceToHost, c->stream));
-    RF_CUDA(c, cudaStreamSynchronize(c->stream));
-    return RF_OK;
+    return copy_out(c, {{hits_out, c->b_hits.p, (size_t)c->b_hits_total * 8},
+                        {F_out, c->d_F.p, (size_t)c->b_hits_total * 8},
+                        {&c->last_refined, &bc->refined, 8},
+                        {c->last_work, bc->work, sizeof c->last_work}});
 }
 
 rf_status rf_converge_batch(rf_ctx *c, const rf_scene_desc *scenes, int32_t n_scenes, double tol,
@@ -1928,15 +1962,13 @@ rf_status rf_converge_batch(rf_ctx *c, const rf_scene_desc *scenes, int32_t n_sc
     RF_CUDA(c, launch_converge_step(c->b_hits.as<unsigned long long>(), d_total, d_off, d_len, nrows,
                                     c->d_F.as<double>(), tol, d_next, 0, &bc->flags[0], c->stream));
     int32_t flags[2] = {0, 0};
-    RF_CUDA(c, cudaMemcpyAsync(flags, &bc->flags[0], 8, cudaMemcpyDeviceToHost, c->stream));
-    RF_CUDA(c, cudaMemcpyAsync(&c->last_refined, &bc->refined, 8, cudaMemcpyDeviceToHost, c->stream));
-    RF_CUDA(c, cudaMemcpyAsync(c->last_work, bc->work, sizeof c->last_work, cudaMemcpyDeviceToHost, c->stream));
-    if (hits_out)
-        RF_CUDA(c, cudaMemcpyAsync(hits_out, c->b_hits.p, (size_t)c->b_hits_total * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (F_out)
-        RF_CUDA(c, cudaMemcpyAsync(F_out, c->d_F.p, (size_t)c->b_hits_total * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (rays_out) RF_CUDA(c, cudaMemcpyAsync(rays_out, d_total, nrows * 8, cudaMemcpyDeviceToHost, c->stream));
-    RF_CUDA(c, cudaStreamSynchronize(c->stream));
+    if ((st = copy_out(c, {{flags, &bc->flags[0], 8},
+                           {&c->last_refined, &bc->refined, 8},
+                           {c->last_work, bc->work, sizeof c->last_work},
+                           {hits_out, c->b_hits.p, (size_t)c->b_hits_total * 8},
+                           {F_out, c->d_F.p, (size_t)c->b_hits_total * 8},
+                           {rays_out, d_total, (size_t)nrows * 8}})) != RF_OK)
+        return st;
     if (rounds_out) *rounds_out = flags[1];
     c->last_launches = 4 * flags[1];
     return RF_OK;

@@ -192,6 +192,15 @@ int prepare_mixed_tables(const rf_primitive *prims, int n, float eps, uint32_t c
                          float4 *bs, float *eps_out);
 
 // FP64 post-processing and probes (rf_kern_post.cu).
+struct FinishHead {
+    unsigned long long refined;
+    unsigned long long work[8];
+    int32_t err;
+    int32_t pad;
+};
+cudaError_t launch_finish(const unsigned long long *hits, const int64_t *rays, int n, unsigned long long *hits_out,
+                          double *F_out, const int32_t *err, const unsigned long long *refined,
+                          const unsigned long long *work, FinishHead *head, cudaStream_t st);
 cudaError_t launch_normalise_single(const unsigned long long *hits, const int64_t *rays, int n,
                                     double *F, cudaStream_t st);
 cudaError_t launch_converge_step(const unsigned long long *hits, int64_t *rays,

@@ -98,10 +98,10 @@ class Tracer:
     def trace(self, rays, use_bv: bool = False, want_F: bool = True):
         """Tally matrix (int64 n x n) and F (float64 n x n, or None)."""
         r = self._rays(rays)
-        hits = np.zeros((self.n, self.n), np.uint64)
-        F = np.zeros((self.n, self.n), np.float64) if want_F else None
+        hits = np.empty((self.n, self.n), np.int64)  # (uint64 counts below 2^63)
+        F = np.empty((self.n, self.n), np.float64) if want_F else None
         self._check(self._L.rf_trace(self._h, ptr(r), 1 if use_bv else 0, ptr(hits), ptr(F)))
-        return hits.astype(np.int64), F
+        return hits, F
 
     def trace_async(self, rays, use_bv: bool = False):
         self._keep = self._rays(rays)
@@ -122,10 +122,10 @@ class Tracer:
 
     def results(self):
         """(int64 tallies, F) of everything traced so far."""
-        hits = np.zeros((self.n, self.n), np.uint64)
-        F = np.zeros((self.n, self.n), np.float64)
+        hits = np.empty((self.n, self.n), np.int64)
+        F = np.empty((self.n, self.n), np.float64)
         self._check(self._L.rf_read_results(self._h, ptr(hits), ptr(F)))
-        return hits.astype(np.int64), F
+        return hits, F
 
     def read_results(self, hits: np.ndarray | None = None, F: np.ndarray | None = None):
         self._check(self._L.rf_read_results(self._h, ptr(hits), ptr(F)))
@@ -150,11 +150,11 @@ class Tracer:
 
     def run_gpurng(self, n_samples: int, use_bv: bool = False):
         rays = np.zeros(self.n, np.int64)
-        hits = np.zeros((self.n, self.n), np.uint64)
-        F = np.zeros((self.n, self.n), np.float64)
+        hits = np.empty((self.n, self.n), np.int64)
+        F = np.empty((self.n, self.n), np.float64)
         self._check(self._L.rf_run_gpurng(self._h, int(n_samples), 1 if use_bv else 0, ptr(rays),
                                           ptr(hits), ptr(F)))
-        return rays, hits.astype(np.int64), F
+        return rays, hits, F
 
     def autotune(self, use_bv: bool = False, cache_path: str | None = None):
         """Time the launch shapes of the current scene and keep the fastest."""
@@ -204,11 +204,11 @@ class Tracer:
         per-scene tally and F matrices."""
         descs, keep = self._descs(scenes, rays_list)
         tot = sum(int(sc.primitives.shape[0]) ** 2 for sc in scenes)
-        hits = np.zeros(tot, np.uint64)
-        F = np.zeros(tot, np.float64)
+        hits = np.empty(tot, np.int64)
+        F = np.empty(tot, np.float64)
         self._check(self._L.rf_trace_batch(self._h, descs, len(scenes), ptr(hits), ptr(F)))
         del keep
-        return self._split(scenes, hits.astype(np.int64)), self._split(scenes, F)
+        return self._split(scenes, hits), self._split(scenes, F)
 
     def converge_batch(self, scenes, rays_list, tol: float, round_rays: int, max_rounds: int):
         """Add rays until every row's binomial standard error is <= tol (CUDA-graph
@@ -216,8 +216,8 @@ class Tracer:
         descs, keep = self._descs(scenes, rays_list)
         tot = sum(int(sc.primitives.shape[0]) ** 2 for sc in scenes)
         nrows = sum(int(sc.primitives.shape[0]) for sc in scenes)
-        hits = np.zeros(tot, np.uint64)
-        F = np.zeros(tot, np.float64)
+        hits = np.empty(tot, np.int64)
+        F = np.empty(tot, np.float64)
         rays = np.zeros(nrows, np.int64)
         rounds = ctypes.c_int32()
         self._check(self._L.rf_converge_batch(self._h, descs, len(scenes), float(tol), int(round_rays),
@@ -229,13 +229,13 @@ class Tracer:
             n = sc.primitives.shape[0]
             rl.append(rays[off:off + n].copy())
             off += n
-        return self._split(scenes, hits.astype(np.int64)), self._split(scenes, F), rl, rounds.value
+        return self._split(scenes, hits), self._split(scenes, F), rl, rounds.value
 
     def smooth_F(self, F: np.ndarray, areas: np.ndarray, closed: bool = True):
         """Reciprocity (and, for a closed enclosure, summation) enforced in FP64."""
         F = np.ascontiguousarray(F, np.float64)
         a = np.ascontiguousarray(areas, np.float64)
-        out = np.zeros_like(F)
+        out = np.empty_like(F)
         it, res = ctypes.c_int32(), ctypes.c_double()
         self._check(self._L.rf_smooth_F(self._h, ptr(F), ptr(a), F.shape[0], 1 if closed else 0, ptr(out),
                                         ctypes.byref(it), ctypes.byref(res)))
