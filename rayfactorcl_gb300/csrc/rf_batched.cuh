@@ -1,8 +1,8 @@
 // rf_batched.cuh -- the batched mixed-precision persistent tracing kernel.
 //
 // One launch traces any number of independent scenes.  Work items are chunks
-// of kBatchDraws*kBatchThreads Philox draws (4 rays each) of one (scene,
-// emitter) segment; a persistent grid pulls them from a device queue (an
+// of up to kBatchDraws*kBatchThreads Philox draws (4 rays each; chunk_for sizes them) of
+// one (scene, emitter) segment; a persistent grid pulls them from a device queue (an
 // atomic counter), so scenes of 10 and of 400 surfaces load-balance.
 //
 // Per chunk (32768 rays) a block
@@ -25,15 +25,15 @@
 //   4. evaluates the surviving tests in FP32, with quadric discriminants in
 //      cancellation-free forms; a discriminant within 16 rounding errors of
 //      its terms (a grazing ray), or a cone whose A lost 12 bits, is
-//      re-evaluated in FP64 after the packet, and
+//      re-evaluated in FP64 at once, and
 //   5. tallies first hits in a shared-memory row histogram (flushed as 64-bit
 //      atomics whenever the (scene, emitter) row changes) straight from the
 //      packet loop.
 // A ray's result depends on the ray alone, never on the rays it shares a packet
 // with: it is the nearest hit among the surfaces the ray's own gate admits (its
 // cell mask bit and its sphere check, both functions of the ray), every one of
-// which its packet tests; a lane whose packet-wide winner fails its own gate,
-// or that deferred more than one test, re-traces over its gated set.  Skipping
+// which its packet tests; a lane whose packet-wide winner fails its own gate
+// re-traces over its gated set.  Skipping
 // a surface that the ray cannot reach does not change its nearest hit; only the
 // arithmetic differs from the exact kernel.  Scenes of at most kBruteMax surfaces skip
 // steps 1-3: every thread tests its own rays against all surfaces.  A segment stack
@@ -78,6 +78,14 @@ struct BatchSmem {
     int hist[kBatchHist];
     rf_primitive emit;
     float4 frame[kFrameWords];
+    struct {                            // the current row (scene, emitter)
+        const uint32_t *masks;          // its cell masks (null: packet bounds instead)
+        const HitRec *tab;              // its scene's records and spheres in global memory
+        const float4 *bs;
+        unsigned long long *hits;       // its tallies
+        int n, skip, hist;              // surfaces; self_skip; tallied in `hist` first
+        float eps;
+    } row;
     int64_t chunk;
     unsigned long long bar;             // mbarrier of the bulk copies of the scene tables
     int next_packet;
@@ -541,6 +549,17 @@ __device__ __forceinline__ float test_f64(const HitRec &h, int j, const Ray<floa
     return hit_f64(h, w, eps, sc);
 }
 
+// FP64 evaluation of surface j's deferred test (record in shared or global memory):
+// t and, in y, the bits of the surface hit.  By value, so that the hot loop's ray and
+// record stay in registers.
+static __device__ __noinline__ float2 deferred_f64(const HitRec *rec, int j, Ray<float> w, float eps, bool sc)
+{
+    const HitRec h = *rec;
+    int idx;
+    const float t = test_f64<true>(h, j, w, eps, sc, idx);
+    return make_float2(t, __int_as_float(idx));
+}
+
 // Sort key of a ray: its direction cell above the 4 x 4 cell of the two surface
 // parameters (r[0], r[1]) of its emission point.
 __device__ __forceinline__ int ray_key(const Ray<float> &ray, const float r[4])
@@ -574,61 +593,24 @@ __device__ __forceinline__ unsigned keep_from(int k)
     return k <= 0 ? ~0u : (k >= 32 ? 0u : (~0u << k));
 }
 
-// The candidate loop's test: hit_mixed's, plus segment stacks.  idx (j on entry)
-// gets the surface hit; a stack's other members leave the candidate word cm and
-// the pair's second candidate (vb = 0 when jb is one): skip_to = one past the
-// stack, for later words.
-__device__ __forceinline__ float hit_hot(int type, const HitRec &h, int j, const HitRec *tab, bool resident,
-                                         const Ray<float> &w, float eps, bool sc, bool &defer, int &idx, int jw,
-                                         unsigned &cm, int &skip_to, int jb, unsigned &vb)
-{
-    switch (type) {
-    case RF_RECTANGLE: return rectangle_hit<MFast>(h, w, eps);
-    case RF_DISC: return disc_hit<MFast>(h, w, eps);
-    case RF_ANNULUS: return annulus_hit<MFast>(h, w, eps);
-    case RF_CYLINDER: return cylinder_mixed(h, w, eps, defer);
-    case RF_FRUSTUM: return frustum_mixed(h, w, eps, defer);
-    case RF_SPHERE: return sphere_mixed(h, w, eps, sc, defer);
-    case kStackType: {
-        int ring;
-        const float t = stack_mixed(h, w, eps, defer, ring);
-        idx = stack_first(h, j) + ring;
-        skip_to = stack_end(h, j);
-        cm &= keep_from(skip_to - jw);
-        if (jb < skip_to) vb = 0u;
-        return t;
-    }
-    case kPlateType: {
-        const float t = plate_mixed(h, j, tab, resident, w, eps, idx);
-        skip_to = stack_end(h, j);
-        cm &= keep_from(skip_to - jw);
-        if (jb < skip_to) vb = 0u;
-        return t;
-    }
-    default: return MFast::inf();
-    }
-}
-
-// Full nearest-hit search for one ray over the surfaces [lo, hi) its gate admits
-// (gated: the cell mask when mcell is set, and the bounding-sphere check; else
-// every surface but skip), with FP64 for every ill-conditioned quadric; nf64
-// counts the FP64 evaluations.  Cold path: rays that deferred a test they could
-// not resolve in their hot loop.
+// Full nearest-hit search for one ray over the surfaces [0, n) its gate admits (the
+// cell mask when mcell is set, and the bounding-sphere check) but skip, with FP64 for
+// every ill-conditioned quadric: the surface, and in y the FP64 evaluations.  tab, bs: shared or global memory.  Cold path; by
+// value, so that the callers' ray stays in registers.
 template <bool STK>
-static __device__ __noinline__ int retrace_f64(int lo, int hi, bool resident, const HitRec *stab, const HitRec *gtab,
-                                        const float4 *sbs, const float4 *gbs, const uint32_t *mcell, bool gated,
-                                        const Ray<float> &ray, float idd, float eps, bool sc, int skip, int &nf64)
+static __device__ __noinline__ int2 retrace_f64(int n, const HitRec *tab, const float4 *bs, const uint32_t *mcell,
+                                                Ray<float> ray, float idd, float eps, bool sc, int skip)
 {
     float tb = MFast::inf();
-    int bi = -1;
-    for (int j = lo; j < hi; ++j) {
+    int bi = -1, nf64 = 0;
+    for (int j = 0; j < n; ++j) {
         if (j == skip) continue;
-        if (gated && !own_gate(mcell, j, ray, idd, resident ? sbs[j] : __ldg(gbs + j))) continue;
-        const HitRec h = resident ? stab[j] : load_rec(gtab, j);
+        if (!own_gate(mcell, j, ray, idd, bs[j])) continue;
+        const HitRec h = tab[j];
         const int type = __float_as_int(h.aux.x);
         bool defer = false;
         int idx;
-        float t = test_mixed<STK>(type, h, j, resident ? stab : gtab, resident, ray, eps, sc, defer, idx);
+        float t = test_mixed<STK>(type, h, j, tab, true, ray, eps, sc, defer, idx);
         if (defer) {
             t = test_f64<STK>(h, j, ray, eps, sc, idx);
             ++nf64;
@@ -636,7 +618,7 @@ static __device__ __noinline__ int retrace_f64(int lo, int hi, bool resident, co
         if (t < tb) { tb = t; bi = idx; }
         if (STK && is_stack(type)) j = stack_end(h, j) - 1;  // one test for the whole stack
     }
-    return bi;
+    return make_int2(bi, nf64);
 }
 
 // Nearest hit of a ray tested against every surface of [lo, hi) but skip, in
@@ -644,14 +626,34 @@ static __device__ __noinline__ int retrace_f64(int lo, int hi, bool resident, co
 // a ray is traced again with FP64 for each deferred test.  Shared by the
 // small-scene paths of the batched kernel and of mixed_small_kernel, so both
 // give the same result.
+// (By reference: with several rays a thread that call costs the hot loop less.)
 template <bool STK>
-__device__ __forceinline__ int resolve_brute(int bi, bool deferred, int lo, int hi, bool resident,
-                                             const HitRec *stab, const HitRec *gtab, const Ray<float> &ray,
-                                             float eps, bool sc, int skip, int &nref)
+static __device__ __noinline__ int retrace_all(int lo, int hi, const HitRec *tab, const Ray<float> &ray, float eps, bool sc,
+                                               int skip, int &nref)
 {
-    if (deferred)
-        bi = retrace_f64<STK>(lo, hi, resident, stab, gtab, nullptr, nullptr, nullptr, false, ray, 0.0f, eps, sc, skip,
-                         nref);
+    float tb = MFast::inf();
+    int bi = -1;
+    for (int j = lo; j < hi; ++j) {
+        if (j == skip) continue;
+        const HitRec h = tab[j];
+        const int type = __float_as_int(h.aux.x);
+        bool defer = false;
+        int idx;
+        float t = test_mixed<STK>(type, h, j, tab, true, ray, eps, sc, defer, idx);
+        if (defer) {
+            t = test_f64<STK>(h, j, ray, eps, sc, idx);
+            ++nref;
+        }
+        if (t < tb) { tb = t; bi = idx; }
+        if (STK && is_stack(type)) j = stack_end(h, j) - 1;  // one test for the whole stack
+    }
+    return bi;
+}
+template <bool STK>
+__device__ __forceinline__ int resolve_brute(int bi, bool deferred, int lo, int hi, const HitRec *tab,
+                                             const Ray<float> &ray, float eps, bool sc, int skip, int &nref)
+{
+    if (deferred) bi = retrace_all<STK>(lo, hi, tab, ray, eps, sc, skip, nref);
     return bi;
 }
 
@@ -692,41 +694,115 @@ __device__ __forceinline__ int bv_select(const HitRec *bvtab, const int4 *bvinfo
     return obj;
 }
 
+// The current row's constants, read where they are used: as loop-long registers they
+// were spilled.  A volatile load, so that it is not hoisted back into one.
+__device__ __forceinline__ const uint32_t *row_masks(const BatchSmem &S)
+{
+    unsigned long long v;
+    asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(smem_addr(&S.row.masks)));
+    return reinterpret_cast<const uint32_t *>(v);
+}
+
+// A chunk of a scene of at most kBruteMax surfaces, too few for culling to pay: every
+// thread traces its own rays against all surfaces in index order.  Out of line: the
+// registers of the packet loop are its own.  Returns the FP64 evaluations.
+template <bool REC, bool RESIDENT, bool COUNT, bool STK>
+static __device__ __noinline__ int brute_chunk(BatchSmem &S, const TraceParams &p, int emitter, int64_t ray_begin,
+                                               int64_t ray_end, int64_t gid0, int cd, uint32_t sid)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = S.row.n, skip = S.row.skip;
+    const bool sc = (p.compat & RF_COMPAT_SPHERE) != 0, hist_on = S.row.hist != 0;
+    const float eps = S.row.eps;
+    const HitRec *gtab = S.row.tab;
+    int nref = 0;
+    uint32_t nv_warp = 0;
+#pragma unroll 1
+    for (int g = 0; g * kBatchThreads < cd; ++g) {
+        const int d = g * kBatchThreads + tid;
+        const int64_t gid = gid0 + d;
+        const bool any = d < cd && gid * 4 + 3 >= ray_begin && gid * 4 < ray_end;
+        const uint4 u = any ? stream_bits(p.compat, p.key1, sid, emitter, gid) : make_uint4(0u, 0u, 0u, 0u);
+        const float uf[4] = {u01(u.x), u01(u.y), u01(u.z), u01(u.w)};
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const int64_t rid = gid * 4 + v;
+            const bool valid = any && rid >= ray_begin && rid < ray_end;
+            int bi = -1;
+            if (valid) {
+                float r[4];
+                rotate_uniforms(uf, v, r);
+                const Ray<float> ray = emit_mixed(S.emit, S.frame, r);
+                float tb = MFast::inf();
+                bool dany = false;
+#pragma unroll 1
+                for (int j = 0; j < n; ++j) {
+                    if (j == skip) continue;  // uniform: every thread's emitter
+                    const HitRec h = RESIDENT ? S.tab[j] : load_rec(gtab, j);
+                    const int type = __float_as_int(h.aux.x);
+                    bool defer = false;
+                    int idx;
+                    const float t = test_mixed<STK>(type, h, j, RESIDENT ? S.tab : gtab, RESIDENT, ray, eps, sc, defer, idx);
+                    if (t < tb) { tb = t; bi = idx; }
+                    dany |= defer;
+                    if (STK && is_stack(type)) j = stack_end(h, j) - 1;
+                }
+                bi = resolve_brute<STK>(bi, dany, 0, n, RESIDENT ? S.tab : gtab, ray, eps, sc, skip, nref);
+            }
+            // all 32 lanes reach the warp-wide calls below
+            if (COUNT) nv_warp += __popc(__ballot_sync(0xffffffffu, valid));
+            if (REC) {
+                if (valid) p.rec[rid - p.rec_base] = bi;
+            } else if (hist_on) {
+                warp_tally(S.hist, bi);
+            } else {
+                warp_tally_global(S.row.hits, bi);
+            }
+        }
+    }
+    if (COUNT && lane == 0 && nv_warp)
+        for (int j = 0; j < n; ++j) {
+            if (j == skip) continue;
+            const HitRec h = RESIDENT ? S.tab[j] : load_rec(gtab, j);
+            const int type = __float_as_int(h.aux.x);
+            S.wcount[warp][stat_type(type)] += nv_warp;
+            if (STK && is_stack(type)) j = stack_end(h, j) - 1;
+        }
+    return nref;
+}
+
 // RESIDENT: every scene of the launch fits the shared-memory tables
 // (n <= kBatchTile); otherwise surfaces are read through L1.  COUNT: also count
 // the tests by surface type, the candidates and the packets (p.work); the
 // counters cost a few per cent, so timed runs leave them out.  STK: some scene
 // has segment stacks (kStackType records); the candidate loops then test a stack once.
 template <bool REC, bool RESIDENT, bool COUNT, bool STK>
-__global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TraceParams p)
+__global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const __grid_constant__ TraceParams p)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchSmem &S = *reinterpret_cast<BatchSmem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool sc = (p.compat & RF_COMPAT_SPHERE) != 0;
-    float eps = p.eps;  // the current scene's (SceneInfo::eps)
     const int64_t total = p.d_total ? *p.d_total : p.total_chunks;
     const int nseg = p.d_nseg ? *p.d_nseg : p.nseg;
+    const int cd = p.d_chunk ? *p.d_chunk : p.chunk_draws;
 
     int cur_scene = -1, cur_emitter = -1;
-    SceneInfo si{};
     int nref = 0;
     if (COUNT) {
         if (tid < 8) S.work[tid] = 0ull;
         if (lane < 8) S.wcount[warp][lane] = 0u;
     }
-    bool hist_on = false;
     int row_chunks = 0;   // chunks tallied into the shared-memory row since its last flush
     uint32_t tcount = 0;  // COUNT, lane t < 6: lane-tests of surfaces of type t by this warp (this chunk)
-    const uint32_t *mrow = nullptr;  // cell masks of the current row (null: packet bounds instead)
     uint32_t bar_parity = 0;         // phase of S.bar the next table copy completes
     if (RESIDENT && tid == 0) bar_init(&S.bar);  // visible after the chunk loop's first barrier
 
     auto flush = [&]() {
         __syncthreads();
-        if (hist_on && cur_emitter >= 0) {
-            unsigned long long *row = p.hits + si.hits_off + (int64_t)cur_emitter * si.n;
-            for (int i = tid; i < si.n; i += blockDim.x) {
+        if (cur_emitter >= 0 && S.row.hist) {
+            unsigned long long *row = S.row.hits;
+            const int n = S.row.n;
+            for (int i = tid; i < n; i += kBatchThreads) {
                 const int v = S.hist[i];
                 if (v) {
                     atomicAdd(row + i, (unsigned long long)v);
@@ -754,33 +830,27 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
         __syncthreads();
         const int64_t c = S.chunk;
         if (c >= total) break;  // block-uniform
-        const int s = find_segment(p.seg, nseg, c);
-        const Segment sg = p.seg[s];
+        const Segment sg = p.seg[find_segment(p.seg, nseg, c)];
 
-        if (!REC && hist_on && ++row_chunks >= 32768) {  // keep the 32-bit bins far from overflow
-            flush();                                     // (at most 32768 hits per bin per chunk)
+        if (!REC && ++row_chunks >= 32768) {  // keep the 32-bit bins far from overflow
+            flush();                          // (at most 32768 hits per bin per chunk)
             row_chunks = 0;
         }
-        bool staged = false;  // RESIDENT: this chunk copies a new scene's tables
         if (sg.scene != cur_scene || sg.emitter != cur_emitter) {
             if (!REC) flush();
             row_chunks = 0;
+            const SceneInfo si = p.scenes[sg.scene];
+            const bool staged = RESIDENT && sg.scene != cur_scene;  // this chunk copies a new scene's tables
             if (sg.scene != cur_scene) {
-                si = p.scenes[sg.scene];
-                eps = si.eps;
-                hist_on = !REC && si.n <= kBatchHist;
-                if (hist_on)
-                    for (int i = tid; i < si.n; i += blockDim.x) S.hist[i] = 0;
-                if (RESIDENT) {  // resident tables: two bulk copies, waited for below
-                    // (every thread finished with the previous tables before the chunk's barrier)
-                    if (tid == 0) {
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        const uint32_t tb = (uint32_t)(sizeof(HitRec) * si.n), sb = (uint32_t)(sizeof(float4) * si.n);
-                        bar_expect(&S.bar, tb + sb);
-                        bulk_load(S.tab, p.tab + si.prim_off, tb, &S.bar);
-                        bulk_load(S.bs, p.bsph + si.prim_off, sb, &S.bar);
-                    }
-                    staged = true;
+                for (int i = tid; i < si.n && i < kBatchHist; i += kBatchThreads) S.hist[i] = 0;
+                // resident tables: two bulk copies, waited for below (every thread finished
+                // with the previous tables before the chunk's barrier)
+                if (RESIDENT && tid == 0) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    const uint32_t tb = (uint32_t)(sizeof(HitRec) * si.n), sb = (uint32_t)(sizeof(float4) * si.n);
+                    bar_expect(&S.bar, tb + sb);
+                    bulk_load(S.tab, p.tab + si.prim_off, tb, &S.bar);
+                    bulk_load(S.bs, p.bsph + si.prim_off, sb, &S.bar);
                 }
                 cur_scene = sg.scene;
             }
@@ -789,102 +859,43 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
                     reinterpret_cast<const float *>(p.emit + si.prim_off + sg.emitter)[tid];
             if (tid < kFrameWords) S.frame[tid] = p.frame[(int64_t)(si.prim_off + sg.emitter) * kFrameWords + tid];
             cur_emitter = sg.emitter;
-            mrow = nullptr;
-            if (p.mask_off) {
-                const int64_t mo = p.mask_off[si.prim_off + sg.emitter];
-                if (mo >= 0) mrow = p.cmask + mo;
+            if (tid == 0) {
+                const int64_t mo = p.mask_off ? p.mask_off[si.prim_off + sg.emitter] : -1;
+                S.row.masks = mo >= 0 ? p.cmask + mo : nullptr;
+                S.row.tab = p.tab + si.prim_off;
+                S.row.bs = p.bsph + si.prim_off;
+                S.row.hits = p.hits + si.hits_off + (int64_t)sg.emitter * si.n;
+                S.row.n = si.n;
+                S.row.eps = si.eps;
+                S.row.skip = self_skip(p.emit[si.prim_off + sg.emitter], sg.emitter);
+                S.row.hist = !REC && si.n <= kBatchHist;
+            }
+            if (staged) {  // block-uniform: every thread waits for the copies
+                const bool ok = bar_wait(&S.bar, bar_parity);
+                if (__syncthreads_or(!ok)) {  // gave up: flag it, let the copies land (bounded), stop
+                    if (!ok) bar_wait(&S.bar, bar_parity);
+                    if (tid == 0 && p.err) atomicExch(p.err, 3);
+                    return;
+                }
+                bar_parity ^= 1u;
             }
         }
-        if (RESIDENT && staged) {  // block-uniform: every thread waits for the copies
-            const bool ok = bar_wait(&S.bar, bar_parity);
-            if (__syncthreads_or(!ok)) {  // gave up: flag it, let the copies land (bounded), stop
-                if (!ok) bar_wait(&S.bar, bar_parity);
-                if (tid == 0 && p.err) atomicExch(p.err, 3);
-                return;
-            }
-            bar_parity ^= 1u;
-        }
-        for (int i = tid; i < kCells; i += blockDim.x) S.cnt[i] = 0;
+        for (int i = tid; i < kCells; i += kBatchThreads) S.cnt[i] = 0;
         if (tid == 0) S.next_packet = 0;
         __syncthreads();
-        const int64_t gid0 = (sg.ray_begin >> 2) + (c - sg.chunk_begin) * (int64_t)kChunkDraws;
+        const int64_t gid0 = (sg.ray_begin >> 2) + (c - sg.chunk_begin) * (int64_t)cd;
         const uint32_t sid = (p.compat & RF_COMPAT_STREAMS) ? 0u : (p.scene_id + (uint32_t)sg.scene);
-        const HitRec *gtab = p.tab + si.prim_off;
-        unsigned long long *grow = p.hits + si.hits_off + (int64_t)cur_emitter * si.n;
 
-        if (si.n <= kBruteMax) {  // block-uniform: too few surfaces for culling to pay
-            // every thread traces its own rays against all surfaces in index order
-            const int skip = self_skip(S.emit, cur_emitter);  // block-uniform
-            uint32_t nv_warp = 0;
-#pragma unroll 1
-            for (int g = 0; g < kBatchDraws; ++g) {
-                const int d = g * kBatchThreads + tid;
-                const int64_t gid = gid0 + d;
-                const bool any = gid * 4 + 3 >= sg.ray_begin && gid * 4 < sg.ray_end;
-                const uint4 u = any ? stream_bits(p.compat, p.key1, sid, sg.emitter, gid) : make_uint4(0u, 0u, 0u, 0u);
-                const float uf[4] = {u01(u.x), u01(u.y), u01(u.z), u01(u.w)};
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int64_t rid = gid * 4 + v;
-                    const bool valid = rid >= sg.ray_begin && rid < sg.ray_end;
-                    int bi = -1;
-                    if (valid) {
-                        float r[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) r[i] = uf[(i + v + 1) & 3];
-                        const Ray<float> ray = emit_mixed(S.emit, S.frame, r);
-                        float tb = MFast::inf();
-                        bool dany = false;
-#pragma unroll 1
-                        for (int j = 0; j < si.n; ++j) {
-                            if (j == skip) continue;  // uniform: every thread's emitter
-                            const HitRec h = RESIDENT ? S.tab[j] : load_rec(gtab, j);
-                            const int type = __float_as_int(h.aux.x);
-                            bool defer = false;
-                            int idx;
-                            const float t = test_mixed<STK>(type, h, j, RESIDENT ? S.tab : gtab, RESIDENT, ray, eps, sc,
-                                                            defer, idx);
-                            if (t < tb) { tb = t; bi = idx; }
-                            dany |= defer;
-                            if (STK && is_stack(type)) j = stack_end(h, j) - 1;
-                        }
-                        bi = resolve_brute<STK>(bi, dany, 0, si.n, RESIDENT, S.tab, gtab, ray, eps, sc, skip, nref);
-                    }
-                    // all 32 lanes reach the warp-wide calls below
-                    if (COUNT) nv_warp += __popc(__ballot_sync(0xffffffffu, valid));
-                    if (REC) {
-                        if (valid) p.rec[gid0 * 4 + 4 * d + v - p.rec_base] = bi;
-                    } else if (hist_on) {
-                        warp_tally(S.hist, bi);
-                    } else {
-                        warp_tally_global(grow, bi);
-                    }
-                }
-            }
-            if (COUNT) {
-                if (lane == 0 && nv_warp)
-                    for (int j = 0; j < si.n; ++j) {
-                        if (j == skip) continue;
-                        const HitRec h = RESIDENT ? S.tab[j] : load_rec(gtab, j);
-                        const int type = __float_as_int(h.aux.x);
-                        if (STK && is_stack(type)) {
-                            S.wcount[warp][type == kStackType ? RF_CYLINDER : RF_ANNULUS] += nv_warp;
-                            j = stack_end(h, j) - 1;
-                        } else if ((unsigned)type < 6u) {
-                            S.wcount[warp][type] += nv_warp;
-                        }
-                    }
-                fold_counts();
-            }
+        if (S.row.n <= kBruteMax) {  // block-uniform
+            nref += brute_chunk<REC, RESIDENT, COUNT, STK>(S, p, sg.emitter, sg.ray_begin, sg.ray_end, gid0, cd, sid);
+            fold_counts();
             __syncthreads();
             continue;
         }
 
-        // 1. uniforms and sort keys (draw d = g*blockDim + tid, ray l = 4d + v);
-        // keys go to perm[l] until the sort
+        // 1. uniforms and sort keys (draw d, ray l = 4d + v); keys go to perm[l] until the sort
 #pragma unroll 1
-        for (int g = 0; g < kBatchDraws; ++g) {
-            const int d = g * kBatchThreads + tid;
+        for (int d = tid; d < cd; d += kBatchThreads) {
             const int64_t gid = gid0 + d;
             uint2 kk = make_uint2(kCells | (kCells << 16), kCells | (kCells << 16));  // no valid ray
             if (gid * 4 + 3 >= sg.ray_begin && gid * 4 < sg.ray_end) {
@@ -895,8 +906,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
                     float r[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) r[i] = uf[(i + v + 1) & 3];
+                    rotate_uniforms(uf, v, r);
                     const Ray<float> ray = emit_mixed(S.emit, S.frame, r);  // the origin is dead code here
                     const int64_t rid = gid * 4 + v;
                     const bool valid = rid >= sg.ray_begin && rid < sg.ray_end;
@@ -912,7 +922,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
         uint2 mykeys[kBatchDraws];
 #pragma unroll
         for (int g = 0; g < kBatchDraws; ++g)
-            mykeys[g] = *reinterpret_cast<const uint2 *>(&S.perm[4 * (g * kBatchThreads + tid)]);
+            if (g * kBatchThreads + tid < cd)
+                mykeys[g] = *reinterpret_cast<const uint2 *>(&S.perm[4 * (g * kBatchThreads + tid)]);
         // 2. counting sort: block-wide exclusive scan of the bucket sizes (four
         // consecutive buckets per thread), then each ray claims a slot of its
         // bucket (in any order: a ray's result does not depend on its packet)
@@ -947,37 +958,36 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
 #pragma unroll
         for (int g = 0; g < kBatchDraws; ++g) {
             const int d = g * kBatchThreads + tid;
+            if (d < cd) {
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const uint32_t w = (v < 2) ? mykeys[g].x : mykeys[g].y;
-                const int key = (int)((w >> (16 * (v & 1))) & 0xffffu);
-                if (key < kCells) S.perm[atomicAdd(&S.cnt[key], 1)] = (uint16_t)(4 * d + v);
+                for (int v = 0; v < 4; ++v) {
+                    const uint32_t w = (v < 2) ? mykeys[g].x : mykeys[g].y;
+                    const int key = (int)((w >> (16 * (v & 1))) & 0xffffu);
+                    if (key < kCells) S.perm[atomicAdd(&S.cnt[key], 1)] = (uint16_t)(4 * d + v);
+                }
             }
         }
         __syncthreads();
-        const int n_valid = S.n_valid;
 
         // 3-5. warps take packets of 32 sorted rays; candidates are the union of
         // the rays' cell masks (or the surfaces the packet's bounds can reach);
         // each candidate gets the lanes' own gates and, if any lane passes, the
         // full test (index order, so ties go to the lower index as in
         // RayFactorGPU.cl:463-467); first hits are tallied at once
-        constexpr bool resident = RESIDENT;
-        const float4 *gbs = p.bsph + si.prim_off;
-        const int n_packets = (n_valid + 31) >> 5;
-        const int nwords_all = (si.n + 31) >> 5;
         for (;;) {
             int k = 0;
             if (lane == 0) k = atomicAdd(&S.next_packet, 1);
             k = __shfl_sync(0xffffffffu, k, 0);
-            if (k >= n_packets) break;  // warp-uniform
+            const int n_valid = S.n_valid;
+            if (k * 32 >= n_valid) break;  // warp-uniform
             const int pos = k * 32 + lane;
             const bool valid = pos < n_valid;
             const int nvalid = COUNT ? __popc(__ballot_sync(0xffffffffu, valid)) : 0;  // every lane
-            int bi = -1;
+            // re-emit the lane's ray (an invalid lane traces the packet's first ray)
+            const int l = S.perm[valid ? pos : k * 32];
+            Ray<float> ray;
+            int cell = 0;
             {
-                // re-emit the lane's ray (an invalid lane traces the packet's first ray)
-                const int l = S.perm[valid ? pos : k * 32];
                 const int d = l >> 2, v = l & 3;
                 float uf[4], r[4];
                 unpack_uniforms(S.unif[0][d], S.unif[1][d], S.unif[2][d], uf);
@@ -986,101 +996,106 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const TracePa
                     const int q = (i + v + 1) & 3;
                     r[i] = q == 0 ? uf[0] : (q == 1 ? uf[1] : (q == 2 ? uf[2] : uf[3]));
                 }
-                const Ray<float> ray = emit_mixed(S.emit, S.frame, r);
-                const float idd = MFast::rcp(ray.cx * ray.cx + ray.cy * ray.cy + ray.cz * ray.cz);
-                const uint32_t *mcell = mrow ? mrow + (int64_t)ray_key(ray, r) * nwords_all : nullptr;
-                {
-                    float tb = MFast::inf();
-                    int dj = -1, ndef = 0;  // deferred FP64 tests of this lane: the last one, and how many
-                    if (COUNT && lane == 0) S.wcount[warp][7] += 1;
-                    // surfaces in blocks of 1024 (one block when the scene has masks)
-                    int skip_to = 0;  // members of a stack already tested are not candidates
+                ray = emit_mixed(S.emit, S.frame, r);
+                cell = ray_key(ray, r);
+            }
+            const float idd = MFast::rcp(ray.cx * ray.cx + ray.cy * ray.cy + ray.cz * ray.cz);
+            const float eps = S.row.eps;
+            const bool masked = row_masks(S) != nullptr;  // block-uniform
+            const int moff = cell * ((S.row.n + 31) >> 5);  // the lane's first mask word
+            float tb = MFast::inf();
+            int bi = -1;
+            if (COUNT && lane == 0) S.wcount[warp][7] += 1;
+            // surfaces in blocks of 1024 (one block when the scene has masks)
+            int skip_to = 0;  // members of a stack already tested are not candidates
 #pragma unroll 1
-                    for (int j0 = 0; j0 < si.n; j0 += 1024) {
-                        const int nwords = min(32, (si.n - j0 + 31) >> 5);
-                        unsigned cmask = 0u;  // without masks: lane w holds candidate word w
-                        if (!mcell) {  // block-uniform
-                            const Packet pk = packet_bounds(ray, idd);
-                            const int self = self_skip(S.emit, cur_emitter);  // (masks leave it out already)
+            for (int j0 = 0; j0 < S.row.n; j0 += 1024) {
+                const int nwords = min(32, (S.row.n - j0 + 31) >> 5);
+                unsigned cmask = 0u;  // without masks: lane w holds candidate word w
+                if (!masked) {
+                    const Packet pk = packet_bounds(ray, idd);
 #pragma unroll 1
-                            for (int w = 0; w < nwords; ++w) {
-                                const int js = j0 + (w << 5) + lane;
-                                bool cand = false;
-                                if (js < si.n && js != self)
-                                    cand = packet_may_hit(pk, resident ? S.bs[js] : __ldg(gbs + js));
-                                const unsigned cm = __ballot_sync(0xffffffffu, cand);
-                                if (lane == w) cmask = cm;
-                            }
-                        }
-#pragma unroll 1
-                        for (int w = 0; w < nwords; ++w) {
-                            const int jw = j0 + (w << 5);
-                            const unsigned cm0 = mcell ? __reduce_or_sync(0xffffffffu, __ldg(mcell + (jw >> 5)))
-                                                       : __shfl_sync(0xffffffffu, cmask, w);  // block-uniform choice
-                            unsigned cm = STK ? cm0 & keep_from(skip_to - jw) : cm0;
-                            // two candidates per pass: their sphere checks are independent
-                            // chains (latency hidden); tests still run in index order
-                            while (cm) {  // cm is the same in every lane
-                                const int ba_ = __ffs(cm) - 1;
-                                cm &= cm - 1;
-                                const int bb_ = cm ? __ffs(cm) - 1 : -1;
-                                cm &= cm - 1;  // 0 stays 0
-                                const int ja = jw + ba_, jb = jw + (bb_ >= 0 ? bb_ : ba_);
-                                if (COUNT && lane == 0) S.wcount[warp][6] += bb_ >= 0 ? 2 : 1;  // candidates checked
-                                const float4 sa = resident ? S.bs[ja] : __ldg(gbs + ja);
-                                const float4 sb = resident ? S.bs[jb] : __ldg(gbs + jb);
-                                const bool ma = ray_may_hit(ray, idd, sa);
-                                const bool mb = bb_ >= 0 && ray_may_hit(ray, idd, sb);
-                                const unsigned va = __ballot_sync(0xffffffffu, ma);
-                                unsigned vb = __ballot_sync(0xffffffffu, mb);
-#pragma unroll
-                                for (int q = 0; q < 2; ++q) {
-                                    if (!(q ? vb : va)) continue;  // warp-uniform
-                                    const int j = q ? jb : ja;
-                                    const HitRec h = resident ? S.tab[j] : load_rec(gtab, j);
-                                    const int type = __float_as_int(h.aux.x);
-                                    if (COUNT) tcount += lane == stat_type(type) ? nvalid : 0;
-                                    bool defer = false;
-                                    int idx = j;
-                                    const float t = STK ? hit_hot(type, h, j, resident ? S.tab : gtab, resident, ray, eps,
-                                                                  sc, defer, idx, jw, cm, skip_to, q ? INT_MAX : jb, vb)
-                                                        : hit_mixed(type, h, ray, eps, sc, defer);
-                                    if (t < tb) { tb = t; bi = idx; }
-                                    ndef += defer;  // predicated, no branch
-                                    dj = defer ? j : dj;
-                                }
-                            }
-                        }
-                    }
-                    // The lane's result must be its nearest hit among the surfaces its own
-                    // gate admits (the set its cell mask and sphere check select), which
-                    // depends on the ray alone.  The loop above took the nearest over the
-                    // packet's tested surfaces, a superset; when the winner passes the
-                    // lane's gate it is also the nearest of the gated set (same index-order
-                    // ties), otherwise -- or when the lane deferred more than one test --
-                    // the lane re-traces over its gated set (cold).  A single deferred test
-                    // is re-evaluated in FP64 (lower index wins a tie: it ran out of order).
-                    bool retrace = valid && ndef > 1;
-                    if (valid && ndef == 1) {
-                        const HitRec hq = RESIDENT ? S.tab[dj] : load_rec(gtab, dj);
-                        int dq;
-                        const float t = test_f64<STK>(hq, dj, ray, eps, sc, dq);
-                        if (t < tb || (t == tb && bi >= 0 && dq < bi)) { tb = t; bi = dq; }
-                        ++nref;
-                        retrace = !own_gate(mcell, dj, ray, idd, resident ? S.bs[dj] : __ldg(gbs + dj));
-                    }
-                    if (valid && !retrace && bi >= 0)
-                        retrace = !own_gate(mcell, bi, ray, idd, resident ? S.bs[bi] : __ldg(gbs + bi));
-                    if (retrace) {
-                        bi = retrace_f64<STK>(0, si.n, RESIDENT, S.tab, gtab, S.bs, gbs, mcell, true, ray, idd, eps, sc,
-                                         self_skip(S.emit, cur_emitter), nref);
+                    for (int w = 0; w < nwords; ++w) {
+                        const int js = j0 + (w << 5) + lane;
+                        bool cand = false;
+                        if (js < S.row.n && js != S.row.skip)  // (masks leave the emitter out already)
+                            cand = packet_may_hit(pk, RESIDENT ? S.bs[js] : __ldg(S.row.bs + js));
+                        const unsigned cm = __ballot_sync(0xffffffffu, cand);
+                        if (lane == w) cmask = cm;
                     }
                 }
-                if (REC && valid) p.rec[gid0 * 4 + l - p.rec_base] = bi;
+#pragma unroll 1
+                for (int w = 0; w < nwords; ++w) {
+                    const int jw = j0 + (w << 5);
+                    unsigned cm = masked ? __reduce_or_sync(0xffffffffu, __ldg(row_masks(S) + moff + (jw >> 5)))
+                                         : __shfl_sync(0xffffffffu, cmask, w);
+                    if (STK) cm &= keep_from(skip_to - jw);
+                    // two candidates per pass: their sphere checks are independent chains
+                    // (latency hidden); tests still run in index order
+                    while (cm) {  // cm is the same in every lane
+                        const int ba_ = __ffs(cm) - 1;
+                        cm &= cm - 1;
+                        const int bb_ = cm ? __ffs(cm) - 1 : ba_;
+                        unsigned go = cm ? 3u : 1u;
+                        cm &= cm - 1;  // 0 stays 0
+                        const int ja = jw + ba_, jb = jw + bb_;
+                        if (COUNT && lane == 0) S.wcount[warp][6] += go > 1u ? 2 : 1;  // candidates checked
+                        const bool ma = ray_may_hit(ray, idd, RESIDENT ? S.bs[ja] : __ldg(S.row.bs + ja));
+                        const bool mb = ray_may_hit(ray, idd, RESIDENT ? S.bs[jb] : __ldg(S.row.bs + jb));
+                        if (!__any_sync(0xffffffffu, ma)) go &= ~1u;
+                        if (!__any_sync(0xffffffffu, mb)) go &= ~2u;
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            if (!((go >> q) & 1u)) continue;  // warp-uniform
+                            const int j = q ? jb : ja;
+                            const HitRec h = RESIDENT ? S.tab[j] : load_rec(S.row.tab, j);
+                            const int type = __float_as_int(h.aux.x);
+                            if (COUNT) tcount += lane == stat_type(type) ? nvalid : 0;
+                            bool defer = false;
+                            int idx = j;
+                            float t;
+                            if (STK && is_stack(type)) {  // its other members are done with it
+                                t = test_mixed<true>(type, h, j, RESIDENT ? S.tab : S.row.tab, RESIDENT, ray, eps, sc, defer,
+                                                     idx);
+                                skip_to = stack_end(h, j);
+                                cm &= keep_from(skip_to - jw);
+                                if (jb < skip_to) go &= 1u;
+                            } else {
+                                t = hit_mixed(type, h, ray, eps, sc, defer);
+                            }
+                            // ill-conditioned for some lane (a few rays in a million): FP64 at once
+                            if (__any_sync(0xffffffffu, defer) && defer) {
+                                const float2 f = deferred_f64((RESIDENT ? S.tab : S.row.tab) + j, j, ray, eps, sc);
+                                t = f.x;
+                                idx = __float_as_int(f.y);
+                                nref += valid;
+                            }
+                            if (t < tb) { tb = t; bi = idx; }
+                        }
+                    }
+                }
             }
-            if (!REC) {  // every lane: warp-aggregated tally
-                if (hist_on) warp_tally(S.hist, valid ? bi : -1);
-                else warp_tally_global(grow, valid ? bi : -1);
+            // The lane's result must be its nearest hit among the surfaces its own
+            // gate admits (the set its cell mask and sphere check select), which
+            // depends on the ray alone.  The loop above took the nearest over the
+            // packet's tested surfaces, a superset; when the winner passes the
+            // lane's gate it is also the nearest of the gated set (same index-order
+            // ties), otherwise the lane re-traces over its gated set (cold).
+            if (valid && bi >= 0) {
+                const uint32_t *mcell = masked ? row_masks(S) + moff : nullptr;
+                if (!own_gate(mcell, bi, ray, idd, RESIDENT ? S.bs[bi] : __ldg(S.row.bs + bi))) {
+                    const int2 q = retrace_f64<STK>(S.row.n, RESIDENT ? S.tab : S.row.tab, RESIDENT ? S.bs : S.row.bs,
+                                                    mcell, ray, idd, eps, sc, S.row.skip);
+                    bi = q.x;
+                    nref += q.y;
+                }
+            }
+            if (REC) {
+                if (valid) p.rec[gid0 * 4 + l - p.rec_base] = bi;
+            } else if (S.row.hist) {  // every lane: warp-aggregated tally
+                warp_tally(S.hist, valid ? bi : -1);
+            } else {
+                warp_tally_global(S.row.hits, valid ? bi : -1);
             }
         }
         fold_counts();

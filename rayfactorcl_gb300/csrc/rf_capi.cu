@@ -329,16 +329,9 @@ rf_status ensure_culled(rf_ctx *c)
     return RF_OK;
 }
 
-// Draws per chunk of the culled kernel: about four chunks per SM, so that the last
-// ones end together, within what a block's shared memory holds and what its
-// threads need (64 surfaces EXACT, ms at 1024 / 2048 / 4096 / 8192 draws: 1e8 rays
-// 8.2 / 7.0 / 6.3 / 5.9, 1e7 rays 0.86 / 0.76 / 0.71 / 0.73, 1e6 rays 0.127 / 0.124 /
-// 0.21 / 0.33: larger chunks sort into more similar packets).
 int culled_chunk(const rf_ctx *c, int64_t draws)
 {
-    const int64_t want = (draws / (4 * (int64_t)c->sms) + 255) / 256 * 256;
-    const int64_t least = c->cfg.precision == RF_PREC_FP64 ? 512 : 1024;  // one draw per thread
-    return (int)std::max(least, std::min<int64_t>(kBatchChunkDraws, want));
+    return chunk_for(draws, c->sms, c->cfg.precision == RF_PREC_FP64 ? 512 : 1024);
 }
 
 // Launch shape for the single-scene kernels.
@@ -913,7 +906,7 @@ struct BatchCounters {
     int64_t total;
     int32_t nseg;
     int32_t flags[2];  // not-converged rows, rounds
-    int32_t pad;
+    int32_t chunk;     // draws per chunk of the round
     unsigned long long work[8];
 };
 
@@ -958,9 +951,11 @@ int batched_grid(rf_ctx *c, bool rec)
     return c->cfg.batched_grid > 0 ? std::min(wave, (int)c->cfg.batched_grid) : wave;
 }
 
+bool mixed_culled(const rf_ctx *c, bool bv);
+
 // One persistent launch over host-planned segments.
 rf_status run_batched(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec,
-                      int32_t *d_rec, int64_t rec_base, bool zero_hits, bool bv = false, int chunk_draws = 0)
+                      int32_t *d_rec, int64_t rec_base, bool zero_hits, bool bv, int64_t chunk_draws)
 {
     c->last_small = false;
     c->last_launches = 0;
@@ -977,14 +972,14 @@ rf_status run_batched(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_
     p.rec_base = rec_base;
     const int grid = (int)std::min<int64_t>(batched_grid(c, rec), total_chunks);
     RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    if (chunk_draws > 0) {  // the culled kernel
+    p.chunk_draws = (int)chunk_draws;
+    if (mixed_culled(c, bv)) {
         p.bvtab = c->b_bvtab.as<HitRec>();
         p.bvinfo = c->b_bvinfo.as<int4>();
         p.bvsph = c->b_bvsph.as<float4>();
         p.nbv = c->nbv;
         p.n = c->n;
         p.eps = c->b_info[0].eps;
-        p.chunk_draws = chunk_draws;
         p.use_smem_hist = 1;
         RF_CUDA(c, launch_mixed_culled(p, bv, rec, c->cfg.work_counts != 0, grid, c->stream));
     } else {
@@ -1025,14 +1020,13 @@ int small_gpt(const rf_ctx *c, bool rec, bool bv = false)
 // surfaces, and with segment stacks, whose members it need not look at.
 bool mixed_culled(const rf_ctx *c, bool bv)
 {
-    return !small_trace(c, bv) && (bv || (c->b_stacks > 0 && c->n <= kBatchTile));
+    return c->b_single && !small_trace(c, bv) && (bv || (c->b_stacks > 0 && c->n <= kBatchTile));
 }
 
 // Draws per chunk of a MIXED trace of so many draws.
 int64_t mixed_chunk_draws(const rf_ctx *c, bool rec, bool bv, int64_t draws)
 {
-    if (mixed_culled(c, bv)) return culled_chunk(c, draws);
-    return small_trace(c, bv) ? (int64_t)kSmallThreads * small_gpt(c, rec, bv) : (int64_t)kBatchChunkDraws;
+    return small_trace(c, bv) ? (int64_t)kSmallThreads * small_gpt(c, rec, bv) : chunk_for(draws, c->sms, 1024);
 }
 
 // One launch of the small-scene kernel over host-planned segments (chunks of
@@ -1094,9 +1088,8 @@ rf_status run_small(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
 rf_status run_mixed(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec, int32_t *d_rec,
                     int64_t rec_base, bool zero_hits, bool bv, int64_t chunk_draws)
 {
-    if (mixed_culled(c, bv)) return run_batched(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, bv, (int)chunk_draws);
     if (small_trace(c, bv)) return run_small(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, bv);
-    return run_batched(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits);
+    return run_batched(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, bv, chunk_draws);
 }
 
 // Can the mixed kernel trace this scene with its bounding surfaces?
@@ -1826,14 +1819,18 @@ rf_status rf_trace_batch(rf_ctx *c, const rf_scene_desc *scenes, int32_t n_scene
     c->b_single = false;
     c->have_results = false;
     std::vector<Segment> seg;
-    int64_t chunks = 0, nrows = 0;
+    int64_t chunks = 0, nrows = 0, draws = 0;
     for (int s = 0; s < n_scenes; ++s) {
         if ((st = check_budgets(c, scenes[s].rays_per_emitter, scenes[s].n_prims)) != RF_OK) return st;
+        draws += total_draws(scenes[s].rays_per_emitter, scenes[s].n_prims);
+    }
+    const int cg = chunk_for(draws, c->sms, 1024);
+    for (int s = 0; s < n_scenes; ++s) {
         for (int e = 0; e < scenes[s].n_prims; ++e)
-            chunks = plan_segments(seg, e, s, 0, scenes[s].rays_per_emitter[e], kBatchChunkDraws, chunks);
+            chunks = plan_segments(seg, e, s, 0, scenes[s].rays_per_emitter[e], cg, chunks);
         nrows += scenes[s].n_prims;
     }
-    if ((st = run_batched(c, seg, chunks, false, nullptr, 0, true)) != RF_OK) return st;
+    if ((st = run_batched(c, seg, chunks, false, nullptr, 0, true, false, cg)) != RF_OK) return st;
     // FP64 normalisation of every row (one warp per row)
     std::vector<int64_t> rows(3 * nrows);
     int64_t r = 0;
@@ -1909,6 +1906,7 @@ rf_status rf_converge_batch(rf_ctx *c, const rf_scene_desc *scenes, int32_t n_sc
     p.seg = c->d_seg.as<Segment>();
     p.d_total = &bc->total;
     p.d_nseg = &bc->nseg;
+    p.d_chunk = &bc->chunk;
     const int grid = batched_grid(c, false);  // also sets the kernel's shared-memory attribute
 
     // Graph: while (not converged && rounds < max) { plan; trace; converge; decide }
@@ -1918,7 +1916,7 @@ rf_status rf_converge_batch(rf_ctx *c, const rf_scene_desc *scenes, int32_t n_sc
     auto body_ops = [&](unsigned long long h) -> cudaError_t {
         cudaError_t e;
         if ((e = launch_plan_round(nrows, d_sc, d_em, d_total, d_next, c->d_seg.as<Segment>(), &bc->nseg, &bc->total, &bc->queue,
-                                   kBatchChunkDraws, c->stream)) != cudaSuccess) return e;
+                                   c->sms, &bc->chunk, c->stream)) != cudaSuccess) return e;
         if ((e = launch_batched(p, false, batch_resident(c), c->cfg.work_counts != 0, c->b_stacks > 0, grid,
                                 c->stream)) != cudaSuccess)
             return e;

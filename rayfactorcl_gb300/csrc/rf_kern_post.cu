@@ -121,15 +121,28 @@ cudaError_t launch_converge_step(const unsigned long long *hits, int64_t *rays,
 
 // One round of the convergence loop, planned on the device: every row with
 // next[r] > 0 rays to add becomes a segment continuing its stream at
-// rays_total[r]; chunks are numbered across segments; the work queue is reset.
+// rays_total[r]; chunks, sized for the round's rays (the last rounds' few rows would
+// otherwise be a few long chunks on as many SMs), are numbered across segments; the
+// work queue is reset.
 __global__ void plan_round_kernel(int64_t nrows, const int32_t *row_scene, const int32_t *row_emitter,
                                   int64_t *rays_total, const int64_t *next, Segment *seg, int32_t *d_nseg,
-                                  int64_t *d_total, unsigned long long *queue, int chunk_draws)
+                                  int64_t *d_total, unsigned long long *queue, int sms, int32_t *d_chunk)
 {
     __shared__ int64_t s_chunks[1024];
     __shared__ int32_t s_nz[1024];
     const int tid = threadIdx.x, T = blockDim.x;
     const int64_t lo = nrows * tid / T, hi = nrows * (tid + 1) / T;
+    int64_t draws = 0;
+    for (int64_t r = lo; r < hi; ++r)
+        if (next[r] > 0) draws += (next[r] + 3) >> 2;
+    s_chunks[tid] = draws;
+    __syncthreads();
+    for (int o = T / 2; o; o >>= 1) {
+        if (tid < o) s_chunks[tid] += s_chunks[tid + o];
+        __syncthreads();
+    }
+    const int chunk_draws = chunk_for(s_chunks[0], sms, 1024);
+    __syncthreads();
     int64_t chunks = 0;
     int32_t nz = 0;
     for (int64_t r = lo; r < hi; ++r) {
@@ -170,15 +183,16 @@ __global__ void plan_round_kernel(int64_t nrows, const int32_t *row_scene, const
         *d_nseg = s_nz[T - 1];
         *d_total = s_chunks[T - 1];
         *queue = 0ull;
+        *d_chunk = chunk_draws;
     }
 }
 
 cudaError_t launch_plan_round(int64_t nrows, const int32_t *row_scene, const int32_t *row_emitter,
                               int64_t *rays_total, const int64_t *next, Segment *seg, int32_t *d_nseg,
-                              int64_t *d_total, unsigned long long *queue, int chunk_draws, cudaStream_t st)
+                              int64_t *d_total, unsigned long long *queue, int sms, int32_t *d_chunk, cudaStream_t st)
 {
     plan_round_kernel<<<1, 1024, 0, st>>>(nrows, row_scene, row_emitter, rays_total, next, seg, d_nseg,
-                                          d_total, queue, chunk_draws);
+                                          d_total, queue, sms, d_chunk);
     return cudaGetLastError();
 }
 

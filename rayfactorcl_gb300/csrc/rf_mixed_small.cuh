@@ -152,8 +152,7 @@ __global__ void __launch_bounds__(kSmallThreads, GPT == 1 ? 4 : 1) mixed_small_k
         for (int k = 0; k < R; ++k) {
             const int64_t rid = (gid0 + (int64_t)(k >> 2) * blockDim.x + tid) * 4 + (k & 3);
             const bool valid = rid >= sg.ray_begin && rid < sg.ray_end;
-            const int h = valid ? resolve_brute<true>(bi[k], (dmask >> k) & 1u, 0, n, true, s_tab, nullptr, ray[k], eps, sc,
-                                                skip, nref)
+            const int h = valid ? resolve_brute<true>(bi[k], (dmask >> k) & 1u, 0, n, s_tab, ray[k], eps, sc, skip, nref)
                                 : -1;
             if (REC) {
                 if (valid) p.rec[rid - p.rec_base] = h;
@@ -268,7 +267,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4) mixed_small_bv_kernel(const 
                     dr |= defer;
                     if (is_stack(type)) j = stack_end(h, j) - 1;
                 }
-                return resolve_brute<true>(br, dr, lo, hi, true, s_tab, nullptr, ray, eps, sc, skip, nref);
+                return resolve_brute<true>(br, dr, lo, hi, s_tab, ray, eps, sc, skip, nref);
             };
             const int h = valid ? bv_select(s_bvtab, s_bvinfo, s_bvbs, p.nbv, ray, eps, sc, stale, find) : -1;
             if (REC) {

@@ -10,6 +10,7 @@
 // prepared surface tables, the segment plan and the work-queue counters) lives
 // in one file-scope device array of RF_NOALLOC_SCRATCH_BYTES, which every GPU
 // that loads this library holds until the process exits.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -106,7 +107,9 @@ extern "C" rf_status rf_trace_mixed_noalloc(const rf_primitive *prims, int32_t n
     const int nstacks = prepare_mixed_tables(prims, n, eps, compat, h_emit, h_tab, h_sph, &seps);
     for (int i = 0; i < n; ++i) emit_frame(h_emit[i], h_frame + (size_t)i * kEmitFrameWords);
     int nseg = 0;
-    int64_t chunks = 0;
+    int64_t chunks = 0, total = 0;
+    for (int e = 0; e < n; ++e) total += (std::max<int64_t>(rays[e], 0) + 3) >> 2;
+    const int cd = chunk_for(total, sms, 1024);
     for (int e = 0; e < n; ++e) {
         if (rays[e] <= 0) continue;
         Segment sg;
@@ -117,7 +120,7 @@ extern "C" rf_status rf_trace_mixed_noalloc(const rf_primitive *prims, int32_t n
         sg.chunk_begin = chunks;
         h_seg[nseg++] = sg;
         const int64_t draws = (rays[e] + 3) >> 2;
-        chunks += (draws + kBatchChunkDraws - 1) / kBatchChunkDraws;
+        chunks += (draws + cd - 1) / cd;
     }
     SceneInfo si{};
     si.n = n;
@@ -154,6 +157,7 @@ extern "C" rf_status rf_trace_mixed_noalloc(const rf_primitive *prims, int32_t n
     p.refined = &cnt->refined;
     p.work = cnt->work;
     p.total_chunks = chunks;
+    p.chunk_draws = cd;
     p.nseg = nseg;
     p.compat = compat;
     p.key1 = key1;
