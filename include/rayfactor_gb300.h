@@ -287,8 +287,8 @@ rf_status rf_autotune(rf_ctx *ctx, int32_t use_bv, const char *cache_path);
 
 /* (No counterpart in the reference.)  The launch shape the context uses now (after rf_autotune, or the defaults).
  * RF_PREC_MIXED: the kernel the next trace of the current scene without bounding surfaces takes -- block
- * 1024 and 32 rays per thread for the batched kernel, 256 and 4 or 8 for the small-scene kernel (with
- * bounding surfaces it is always the batched kernel). */
+ * 1024 and 32 rays per thread for the batched kernel, 256 and 4 or 8 for the small-scene kernel.  Traces
+ * that sort rays into packets and traces of few rays have launch shapes of their own, whatever this says. */
 rf_status rf_get_launch_config(rf_ctx *ctx, int32_t *block, int32_t *rays_per_thread,
                                int32_t *smem_hist, int32_t *smem_table, int32_t *one_ray_at_a_time);
 

@@ -39,7 +39,8 @@ UNITS = {
     "rf_masks.cu": [],
     "rf_noalloc.cu": [],
 }
-HEADERS = ["rf_internal.h", "rf_device.cuh", "rf_trace_kernels.cuh", "rf_batched.cuh", "rf_mixed_small.cuh", "rf_culled.cuh"]
+HEADERS = ["rf_internal.h", "rf_device.cuh", "rf_trace_kernels.cuh", "rf_batched.cuh", "rf_mixed_small.cuh",
+           "rf_culled.cuh", "rf_narrow.cuh"]
 
 
 def nvcc() -> str:

@@ -277,7 +277,11 @@ struct Plan {
     bool hist = false;
     bool stage = true;
     int chunk_draws = 0;  // > 0: the culled kernel, with chunks of this many draws
-    int64_t chunk_gids() const { return chunk_draws > 0 ? chunk_draws : (int64_t)lc.block * lc.gpt; }
+    int split = 0;        // > 0: the narrow kernel
+    int64_t chunk_gids() const
+    {
+        return split > 0 ? 64 / split : (chunk_draws > 0 ? chunk_draws : (int64_t)lc.block * lc.gpt);
+    }
 };
 
 // The culled kernel (rf_culled.cuh) takes a trace when the scene's bounds leave
@@ -309,6 +313,56 @@ bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
     return n >= 128 || (n >= 16 && rays >= 400000) || (n >= 24 && rays <= 400 * n);
 }
 
+// The narrow kernel (rf_narrow.cuh) takes traces of few rays, unless a launch shape of
+// another kernel is pinned: how many warps share a ray's surfaces, 0 for the other
+// kernels.  Best split against the kernel that took the trace before, measured, us:
+//   EXACT  surfaces: 3 at 6e4 rays 8.4 / 10.2, at 1.5e5 12.1 / 10.5; 20 at 1e4 9.6 / 24; 64 at
+//     1.5e5 43 / 65, at 2e5 59 / 66, at 3e5 66 / 84; 201 at 2e5 157 / 201, at 3e5 219 / 206; 400
+//     at 1e4 35 / 230, at 1e5 160 / 304; 252 rings that the culled kernel searches as one
+//     stack at 1e4 22 / 48, at 1e5 92 / 92, at 2e5 186 / 97
+//   FAST  3 at 2.5e4 7.8 / 7.8, at 4.9e4 9.6 / 7.9; 32 at 1.5e5 19 / 26, at 2e5 28 / 26; 201 at 2e5 116 / 163, at 3e5 163 / 163
+//   MIXED  12 at 2e5 20 / 26; 32 at 2e5 36 / 39, at 3e5 41 / 39; 64 at 6e4 26 / 45, at 1.5e5
+//     47 / 49; 201 at 6e4 61 / 86, at 1.5e5 127 / 116; rings in stacks at 2e5 47 / 57; 1000 (no
+//     longer in the batched kernel's shared memory) at 2e5 854 / 1339
+//   FP64  3 at 1e4 24 / 94; 12 at 4e4 144 / 251; 32 at 4e4 297 / 359; 64 at 2e4 300 / 318, at 4e4
+//     457 / 524; 100 at 1e4 246 / 214
+int narrow_split(const rf_ctx *c, bool bv, int64_t draws)
+{
+    const rf_config &f = c->cfg;
+    const int n = c->n;
+    if (bv || c->tuning || f.block_size || f.rays_per_thread || f.tally_mode || f.table_mode || f.test_order ||
+        f.batched_grid || f.work_counts || n > kNarrowMax)
+        return 0;
+    const int64_t rays = 4 * draws;
+    int64_t most;
+    switch (f.precision) {
+    case RF_PREC_FP64: most = n <= 64 ? std::min<int64_t>(50000, 1200000 / n) : 0; break;
+    case RF_PREC_FAST: most = n < 200 ? 160000 : 220000; break;
+    case RF_PREC_MIXED: most = n <= 40 || n > kBatchTile || c->b_stacks > 0 ? 200000 : 90000; break;
+    default: most = n < 128 ? 220000 : 100000; break;
+    }
+    if (rays > std::min<int64_t>(most, 16000 * n)) return 0;
+    if (f.precision == RF_PREC_FP64) {  // its pipe is full at a warp a scheduler: no more warps than that
+        int s = 8;
+        while (s > 1 && rays * s > 160 * (int64_t)c->sms) s /= 2;
+        return s;
+    }
+    // passes of the resident blocks x what a ray costs a warp: its part of the tests, and an
+    // emission of about 16 tests (64 surfaces, 1.5e5 rays, EXACT, split 1 2 4 8: 60 43 49 58 us;
+    // 400 surfaces, 1e4 rays: 145 90 49 35)
+    int best = 1;
+    int64_t least = INT64_MAX;
+    for (int s = 1; s <= 8; s *= 2) {
+        const int64_t chunks = rays * s / kNarrowThreads + n, blocks = kNarrowBlocks * (int64_t)c->sms;
+        const int64_t cost = (chunks + blocks - 1) / blocks * (n / s + 16);
+        if (cost < least) {
+            least = cost;
+            best = s;
+        }
+    }
+    return best;
+}
+
 rf_status ensure_culled(rf_ctx *c)
 {
     const size_t n = c->n, words = 8 * n + c->nbv;  // float4
@@ -338,7 +392,8 @@ int culled_chunk(const rf_ctx *c, int64_t draws)
 Plan make_plan(const rf_ctx *c, bool bv, bool rec, int64_t draws)
 {
     Plan pl;
-    if (c->cull > 0 && culled_pays(c, bv, draws)) pl.chunk_draws = culled_chunk(c, draws);
+    pl.split = narrow_split(c, bv, draws);
+    if (pl.split == 0 && c->cull > 0 && culled_pays(c, bv, draws)) pl.chunk_draws = culled_chunk(c, draws);
     pl.lc.bv = bv;
     pl.lc.rec = rec;
     pl.lc.block = c->block > 0 ? c->block : (c->cfg.block_size > 0 ? c->cfg.block_size : kBlock);
@@ -438,6 +493,18 @@ rf_status run_trace(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
     p.use_smem_hist = pl.hist ? 1 : 0;
 
     const int arith = arith_of(c);
+    if (pl.split > 0) {
+        RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+        switch (arith) {
+        case RF_PREC_EXACT: RF_CUDA(c, launch_narrow<MExact>(p, pl.split, pl.lc.rec, c->sms, c->stream)); break;
+        case RF_PREC_FP64: RF_CUDA(c, launch_narrow<MF64>(p, pl.split, pl.lc.rec, c->sms, c->stream)); break;
+        default: RF_CUDA(c, launch_narrow<MFast>(p, pl.split, pl.lc.rec, c->sms, c->stream)); break;
+        }
+        RF_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+        c->last_launches = 1;
+        c->timed = true;
+        return RF_OK;
+    }
     if (pl.chunk_draws > 0) {
         p.queue = queue;
         p.tab = c->d_cull.as<HitRec>();
@@ -953,6 +1020,33 @@ int batched_grid(rf_ctx *c, bool rec)
 
 bool mixed_culled(const rf_ctx *c, bool bv);
 
+// The narrow kernel on the scene held in the batch tables.
+rf_status run_mixed_narrow(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec, int32_t *d_rec,
+                           int64_t rec_base, bool zero_hits, int split)
+{
+    c->last_small = false;
+    c->last_launches = 0;
+    c->timed = false;
+    if (zero_hits) RF_CUDA(c, cudaMemsetAsync(c->b_hits.p, 0, (size_t)c->b_hits_total * 8, c->stream));
+    RF_CUDA(c, cudaMemsetAsync(c->b_counters.p, 0, sizeof(BatchCounters), c->stream));
+    if (seg.empty() || total_chunks == 0) return RF_OK;
+    if (rf_status st = upload_segments(c, seg); st != RF_OK) return st;
+    TraceParams p = batch_params(c);
+    p.n = c->b_info[0].n;
+    p.eps = c->b_info[0].eps;
+    p.seg = c->d_seg.as<Segment>();
+    p.nseg = (int32_t)seg.size();
+    p.total_chunks = total_chunks;
+    p.rec = d_rec;
+    p.rec_base = rec_base;
+    RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+    RF_CUDA(c, launch_mixed_narrow(p, split, rec, c->sms, c->stream));
+    RF_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+    c->last_launches = 1;
+    c->timed = true;
+    return RF_OK;
+}
+
 // One persistent launch over host-planned segments.
 rf_status run_batched(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec,
                       int32_t *d_rec, int64_t rec_base, bool zero_hits, bool bv, int64_t chunk_draws)
@@ -1023,9 +1117,15 @@ bool mixed_culled(const rf_ctx *c, bool bv)
     return c->b_single && !small_trace(c, bv) && (bv || (c->b_stacks > 0 && c->n <= kBatchTile));
 }
 
+int mixed_split(const rf_ctx *c, bool bv, int64_t draws)
+{
+    return c->b_single && c->mixed_path == 0 ? narrow_split(c, bv, draws) : 0;
+}
+
 // Draws per chunk of a MIXED trace of so many draws.
 int64_t mixed_chunk_draws(const rf_ctx *c, bool rec, bool bv, int64_t draws)
 {
+    if (const int split = mixed_split(c, bv, draws)) return 64 / split;
     return small_trace(c, bv) ? (int64_t)kSmallThreads * small_gpt(c, rec, bv) : chunk_for(draws, c->sms, 1024);
 }
 
@@ -1088,6 +1188,8 @@ rf_status run_small(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
 rf_status run_mixed(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec, int32_t *d_rec,
                     int64_t rec_base, bool zero_hits, bool bv, int64_t chunk_draws)
 {
+    if (chunk_draws <= 64)  // (no other kernel has chunks this short)
+        return run_mixed_narrow(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, 64 / (int)chunk_draws);
     if (small_trace(c, bv)) return run_small(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, bv);
     return run_batched(c, seg, total_chunks, rec, d_rec, rec_base, zero_hits, bv, chunk_draws);
 }

@@ -1,7 +1,8 @@
 // rf_culled_mixed.cu -- the culled kernel in mixed precision, for scenes with
-// bounding surfaces; default contraction like rf_kern_batched.cu, so that its
-// tests are the batched kernel's.
+// bounding surfaces or segment stacks, and the narrow kernel; default contraction
+// like rf_kern_batched.cu, so that their tests are the batched kernel's.
 #include "rf_culled.cuh"
+#include "rf_narrow.cuh"
 
 namespace rf {
 
@@ -16,6 +17,11 @@ cudaError_t launch_mixed_culled(const TraceParams &p, bool bv, bool rec, bool co
     if (rec) return launch_culled_k<MMixed, false, true, true>(p, blocks, st);
     return count ? launch_culled_k<MMixed, false, false, true, true>(p, blocks, st)
                  : launch_culled_k<MMixed, false, false, true>(p, blocks, st);
+}
+
+cudaError_t launch_mixed_narrow(const TraceParams &p, int split, bool rec, int sms, cudaStream_t st)
+{
+    return launch_narrow<MMixed>(p, split, rec, sms, st);
 }
 
 }  // namespace rf

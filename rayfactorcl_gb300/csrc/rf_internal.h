@@ -134,6 +134,12 @@ template <class M> cudaError_t launch_culled(const TraceParams &p, bool bv, bool
 // the box's sphere for spheres (RF_COMPAT_SPHERE's uncorrected discriminant).
 float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, double reach, bool loose_balls);
 
+// Few rays: one ray a thread, the surfaces split over `split` warps (rf_narrow.cuh;
+// chunks of 64 / split draws, scenes of at most kNarrowMax surfaces).
+constexpr int kNarrowMax = 1024, kNarrowThreads = 256, kNarrowBlocks = 4;
+template <class M> cudaError_t launch_narrow(const TraceParams &p, int split, bool rec, int sms, cudaStream_t st);
+cudaError_t launch_mixed_narrow(const TraceParams &p, int split, bool rec, int sms, cudaStream_t st);
+
 // The culled kernel's tables of one scene (rf_bounds.cu): sph (n), a ball around
 // the points a surface can return as hits (squared radius in w, infinite when there
 // is no bound, negative for a frustum, whose bound holds outside its band, 0 for a
