@@ -146,6 +146,22 @@ __device__ __forceinline__ bool reaches(const Ray<float> &r, float idd, const fl
     return fmaf(-bb * bb, idd, oc2) <= fabsf(b.w);
 }
 
+// The same for the ray's points up to the nearest hit so far, beyond which no hit
+// counts: the distance from the centre at the nearest parameter t of those, oc2 - 2 t
+// bb + t^2 cc, rounded by a few u reach^2 (the spheres allow for 64, rf_bounds.cu:
+// check_w).  For FP64, whose tests cost 70 times a gate: 1e6 rays 48 surfaces 1.37 ->
+// 1.33 ms, 400 surfaces 7.6 -> 5.6.  In FP32 the three more instructions a gate cost
+// more than the tests they save below 200 surfaces (EXACT 1e8 rays, 64: 5.83 -> 5.94
+// ms; 2e7 rays, 400: 5.53 -> 5.25).
+__device__ __forceinline__ bool reaches_before(const Ray<float> &r, float cc, float idd, const float4 b, double tb)
+{
+    const float ox = b.x - r.sx, oy = b.y - r.sy, oz = b.z - r.sz;
+    const float oc2 = dot3(ox, oy, oz, ox, oy, oz);
+    const float bb = dot3(ox, oy, oz, r.cx, r.cy, r.cz);
+    const float t = fminf(fmaxf(bb * idd, 0.0f), __double2float_ru(tb));
+    return fmaf(t, fmaf(t, cc, -bb) - bb, oc2) <= fabsf(b.w);
+}
+
 __device__ __forceinline__ Packet bounds_of(const Ray<float> &r, float idd)
 {
     Packet pk;
@@ -600,8 +616,12 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                 }
             };
             // can the lane's ray be hit by the surface at q (a packet's sphere candidate)
-            auto gate = [&](int q) {
-                return odd || reaches(rf, idd, RESIDENT ? s_bs[q] : __ldg(p.bsph + q));
+            auto gate = [&](int q, T tb) {
+                const float4 b = RESIDENT ? s_bs[q] : __ldg(p.bsph + q);
+                if constexpr (M::kF64)  // (RF_COMPAT_SPHERE's hits need not lie on the sphere)
+                    return odd || reaches_before(rf, cc, idd, b, sc ? M::inf() : tb);
+                else
+                    return odd || reaches(rf, idd, b);
             };
             auto test = [&](int j, T &tb, int &bi) {  // every lane, the same j
                 const HitRec h = RESIDENT ? s_tab[j] : load_rec(p.tab, j);
@@ -652,7 +672,7 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                         const bool two = cm != 0u;
                         if (COUNT && lane == 6) tcount += two ? 2 : 1;
                         cm &= cm - 1;  // 0 stays 0
-                        const bool ma = gate(qw + ba_), mb = gate(qw + bb_);
+                        const bool ma = gate(qw + ba_, tb), mb = gate(qw + bb_, tb);
                         unsigned go = (__any_sync(0xffffffffu, ma) || ((bm >> ba_) & 1u)) ? 1u : 0u;
                         if (two && (__any_sync(0xffffffffu, mb) || ((bm >> bb_) & 1u))) go |= 2u;
                         if constexpr (kMixed) {  // one copy of the tests: two spill (furnace 2.55 -> 2.60 ms)
