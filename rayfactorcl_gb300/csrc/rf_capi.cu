@@ -1164,7 +1164,7 @@ rf_status run_small(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
     p.rec = d_rec;
     p.rec_base = rec_base;
     const int gpt = small_gpt(c, rec, bv);
-    int bps = bv ? 4 : mixed_small_blocks_per_sm(gpt, rec);
+    int bps = bv ? 4 : mixed_small_blocks_per_sm(p.n, gpt, rec);
     if (bps <= 0) bps = 1;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sms * bps, total_chunks));
     RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));

@@ -166,7 +166,7 @@ cudaError_t launch_build_masks(const MaskInputs &in, uint32_t *out, cudaStream_t
 constexpr int kSmallMax = 64;       // surfaces of the largest scene it takes
 constexpr int kSmallThreads = 256;
 cudaError_t launch_mixed_small(const TraceParams &p, int gpt, bool rec, int grid, cudaStream_t st);
-int mixed_small_blocks_per_sm(int gpt, bool rec);
+int mixed_small_blocks_per_sm(int n, int gpt, bool rec);
 // The same with bounding surfaces (runBVGPU's walk), 4 rays per thread; 4 blocks fit an SM.
 cudaError_t launch_mixed_small_bv(const TraceParams &p, bool rec, int grid, cudaStream_t st);
 size_t batched_smem_bytes();
