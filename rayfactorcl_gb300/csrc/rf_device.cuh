@@ -447,14 +447,21 @@ __device__ __forceinline__ void rotate_uniforms(const float u[4], int v, float r
     for (int i = 0; i < 4; ++i) r[i] = u[(i + v + 1) & 3];
 }
 
-// Segment of global chunk c: the last segment whose chunk_begin <= c.
+// Segment of global chunk c: the last segment whose chunk_begin <= c.  Called by whole
+// warps with the same arguments: each step is 32 probes at once, so 1024 segments are
+// two dependent loads instead of ten (a chunk of the batched kernel spent 2500 to 3200
+// of 45000 clocks here at 1e5 rays).
 __device__ __forceinline__ int find_segment(const Segment *seg, int nseg, int64_t c)
 {
-    int lo = 0, hi = nseg - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (seg[mid].chunk_begin <= c) lo = mid;
-        else hi = mid - 1;
+    const int lane = threadIdx.x & 31;
+    int lo = 0, len = nseg;  // the answer lies in [lo, lo + len)
+    while (len > 1) {
+        const int step = (len + 31) >> 5;
+        const int i = lane * step;
+        const bool at = i == 0 || (i < len && seg[lo + i].chunk_begin <= c);
+        const int k = __popc(__ballot_sync(0xffffffffu, at)) - 1;  // chunk_begin never decreases
+        lo += k * step;
+        len = min(step, len - k * step);
     }
     return lo;
 }
