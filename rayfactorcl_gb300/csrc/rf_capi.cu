@@ -241,6 +241,20 @@ int64_t total_draws(const int64_t *count, int n)
     return d;
 }
 
+// The rays of a single-scene trace, by emitter.
+struct Budget {
+    const int64_t *count;
+    int n;
+    int64_t draws;
+    Budget(const int64_t *count_, int n_) : count(count_), n(n_), draws(total_draws(count_, n_)) {}
+    int64_t chunks(int64_t cg) const  // of cg draws (ranges that begin inside a chunk may have one more)
+    {
+        int64_t k = 0;
+        for (int e = 0; e < n; ++e) k += (((count[e] + 3) >> 2) + cg - 1) / cg;
+        return k;
+    }
+};
+
 rf_status check_budgets(rf_ctx *c, const int64_t *rays, int n)
 {
     for (int e = 0; e < n; ++e) {
@@ -326,14 +340,14 @@ bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
 //     longer in the batched kernel's shared memory) at 2e5 854 / 1339
 //   FP64  3 at 1e4 24 / 94; 12 at 4e4 144 / 251; 32 at 4e4 297 / 359; 64 at 2e4 300 / 318, at 4e4
 //     457 / 524; 100 at 1e4 246 / 214
-int narrow_split(const rf_ctx *c, bool bv, int64_t draws)
+int narrow_split(const rf_ctx *c, bool bv, const Budget &b)
 {
     const rf_config &f = c->cfg;
     const int n = c->n;
     if (bv || c->tuning || f.block_size || f.rays_per_thread || f.tally_mode || f.table_mode || f.test_order ||
         f.batched_grid || f.work_counts || n > kNarrowMax)
         return 0;
-    const int64_t rays = 4 * draws;
+    const int64_t rays = 4 * b.draws;
     int64_t most;
     switch (f.precision) {
     case RF_PREC_FP64: most = n <= 64 ? std::min<int64_t>(50000, 1200000 / n) : 0; break;
@@ -348,13 +362,13 @@ int narrow_split(const rf_ctx *c, bool bv, int64_t draws)
         return s;
     }
     // passes of the resident blocks x what a ray costs a warp: its part of the tests, and an
-    // emission of about 16 tests (64 surfaces, 1.5e5 rays, EXACT, split 1 2 4 8: 60 43 49 58 us;
-    // 400 surfaces, 1e4 rays: 145 90 49 35)
+    // emission of about 16 tests (64 surfaces, 1.5e5 rays, EXACT, split 1 2 4 8: 60 43 49 58
+    // us; 400 surfaces, 1e4 rays: 145 90 49 35)
     int best = 1;
     int64_t least = INT64_MAX;
     for (int s = 1; s <= 8; s *= 2) {
-        const int64_t chunks = rays * s / kNarrowThreads + n, blocks = kNarrowBlocks * (int64_t)c->sms;
-        const int64_t cost = (chunks + blocks - 1) / blocks * (n / s + 16);
+        const int64_t blocks = kNarrowBlocks * (int64_t)c->sms;
+        const int64_t cost = (b.chunks(64 / s) + blocks - 1) / blocks * (n / s + 16);
         if (cost < least) {
             least = cost;
             best = s;
@@ -389,11 +403,11 @@ int culled_chunk(const rf_ctx *c, int64_t draws)
 }
 
 // Launch shape for the single-scene kernels.
-Plan make_plan(const rf_ctx *c, bool bv, bool rec, int64_t draws)
+Plan make_plan(const rf_ctx *c, bool bv, bool rec, const Budget &b)
 {
     Plan pl;
-    pl.split = narrow_split(c, bv, draws);
-    if (pl.split == 0 && c->cull > 0 && culled_pays(c, bv, draws)) pl.chunk_draws = culled_chunk(c, draws);
+    pl.split = narrow_split(c, bv, b);
+    if (pl.split == 0 && c->cull > 0 && culled_pays(c, bv, b.draws)) pl.chunk_draws = culled_chunk(c, b.draws);
     pl.lc.bv = bv;
     pl.lc.rec = rec;
     pl.lc.block = c->block > 0 ? c->block : (c->cfg.block_size > 0 ? c->cfg.block_size : kBlock);
@@ -1117,16 +1131,16 @@ bool mixed_culled(const rf_ctx *c, bool bv)
     return c->b_single && !small_trace(c, bv) && (bv || (c->b_stacks > 0 && c->n <= kBatchTile));
 }
 
-int mixed_split(const rf_ctx *c, bool bv, int64_t draws)
+int mixed_split(const rf_ctx *c, bool bv, const Budget &b)
 {
-    return c->b_single && c->mixed_path == 0 ? narrow_split(c, bv, draws) : 0;
+    return c->b_single && c->mixed_path == 0 ? narrow_split(c, bv, b) : 0;
 }
 
 // Draws per chunk of a MIXED trace of so many draws.
-int64_t mixed_chunk_draws(const rf_ctx *c, bool rec, bool bv, int64_t draws)
+int64_t mixed_chunk_draws(const rf_ctx *c, bool rec, bool bv, const Budget &b)
 {
-    if (const int split = mixed_split(c, bv, draws)) return 64 / split;
-    return small_trace(c, bv) ? (int64_t)kSmallThreads * small_gpt(c, rec, bv) : chunk_for(draws, c->sms, 1024);
+    if (const int split = mixed_split(c, bv, b)) return 64 / split;
+    return small_trace(c, bv) ? (int64_t)kSmallThreads * small_gpt(c, rec, bv) : chunk_for(b.draws, c->sms, 1024);
 }
 
 // One launch of the small-scene kernel over host-planned segments (chunks of
@@ -1448,15 +1462,15 @@ rf_status rf_trace_async(rf_ctx *c, const int64_t *rays, int32_t use_bv)
         if (!c->b_single) return fail(c, RF_ERR_STATE, "scene not prepared for the mixed kernel");
         std::vector<Segment> seg;
         int64_t chunks = 0;
-        const int64_t cg = mixed_chunk_draws(c, false, use_bv != 0, total_draws(rays, c->n));
+        const int64_t cg = mixed_chunk_draws(c, false, use_bv != 0, Budget(rays, c->n));
         for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, 0, rays[e], cg, chunks);
         if ((s = run_mixed(c, seg, chunks, false, nullptr, 0, true, use_bv != 0, cg)) != RF_OK) return s;
         c->have_results = true;
         return RF_OK;
     }
-    const int64_t draws = total_draws(rays, c->n);
-    if (c->cull == 0 && culled_pays(c, use_bv != 0, draws) && (s = ensure_culled(c)) != RF_OK) return s;
-    Plan pl = make_plan(c, use_bv != 0, false, draws);
+    const Budget budget(rays, c->n);
+    if (c->cull == 0 && culled_pays(c, use_bv != 0, budget.draws) && (s = ensure_culled(c)) != RF_OK) return s;
+    Plan pl = make_plan(c, use_bv != 0, false, budget);
     std::vector<Segment> seg;
     int64_t chunks = 0;
     for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, 0, rays[e], pl.chunk_gids(), chunks);
@@ -1488,10 +1502,10 @@ rf_status rf_trace_range(rf_ctx *c, const int64_t *first_ray, const int64_t *cou
     std::vector<Segment> seg;
     int64_t chunks = 0;
     const bool mixed = c->cfg.precision == RF_PREC_MIXED;
-    const int64_t draws = total_draws(count, c->n);
-    if (c->cull == 0 && culled_pays(c, use_bv != 0, draws) && (s = ensure_culled(c)) != RF_OK) return s;
-    Plan pl = make_plan(c, use_bv != 0, false, draws);
-    const int64_t chunk_gids = mixed ? mixed_chunk_draws(c, false, use_bv != 0, draws) : pl.chunk_gids();
+    const Budget budget(count, c->n);
+    if (c->cull == 0 && culled_pays(c, use_bv != 0, budget.draws) && (s = ensure_culled(c)) != RF_OK) return s;
+    Plan pl = make_plan(c, use_bv != 0, false, budget);
+    const int64_t chunk_gids = mixed ? mixed_chunk_draws(c, false, use_bv != 0, budget) : pl.chunk_gids();
     for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, first_ray[e], count[e], chunk_gids, chunks);
     if (!accumulate) c->last_rays.assign(c->n, 0);
     for (int e = 0; e < c->n; ++e) c->last_rays[e] += count[e];
@@ -1615,14 +1629,14 @@ rf_status rf_trace_rays(rf_ctx *c, int32_t emitter, int64_t first_ray, int64_t n
     if (c->cfg.precision == RF_PREC_MIXED) {
         if (use_bv && (s = check_mixed_bv(c)) != RF_OK) return s;
         std::vector<Segment> seg;
-        const int64_t cg = mixed_chunk_draws(c, true, use_bv != 0, (n_rays + 3) / 4);
+        const int64_t cg = mixed_chunk_draws(c, true, use_bv != 0, Budget(&n_rays, 1));
         const int64_t chunks = plan_segments(seg, emitter, 0, first_ray, n_rays, cg, 0);
         if ((s = run_mixed(c, seg, chunks, true, c->d_rec.as<int32_t>(), first_ray, false, use_bv != 0, cg)) != RF_OK)
             return s;
     } else {
-        const int64_t draws = (n_rays + 3) / 4;
-        if (c->cull == 0 && culled_pays(c, use_bv != 0, draws) && (s = ensure_culled(c)) != RF_OK) return s;
-        Plan pl = make_plan(c, use_bv != 0, true, draws);
+        const Budget budget(&n_rays, 1);
+        if (c->cull == 0 && culled_pays(c, use_bv != 0, budget.draws) && (s = ensure_culled(c)) != RF_OK) return s;
+        Plan pl = make_plan(c, use_bv != 0, true, budget);
         std::vector<Segment> seg;
         const int64_t chunks = plan_segments(seg, emitter, 0, first_ray, n_rays, pl.chunk_gids(), 0);
         if ((s = run_trace(c, seg, chunks, pl, c->d_rec.as<int32_t>(), first_ray, false)) != RF_OK) return s;
