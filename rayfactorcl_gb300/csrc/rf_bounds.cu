@@ -213,6 +213,40 @@ float check_w(const Ball &b, double size, double reach)
     return w < 1e30 ? (float)(w * (1 + 1e-6)) : INFINITY;
 }
 
+// What the FP64 kernel's FP32 look at a surface (rf_culled.cuh: cone_may, plane_may,
+// ring_hits) must allow for, given the surface's true extent x; w = 0: no look.  The
+// FP64 test's own rounding is nothing here; the FP32 ray in object space is off by at
+// most 8 u of the terms S_k it is summed from, at every point up to the hit.
+// * Planar: x, y = 32 u S of the hit's place and of its height.
+// * Quadrics: a true root t leaves |Q(t)| <= x = 128 u S^2 (cones 256) in the FP32
+//   coordinates (2 S times their error, and the rounding of A and B); y: z's slack; z:
+//   of a cylinder 64 u S, which over sqrt(A) is the rounding of its roots, of a cone S.
+float4 look_slack(const float *im, int type, float util1, const Extent &x, const Ball &b, const Ball &from, double smax)
+{
+    constexpr double u = 1.0 / (1 << 24);
+    double off[3], S[3];
+    for (int k = 0; k < 3; ++k) off[k] = b.c[k] - from.c[k];
+    const double reach = 1.25 * (std::sqrt(dot(off, off)) + from.r + b.r);
+    for (int k = 0; k < 3; ++k) {
+        const double l[3] = {im[4 * k], im[4 * k + 1], im[4 * k + 2]};
+        S[k] = std::sqrt(dot(l, l)) * (smax + reach) + std::fabs((double)im[4 * k + 3]) + std::max(1.0, std::max(x.r0, x.r1));
+    }
+    const double Sxy = std::max(S[0], S[1]), sz = 128 * u * S[2] + 1e-6;
+    double S2 = S[0] * S[0] + S[1] * S[1] + 1.0;
+    float4 sl = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (type == RF_CYLINDER) {
+        sl = make_float4((float)(128 * u * S2), (float)sz, (float)(64 * u * Sxy), 1.f);
+    } else if (type == RF_FRUSTUM) {
+        const double fS = std::fabs((double)util1 - 1.0) * S[2] + 1.0;
+        S2 += fS * fS;
+        sl = make_float4((float)(256 * u * S2), (float)sz, (float)std::sqrt(S2), 1.f);
+    } else if (type != RF_SPHERE) {  // (a sphere's ball is all there is to look at)
+        sl = make_float4((float)(32 * u * Sxy), (float)(32 * u * S[2]), 0.f, 1.f);
+    }
+    if (!(sl.x < 0.25f) || !(sl.y < 0.25f)) sl.w = 0.f;
+    return sl;
+}
+
 // Rings [i, i + m) that one cylinder search finds (ring_hits): cylinders that tile
 // a longer one.  Returns m (1: none); x becomes the stack's extent in the first
 // ring's frame, sl its slack.  Ring k's object coordinates along a ray, with z
@@ -363,6 +397,9 @@ bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs
         const Ball b = hit_ball(p.invm, p.type, p.util1, x, from, smax, quad + 2 * i);
         const float4 s = ball_out(b, p.type == RF_FRUSTUM);
         if (std::isfinite(s.w)) bounded += m;
+        double M[9], t[3];
+        if (m == 1 && std::isfinite(s.w) && inverse_of(p.invm, M, t))
+            sl = look_slack(p.invm, p.type, p.util1, x, image_ball(M, t, x), from, smax);
         for (int k = 0; k < m; ++k) {
             sph[i + k] = s;
             slack[i + k] = sl;

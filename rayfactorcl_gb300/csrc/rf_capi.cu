@@ -310,7 +310,8 @@ struct Plan {
 //     0.099 / 0.140 -> from 4e5 rays (FAST 1e6) or 128 surfaces (FAST 256) on, in FP64
 //     always (64 surfaces, 1e5 rays: 0.58 / 1.01);
 //   a few hundred rays per emitter leave most threads of a plain chunk idle: 1e4 rays,
-//     64 surfaces EXACT 0.033 / 0.056, FAST 0.029 / 0.032.
+//     64 surfaces EXACT 0.033 / 0.056, FAST 0.029 / 0.032 (bounding surfaces only: other
+//     traces of so few rays take the narrow kernel).
 // The tables are made for the first trace that takes this kernel (about 40 us at 64
 // surfaces), not in rf_set_scene, where a scene traced otherwise would pay for them.
 bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)

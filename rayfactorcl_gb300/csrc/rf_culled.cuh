@@ -9,17 +9,17 @@
 // out only when its test, rounding included, could not return a hit, so every
 // ray gets the plain kernel's nearest hit bit for bit, whatever packet it is in:
 //
-// * rf_capi.cu (cull_tables) bounds the points where a test can place a hit: the
-//   object-space shape grown by the test's rounding (for quadrics the
-//   cancellation in B^2 - AC, about 32 ulps of the largest squared object-space
-//   coordinate of the scene), as a world sphere grown again by this file's own
+// * rf_bounds.cu (cull_tables) bounds the points where a test can place a hit: the
+//   object-space shape grown by the test's rounding (for quadrics |Q| <= 128 u S^2 at
+//   the hit, from the cancellation in B^2 - AC, S the longest object-space
+//   coordinate of a ray up to it), as a world sphere grown again by this file's own
 //   FP32 rounding.  The bound of a cone fails for rays whose direction makes its
 //   A = c^T N c vanish; `band` lets those through (a frustum's sphere carries the
 //   sign bit in its radius as the mark).
 // * A ray with a non-finite or vanishing component is tested against everything,
 //   with the rest of its packet.
-// * Consecutive cylinders with one linear part that tile a longer cylinder (a
-//   furnace wall of rings) are first intersected as one, in FP32: the roots, with
+// * Consecutive cylinders with nearly the same linear part (to 1e-5) that tile a
+//   longer cylinder (a furnace wall of rings) are first intersected as one, in FP32: the roots, with
 //   error bounds, name the one or two rings that a ring's own test could accept,
 //   and only those are tested, each lane its own.  Concentric annuli in one plane
 //   whose radii meet share one plane hit, exactly: the same operations give the
@@ -30,8 +30,8 @@
 // (plain 18.2), of which draws, keys and sort 0.6, emission and packet bounds 1.3,
 // the spheres 2.2 (9 candidates per packet) and the tests 1.7 (5.3 per packet, of
 // which 2.4 find a hit for some ray; the plain kernel makes 64 per ray).  The
-// furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.10 ms EXACT
-// (plain 7.9), 0.84 FAST (5.7); 1e6 rays in FP64 2.3 (35.4).  In mixed precision, 5e7
+// furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.07 ms EXACT
+// (plain 7.9), 0.85 FAST (5.7); 1e6 rays in FP64 2.4 (35.4).  In mixed precision, 5e7
 // rays: 2.55 ms with bounding surfaces (3.36 as a variant of the batched kernel, which
 // spilled 600 bytes a thread), 1.99 without (2.30); the reference's furnace model,
 // 2e7 rays, 0.96 (1.65).
@@ -291,6 +291,56 @@ __device__ __forceinline__ void ring_hits(const HitRec *tab, bool resident, int 
             ++k1;
         }
     }
+}
+
+// FP32 looks at a surface whose FP64 test costs fifty times as much (16 clocks of an SM
+// an instruction): false only when no point of the ray with eps < t < tb, as the FP64
+// test finds them, can be a hit.  sl: rf_bounds.cu, look_slack; NaN anywhere keeps the
+// test.  1e6 rays: 48 surfaces 1.33 -> 1.27 ms, 201 (5e5 rays) 2.10 -> 1.85, 400 5.65 ->
+// 4.78; what is left is emission (20 surfaces 0.91).
+__device__ __forceinline__ bool root_may(const Ray<float> &o, float t0, float t1, float te, float zslack, float eps,
+                                         float tb)
+{
+    const float lo = fminf(t0, t1), hi = fmaxf(t0, t1);
+    const float s = fmaf(8e-6f, fabsf(lo) + fabsf(hi), te), zs = fmaf(fabsf(o.cz), s, zslack);
+    const float z0 = fmaf(o.cz, lo, o.sz), z1 = fmaf(o.cz, hi, o.sz);
+    return !(hi + s < eps || lo - s > tb || fmaxf(z0, z1) + zs < 0.0f || fminf(z0, z1) - zs > 1.0f);
+}
+
+// A frustum, for rays out of its band (A then keeps 1e-3 of its terms or more).  D
+// by Lagrange's identity is off by 32 u S^2 a, a the squared length of c over the
+// quadric's coordinates; B by 8 u S sqrt(a).
+__device__ __forceinline__ bool cone_may(const HitRec &h, const float4 sl, const Ray<float> &w, float eps, float tb)
+{
+    const Ray<float> o = xfrm_ray<MFast>(h, w);
+    const float f = h.aux.y - 1.0f, fd = f * o.cz, fs = fmaf(f, o.sz, 1.0f);
+    const float a2 = fmaf(o.cx, o.cx, o.cy * o.cy), A = fmaf(-fd, fd, a2), a = fmaf(fd, fd, a2);
+    const float B = -fmaf(o.sx, o.cx, fmaf(o.sy, o.cy, -fs * fd));
+    const float u = fmaf(o.cx, fs, -o.sx * fd), v = fmaf(o.cy, fs, -o.sy * fd), wz = fmaf(o.sx, o.cy, -o.sy * o.cx);
+    const float D = fmaf(u, u, fmaf(v, v, -wz * wz));
+    const float dk = fmaf(fabsf(A), sl.x, 0x1p-19f * sl.z * sl.z * a);
+    if (D + dk < 0.0f) return false;
+    const float ra = MFast::rcp(A), te = 0x1p-19f * sl.z * MFast::sqrt(a) * fabsf(ra);
+    if (!(te < 1e30f)) return true;
+    const float hi = MFast::sqrt(D + dk), lo = MFast::sqrt(fmaxf(D - dk, 0.0f));
+    return root_may(o, (B - hi) * ra, (B - lo) * ra, te, sl.y, eps, tb) ||
+           root_may(o, (B + lo) * ra, (B + hi) * ra, te, sl.y, eps, tb);
+}
+
+__device__ __forceinline__ bool plane_may(const HitRec &h, int type, const float4 sl, const Ray<float> &w, float eps,
+                                          float tb)
+{
+    const Ray<float> o = xfrm_ray<MFast>(h, w);
+    const float rz = MFast::rcp(o.cz), th = -o.sz * rz;
+    const float dt = fmaf(sl.y, fabsf(rz), 1e-6f * fabsf(th));
+    if (!(dt < 1e30f)) return true;
+    const float hx = fmaf(o.cx, th, o.sx), hy = fmaf(o.cy, th, o.sy);
+    const float m = 2.0f * fmaf(fabsf(o.cx) + fabsf(o.cy), dt, sl.x);
+    if (th + dt < eps || th - dt > tb) return false;
+    if (type == RF_RECTANGLE) return !(fabsf(hx) > 1.0f + m || fabsf(hy) > 1.0f + m);
+    const float e = MFast::sqrt(fmaf(hx, hx, hy * hy));
+    if (type == RF_DISC) return !(e > 1.00001f + m);
+    return !(e > fmaf(MFast::sqrt(h.aux.z), 1.00001f, m) || e < fmaf(MFast::sqrt(h.aux.y), 0.99999f, -m));
 }
 
 // Nearest hit among the annuli [a, a + m) of a plate: one plane, one radius.
@@ -650,6 +700,20 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                     else
                         ring_hits<M>(tab, RESIDENT, j, (int)m, __ldg(p.cstack + j), ray, rf, eps, odd, tb, bi);
                 } else {
+                    if constexpr (M::kF64) {  // FP32 first: half the tests find a hit for no ray
+                        const float4 sl = __ldg(p.cstack + j);
+                        if (type == RF_CYLINDER && sl.w != 0.0f) {
+                            ring_hits<M>(tab, RESIDENT, j, 1, sl, ray, rf, eps, odd, tb, bi);
+                            return;
+                        }
+                        bool may = odd || sl.w == 0.0f;
+                        if (!may) {
+                            const float feps = __double2float_rd(eps), ftb = __double2float_ru(tb);
+                            may = type == RF_FRUSTUM ? band(p.cquad, j, rf, cc) || cone_may(h, sl, rf, feps, ftb)
+                                                     : plane_may(h, type, sl, rf, feps, ftb);
+                        }
+                        if (!__any_sync(0xffffffffu, may)) return;
+                    }
                     const T t = hit_any<M>(type, h, ray, eps, sc, M::inf());
                     if (t < tb) {
                         tb = t;
