@@ -511,6 +511,8 @@ def run_ours(args):
             traffic = None
 
     kname = {"mixed": ("small-scene mixed-precision kernel (rf::mixed_small_kernel)" if mixed_small else
+                       "mixed-precision packets, candidates by bounding spheres (rf::culled_kernel)"
+                       if args.workload in ("furnace", "ref-furnace") else  # bounding surfaces, segment stacks
                        "batched mixed-precision persistent kernel (rf::batched_kernel)"),
              "exact": "plain bit-exact kernel (rf::trace_kernel<MExact>)",
              "fast": "plain FP32-approximation kernel (rf::trace_kernel<MFast>)"}[args.precision]

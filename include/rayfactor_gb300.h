@@ -96,6 +96,9 @@ typedef struct rf_config {
                            * < 0 relative, |eps| x the diagonal of the scene's bounding box
                            * (per scene in a batch)                                          */
     int32_t device;       /* CUDA device ordinal                                            */
+    /* The five launch-shape fields below pin the plain kernel (RF_PREC_MIXED: the small-scene
+     * or batched kernel) when one of them is not 0; otherwise a trace takes the kernel that is
+     * fastest for its surfaces and rays.  Results do not depend on it.                      */
     int32_t block_size;   /* 0: autotuned / built-in default                                */
     int32_t rays_per_thread; /* 0: default; 4 or 8 (one or two Philox draws)                */
     uint32_t scene_id;    /* folded into the stream counter outside RF_COMPAT_STREAMS       */
@@ -103,8 +106,9 @@ typedef struct rf_config {
     int32_t table_mode;   /* 0: autotuned / default; 1: surfaces staged in shared memory; 2: read through L1 */
     int32_t test_order;   /* 0: autotuned / default; 1: a thread's 4 or 8 rays tested together against
                            * each surface; 2: one ray at a time against all surfaces (smaller code) */
-    int32_t work_counts;  /* RF_PREC_MIXED: 1 = the batched kernel also counts its tests for
-                           * rf_last_work_counts (a few per cent slower); 0 = no counting      */
+    int32_t work_counts;  /* RF_PREC_MIXED: 1 = also count the tests for
+                           * rf_last_work_counts (a few per cent slower; traces of few rays
+                           * then take the kernels of larger ones); 0 = no counting           */
     int32_t batched_grid; /* RF_PREC_MIXED: 0 = one persistent block per SM; > 0 = at most this
                            * many blocks (results do not depend on it)                         */
     int32_t split_stacks; /* RF_PREC_MIXED: 0 = a segment stack is one test -- consecutive cylinders
@@ -281,7 +285,7 @@ rf_status rf_smooth_F(rf_ctx *ctx, const double *F, const double *areas, int32_t
  * is not NULL, appended to that file and read back by later processes.  Applies
  * the choice to the context.  RF_PREC_MIXED: for one scene of at most 64 surfaces, the choice
  * between the batched kernel and the small-scene kernel with 4 or 8 rays per thread (cached
- * the same way); with use_bv, a check that the scene fits the bounding-surface variant.
+ * the same way); with use_bv, a check that the scene fits the bounding-surface kernels.
  * Results of a trace do not depend on the launch shape. */
 rf_status rf_autotune(rf_ctx *ctx, int32_t use_bv, const char *cache_path);
 
