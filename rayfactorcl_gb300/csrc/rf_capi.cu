@@ -107,8 +107,8 @@ struct rf_ctx {
     DevBuf d_tab, d_emit, d_bvtab, d_bvinfo;
     std::vector<rf_bounding_volume> bvs;
     int cull = 0;   // the culled kernel's tables: 0 not made yet, 1 in d_cull, -1 of no use for this scene
-    DevBuf d_cull;  // hit records (n), then float4: spheres (n), cone words (2 n), ring slack (n), bounding
-                    // surfaces' spheres (nbv)
+    DevBuf d_cull;  // hit records (n), then float4: spheres (n), cone words (2 n), slack (n), bounding
+                    // surfaces' spheres (nbv), and in FP64 each one's invm in doubles (6 (n + nbv))
     bool tuning = false;  // rf_autotune is timing the plain kernel's launch shapes
 
     // trace state
@@ -380,11 +380,17 @@ int narrow_split(const rf_ctx *c, bool bv, const Budget &b)
 
 rf_status ensure_culled(rf_ctx *c)
 {
-    const size_t n = c->n, words = 8 * n + c->nbv;  // float4
+    const bool f64 = c->cfg.precision == RF_PREC_FP64;
+    const size_t n = c->n, at64 = 8 * n + c->nbv, words = at64 + (f64 ? 6 * (n + c->nbv) : 0);  // float4
     std::vector<float4> buf(words);
     HitRec *tab = reinterpret_cast<HitRec *>(buf.data());
     for (size_t i = 0; i < n; ++i)
         tab[i] = make_hitrec(c->prims[i].invm, c->prims[i].type, c->prims[i].util1, c->prims[i].util2);
+    if (f64) {
+        double *d = reinterpret_cast<double *>(buf.data() + at64);
+        for (size_t i = 0; i < n; ++i) std::copy(c->prims[i].invm, c->prims[i].invm + 12, d + 12 * i);
+        for (int i = 0; i < c->nbv; ++i) std::copy(c->bvs[i].invm, c->bvs[i].invm + 12, d + 12 * (n + i));
+    }
     float4 *q = buf.data() + 4 * n;
     const bool ok = cull_tables(c->prims.data(), c->n, c->bvs.data(), c->nbv, c->cfg.split_stacks == 0, tab, q, q + n,
                                 q + 3 * n, q + 4 * n);
@@ -527,6 +533,7 @@ rf_status run_trace(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
         p.cquad = p.bsph + n;
         p.cstack = p.bsph + 3 * (size_t)n;
         p.bvsph = p.bsph + 4 * (size_t)n;
+        p.tab64 = reinterpret_cast<const double *>(p.bvsph + c->nbv);
         p.chunk_draws = pl.chunk_draws;
         p.use_smem_hist = n <= kBatchTile ? 1 : 0;
         RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));

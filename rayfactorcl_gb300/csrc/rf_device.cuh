@@ -143,12 +143,24 @@ struct MF64 {
 template <class T> struct Ray { T sx, sy, sz, cx, cy, cz; };
 template <class T> struct V3 { T x, y, z; };
 
+// A surface's and an emitter's records for FP64, their matrices converted once: a
+// conversion costs as much as an FP64 operation, and a ray and a test had 21 and 12.
+struct HitRec64 {
+    struct Row { double x, y, z, w; } r0, r1, r2;
+    float4 aux;
+};
+struct Emit64 {
+    double m[12], invm[12];
+    float util1, util2;
+    int type;
+};
+
 // ---------------------------------------------------------------------------
 // Intersection tests (RayFactorGPU.cl:99-291).  `h` is the surface's invm in
 // rows r0..r2 and (type, util1, util2) in aux.
 // ---------------------------------------------------------------------------
-template <class M>
-__device__ __forceinline__ Ray<typename M::T> xfrm_ray(const HitRec &h, const Ray<typename M::T> &w)
+template <class M, class H = HitRec>
+__device__ __forceinline__ Ray<typename M::T> xfrm_ray(const H &h, const Ray<typename M::T> &w)
 {
     using T = typename M::T;
     Ray<T> o;  // RayFactorGPU.cl:99-109
@@ -161,8 +173,8 @@ __device__ __forceinline__ Ray<typename M::T> xfrm_ray(const HitRec &h, const Ra
     return o;
 }
 
-template <class M>
-__device__ __forceinline__ typename M::T rectangle_hit(const HitRec &h, const Ray<typename M::T> &w,
+template <class M, class H = HitRec>
+__device__ __forceinline__ typename M::T rectangle_hit(const H &h, const Ray<typename M::T> &w,
                                                        typename M::T eps)
 {
     using T = typename M::T;  // RayFactorGPU.cl:126-145
@@ -174,8 +186,8 @@ __device__ __forceinline__ typename M::T rectangle_hit(const HitRec &h, const Ra
     return th;
 }
 
-template <class M>
-__device__ __forceinline__ typename M::T disc_hit(const HitRec &h, const Ray<typename M::T> &w,
+template <class M, class H = HitRec>
+__device__ __forceinline__ typename M::T disc_hit(const H &h, const Ray<typename M::T> &w,
                                                   typename M::T eps)
 {
     using T = typename M::T;  // RayFactorGPU.cl:147-166
@@ -188,8 +200,8 @@ __device__ __forceinline__ typename M::T disc_hit(const HitRec &h, const Ray<typ
     return M::inf();
 }
 
-template <class M>
-__device__ __forceinline__ typename M::T annulus_hit(const HitRec &h, const Ray<typename M::T> &w,
+template <class M, class H = HitRec>
+__device__ __forceinline__ typename M::T annulus_hit(const H &h, const Ray<typename M::T> &w,
                                                      typename M::T eps)
 {
     using T = typename M::T;  // RayFactorGPU.cl:168-187 (util1/util2: squared radii)
@@ -214,8 +226,8 @@ __device__ __forceinline__ typename M::T quadric_pick(const Ray<typename M::T> &
     return t1;
 }
 
-template <class M>
-__device__ __forceinline__ typename M::T cylinder_hit(const HitRec &h, const Ray<typename M::T> &w,
+template <class M, class H = HitRec>
+__device__ __forceinline__ typename M::T cylinder_hit(const H &h, const Ray<typename M::T> &w,
                                                       typename M::T eps)
 {
     using T = typename M::T;  // RayFactorGPU.cl:189-222
@@ -228,8 +240,8 @@ __device__ __forceinline__ typename M::T cylinder_hit(const HitRec &h, const Ray
     return quadric_pick<M>(o, ra * (B - disc), ra * (B + disc), eps);
 }
 
-template <class M>
-__device__ __forceinline__ typename M::T frustum_hit(const HitRec &h, const Ray<typename M::T> &w,
+template <class M, class H = HitRec>
+__device__ __forceinline__ typename M::T frustum_hit(const H &h, const Ray<typename M::T> &w,
                                                      typename M::T eps)
 {
     using T = typename M::T;  // RayFactorGPU.cl:224-260
@@ -245,8 +257,8 @@ __device__ __forceinline__ typename M::T frustum_hit(const HitRec &h, const Ray<
     return quadric_pick<M>(o, ra * (B - disc), ra * (B + disc), eps);
 }
 
-template <class M>
-__device__ __forceinline__ typename M::T sphere_hit(const HitRec &h, const Ray<typename M::T> &w,
+template <class M, class H = HitRec>
+__device__ __forceinline__ typename M::T sphere_hit(const H &h, const Ray<typename M::T> &w,
                                                     typename M::T eps, bool compat)
 {
     using T = typename M::T;  // RayFactorGPU.cl:262-291
@@ -277,8 +289,8 @@ __device__ __forceinline__ typename M::T sphere_hit(const HitRec &h, const Ray<t
 }
 
 // switch of RayFactorGPU.cl:452-460; an unknown type keeps the previous t.
-template <class M>
-__device__ __forceinline__ typename M::T hit_any(int type, const HitRec &h, const Ray<typename M::T> &w,
+template <class M, class H = HitRec>
+__device__ __forceinline__ typename M::T hit_any(int type, const H &h, const Ray<typename M::T> &w,
                                                  typename M::T eps, bool sphere_compat,
                                                  typename M::T stale)
 {
@@ -296,8 +308,8 @@ __device__ __forceinline__ typename M::T hit_any(int type, const HitRec &h, cons
 // ---------------------------------------------------------------------------
 // Emission (RayFactorGPU.cl:64-121, 298-443).
 // ---------------------------------------------------------------------------
-template <class M>
-__device__ __forceinline__ V3<typename M::T> transform_point(const float *m, V3<typename M::T> p)
+template <class M, class S>
+__device__ __forceinline__ V3<typename M::T> transform_point(const S *m, V3<typename M::T> p)
 {
     using T = typename M::T;  // RayFactorGPU.cl:64-71, dot() as an fma chain
     V3<T> w;
@@ -307,8 +319,8 @@ __device__ __forceinline__ V3<typename M::T> transform_point(const float *m, V3<
     return w;
 }
 
-template <class M>
-__device__ __forceinline__ V3<typename M::T> transform_normal(const float *im, V3<typename M::T> n)
+template <class M, class S>
+__device__ __forceinline__ V3<typename M::T> transform_normal(const S *im, V3<typename M::T> n)
 {
     using T = typename M::T;  // RayFactorGPU.cl:73-85
     V3<T> w;
@@ -357,8 +369,8 @@ __device__ __forceinline__ V3<typename M::T> os_ray_direction(const float r[4])
 }
 
 // One ray from emitter record e with the rotated uniforms r = (x, y, z, w).
-template <class M>
-__device__ __forceinline__ Ray<typename M::T> emit_ray(const rf_primitive &e, const float r[4])
+template <class M, class E = rf_primitive>
+__device__ __forceinline__ Ray<typename M::T> emit_ray(const E &e, const float r[4])
 {
     using T = typename M::T;
     V3<T> p, n, o, s, c;

@@ -70,7 +70,8 @@ struct TraceParams {
     const int64_t *mask_off;        // per global row (prim_off + emitter): first mask word, -1 = none
     const float4 *bvsph;            // mixed kernels: bounding sphere of each bounding surface (as bsph)
     const float4 *cquad;            // culled kernel: two words per surface, a frustum's A and its threshold
-    const float4 *cstack;           // culled kernel: per surface, slack of its ring stack
+    const float4 *cstack;           // culled kernel: per surface, slack of its ring stack or FP32 look
+    const double *tab64;            // culled kernel in FP64: invm of each surface, then bounding surface, 12 doubles
     int32_t chunk_draws;            // batched and culled kernels: draws of a chunk
     const int32_t *d_chunk;         // batched kernel: the same, device-resident (or null)
 };

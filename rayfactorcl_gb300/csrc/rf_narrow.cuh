@@ -30,7 +30,9 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
     constexpr int kRays = kNarrowThreads / SPLIT;  // rays of a chunk
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HitRec *s_tab = reinterpret_cast<HitRec *>(smem_raw);
+    double *s_tab64 = reinterpret_cast<double *>(s_tab + p.n);  // FP64: invm, 12 doubles a surface
     __shared__ rf_primitive s_emit;
+    __shared__ Emit64 s_emit64;  // FP64
     __shared__ float4 s_frame[kMixed ? kFrameWords : 1];
     __shared__ T s_t[SPLIT > 1 ? kNarrowThreads : 1];
     __shared__ int s_i[SPLIT > 1 ? kNarrowThreads : 1];
@@ -42,6 +44,9 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
     const T eps = T(p.eps);
     for (int i = tid; i < 4 * n; i += kNarrowThreads)
         reinterpret_cast<float4 *>(s_tab)[i] = __ldg(reinterpret_cast<const float4 *>(p.tab) + i);
+    if (M::kF64)
+        for (int i = tid; i < 12 * n; i += kNarrowThreads)
+            s_tab64[i] = __ldg(reinterpret_cast<const float *>(p.tab + i / 12) + i % 12);
     if (tid <= SPLIT) s_lo[tid] = n * tid / SPLIT;
     __syncthreads();
     if (kMixed && SPLIT > 1)  // no part begins inside a segment stack, which is one test
@@ -69,6 +74,7 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
             __syncthreads();
             if (tid < (int)(sizeof(rf_primitive) / 4))
                 reinterpret_cast<float *>(&s_emit)[tid] = reinterpret_cast<const float *>(p.emit + sg.emitter)[tid];
+            if (M::kF64) fill_emit64(s_emit64, p.emit[sg.emitter], tid);
             if (kMixed && tid < kFrameWords) s_frame[tid] = p.frame[(int64_t)sg.emitter * kFrameWords + tid];
             __syncthreads();
         }
@@ -85,6 +91,8 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
         Ray<T> ray;
         if constexpr (kMixed)
             ray = emit_mixed(s_emit, s_frame, r);
+        else if constexpr (M::kF64)
+            ray = emit_ray<M>(s_emit64, r);
         else
             ray = emit_ray<M>(s_emit, r);
         const int skip = kMixed && planar(s_emit.type) ? sg.emitter : -1;
@@ -111,7 +119,13 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
                 }
                 if (is_stack(type)) j = stack_end(h, j) - 1;
             } else {
-                const T t = hit_any<M>(type, h, ray, eps, sc, M::inf());
+                T t;
+                if constexpr (M::kF64) {
+                    const HitRec64::Row *q = reinterpret_cast<const HitRec64::Row *>(s_tab64 + 12 * j);
+                    t = hit_any<M>(type, HitRec64{q[0], q[1], q[2], h.aux}, ray, eps, sc, M::inf());
+                } else {
+                    t = hit_any<M>(type, h, ray, eps, sc, M::inf());
+                }
                 if (t < tb) {
                     tb = t;
                     bi = j;
@@ -151,7 +165,7 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
 template <class M, int SPLIT>
 static cudaError_t launch_narrow_s(const TraceParams &p, bool rec, int sms, cudaStream_t st)
 {
-    const size_t smem = (size_t)p.n * sizeof(HitRec);
+    const size_t smem = (size_t)p.n * (sizeof(HitRec) + (M::kF64 ? 12 * sizeof(double) : 0));
     const void *k = rec ? (const void *)narrow_kernel<M, SPLIT, true> : (const void *)narrow_kernel<M, SPLIT, false>;
     if (smem > 40 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
