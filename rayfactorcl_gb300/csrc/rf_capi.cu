@@ -303,12 +303,13 @@ struct Plan {
 // autotuner is timing those.  Culled against plain, measured on scenes of the
 // benchmark's type mix, ms:
 //   surfaces: at 1e7 rays (FP64: 1e6)  EXACT 16: 0.41 / 0.60, 64: 0.71 / 1.88, 400: 3.2 / 9.9;
-//     FAST 16: 0.34 / 0.33, 24: 0.38 / 0.47, 64: 0.62 / 1.11; FP64 16: 0.89 / 2.10
-//     -> from 16 surfaces on, FAST from 24;
+//     FAST 16: 0.34 / 0.33, 24: 0.38 / 0.47, 64: 0.62 / 1.11 -> from 16 surfaces on, FAST
+//     from 24; FP64 3: 0.61 / 0.71, 8: 0.63 / 1.28, 15: 0.65 / 2.01, at 1e5 rays 3: 0.160 / 0.094,
+//     5: 0.166 / 0.150, 8: 0.175 / 0.188 -> from 8, or from 3 at 2.5e5 rays;
 //   rays: the sort's fixed cost, EXACT at 1e5 rays  64 surfaces: 0.065 / 0.056, 201: 0.15 / 0.19;
 //     at 3e5 rays 24: 0.044 / 0.040, 64: 0.071 / 0.085, FAST 64: 0.060 / 0.060, at 1e6 rays
-//     0.099 / 0.140 -> from 4e5 rays (FAST 1e6) or 128 surfaces (FAST 256) on, in FP64
-//     always (64 surfaces, 1e5 rays: 0.58 / 1.01);
+//     0.099 / 0.140 -> from 4e5 rays (FAST 1e6) or 128 surfaces (FAST 256) on (FP64 64
+//     surfaces, 1e5 rays: 0.58 / 1.01);
 //   a few hundred rays per emitter leave most threads of a plain chunk idle: 1e4 rays,
 //     64 surfaces EXACT 0.033 / 0.056, FAST 0.029 / 0.032 (bounding surfaces only: other
 //     traces of so few rays take the narrow kernel).
@@ -323,7 +324,7 @@ bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
     if (bv && (c->n > kBatchTile || c->nbv > kBatchMaxBV)) return false;
     const int n = c->n;
     const int64_t rays = 4 * draws;
-    if (f.precision == RF_PREC_FP64) return n >= 16;
+    if (f.precision == RF_PREC_FP64) return n >= 8 || (n >= 3 && rays >= 250000);
     if (f.precision == RF_PREC_FAST) return n >= 256 || (n >= 24 && rays >= 1000000) || (n >= 64 && rays <= 200 * n);
     return n >= 128 || (n >= 16 && rays >= 400000) || (n >= 24 && rays <= 400 * n);
 }

@@ -31,7 +31,7 @@
 // the spheres 2.2 (9 candidates per packet) and the tests 1.7 (5.3 per packet, of
 // which 2.4 find a hit for some ray; the plain kernel makes 64 per ray).  The
 // furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.07 ms EXACT
-// (plain 7.9), 0.85 FAST (5.7); 1e6 rays in FP64 2.4 (35.4).  In mixed precision, 5e7
+// (plain 7.9), 0.85 FAST (5.7); 1e6 rays in FP64 2.0 (35.4).  In mixed precision, 5e7
 // rays: 2.55 ms with bounding surfaces (3.36 as a variant of the batched kernel, which
 // spilled 600 bytes a thread), 1.99 without (2.30); the reference's furnace model,
 // 2e7 rays, 0.96 (1.65).
