@@ -162,6 +162,22 @@ __device__ __forceinline__ void unpack_uniforms(uint32_t w0, uint32_t w1, uint32
     uf[3] = __fmul_rn(__uint2float_rn(d), 0x1p-24f);
 }
 
+// The uniforms of sub-ray v (rotate_uniforms) of a packed draw, v known at run time:
+// two conditional rotations.  (Each uniform picked by its own index took twice the
+// selects and their compares, on the ALU pipe that bounds the packet kernels: with the
+// spread above, 64 surfaces MIXED 4.01 -> 3.81 ms, EXACT 5.93 -> 5.74, 24 FAST 3.30 -> 3.11.)
+__device__ __forceinline__ void unpack_rotated(uint32_t w0, uint32_t w1, uint32_t w2, int v, float r[4])
+{
+    float uf[4];
+    unpack_uniforms(w0, w1, w2, uf);
+    const bool two = ((v + 1) & 2) != 0, one = ((v + 1) & 1) != 0;
+    const float a = two ? uf[2] : uf[0], b = two ? uf[3] : uf[1], c = two ? uf[0] : uf[2], d = two ? uf[1] : uf[3];
+    r[0] = one ? b : a;
+    r[1] = one ? c : b;
+    r[2] = one ? d : c;
+    r[3] = one ? a : d;
+}
+
 // Emission of the mixed-precision kernels.  A planar emitter (disc, annulus,
 // rectangle) has one world frame for all its rays: EmitFrame holds its origin
 // and in-plane axes (the columns of m) and the rotation that alignRayDirection
@@ -210,10 +226,11 @@ __device__ __forceinline__ int direction_cell(float x, float y, float z)
     const int i = min(kDirGrid - 1, max(0, (int)((u + 1.0f) * h)));
     const int j = min(kDirGrid - 1, max(0, (int)((v + 1.0f) * h)));
     static_assert(kDirGrid == 16, "4-bit Morton spread");
-    // spread the 4 bits of i and j to the even / odd bits of an 8-bit code
-    const int si = ((i | (i << 2)) & 0x33) | (((i | (i << 2)) & 0x33) << 1);
-    const int sj = ((j | (j << 2)) & 0x33) | (((j | (j << 2)) & 0x33) << 1);
-    return (si & 0x55) | ((sj & 0x55) << 1);
+    // spread the 4 bits of i and j to the even / odd bits of an 8-bit code, both at once
+    int k = i | (j << 16);
+    k = (k | (k << 2)) & 0x00330033;
+    k = (k | (k << 1)) & 0x00550055;
+    return (k | (k >> 15)) & 0xff;
 }
 
 // Can the ray (origin s, direction c, idd = 1/|c|^2) reach the sphere b?  b.w
@@ -988,14 +1005,9 @@ __global__ void __launch_bounds__(kBatchThreads, 1) batched_kernel(const __grid_
             Ray<float> ray;
             int cell = 0;
             {
-                const int d = l >> 2, v = l & 3;
-                float uf[4], r[4];
-                unpack_uniforms(S.unif[0][d], S.unif[1][d], S.unif[2][d], uf);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int q = (i + v + 1) & 3;
-                    r[i] = q == 0 ? uf[0] : (q == 1 ? uf[1] : (q == 2 ? uf[2] : uf[3]));
-                }
+                const int d = l >> 2;
+                float r[4];
+                unpack_rotated(S.unif[0][d], S.unif[1][d], S.unif[2][d], l & 3, r);
                 ray = emit_mixed(S.emit, S.frame, r);
                 cell = ray_key(ray, r);
             }

@@ -671,14 +671,9 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
             const int l = perm[valid ? pos : k * 32];  // (an idle lane repeats the packet's first ray)
             Ray<T> ray;
             {
-                const int d = l >> 2, v = l & 3;
-                float uf[4], r[4];
-                unpack_uniforms(unif[d], unif[cd + d], unif[2 * cd + d], uf);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int q = (i + v + 1) & 3;
-                    r[i] = q == 0 ? uf[0] : (q == 1 ? uf[1] : (q == 2 ? uf[2] : uf[3]));
-                }
+                const int d = l >> 2;
+                float r[4];
+                unpack_rotated(unif[d], unif[cd + d], unif[2 * cd + d], l & 3, r);
                 if constexpr (kMixed)
                     ray = emit_mixed(s_emit, s_mframe, r);
                 else if constexpr (M::kF64)
