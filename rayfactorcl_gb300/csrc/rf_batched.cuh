@@ -223,8 +223,9 @@ __device__ __forceinline__ int direction_cell(float x, float y, float z)
         v = vv;
     }
     constexpr float h = 0.5f * kDirGrid;
-    const int i = min(kDirGrid - 1, max(0, (int)((u + 1.0f) * h)));
-    const int j = min(kDirGrid - 1, max(0, (int)((v + 1.0f) * h)));
+    // |u|, |v| <= 1 + 2^-22 (0 or NaN for an infinite direction, and (int)NaN is 0)
+    const int i = min(kDirGrid - 1, (int)((u + 1.0f) * h));
+    const int j = min(kDirGrid - 1, (int)((v + 1.0f) * h));
     static_assert(kDirGrid == 16, "4-bit Morton spread");
     // spread the 4 bits of i and j to the even / odd bits of an 8-bit code, both at once
     int k = i | (j << 16);
@@ -351,8 +352,8 @@ static __device__ __noinline__ float sphere_f64(const HitRec &h, const Ray<float
     return (float)sphere_hit<MF64>(h, to_f64(w), (double)eps, sc);
 }
 
-// The mixed tests set `defer` instead of computing an ill-conditioned root: the
-// caller re-evaluates those tests in FP64 outside its hot loop.
+// The mixed tests set `defer` for an ill-conditioned root, whose t then means nothing:
+// every caller puts the FP64 test's in its place, or traces the ray again.
 __device__ __forceinline__ float cylinder_mixed(const HitRec &h, const Ray<float> &w, float eps, bool &defer)
 {
     const Ray<float> o = xfrm_ray<MFast>(h, w);
@@ -365,8 +366,8 @@ __device__ __forceinline__ float cylinder_mixed(const HitRec &h, const Ray<float
     const float disc = MFast::sqrt(d);  // NaN for a miss, rejected by the comparisons
     const float ra = MFast::rcp(A);
     const float t = quadric_pick<MFast>(o, ra * (B - disc), ra * (B + disc), eps);
-    defer = ill;  // selects, not a branch: the lanes of a warp stay together
-    return ill ? MFast::inf() : t;
+    defer = ill;
+    return t;
 }
 
 __device__ __forceinline__ float frustum_mixed(const HitRec &h, const Ray<float> &w, float eps, bool &defer)
@@ -393,7 +394,7 @@ __device__ __forceinline__ float frustum_mixed(const HitRec &h, const Ray<float>
     const float ra = MFast::rcp(A);
     const float t = quadric_pick<MFast>(o, ra * (B - disc), ra * (B + disc), eps);
     defer = ill;
-    return ill ? MFast::inf() : t;
+    return t;
 }
 
 __device__ __forceinline__ float sphere_mixed(const HitRec &h, const Ray<float> &w, float eps, bool sc,
@@ -415,7 +416,7 @@ __device__ __forceinline__ float sphere_mixed(const HitRec &h, const Ray<float> 
     const float t1 = (-B - d) * ra, t2 = (-B + d) * ra;
     const float t = t1 > eps ? t1 : (t2 > eps ? t2 : MFast::inf());
     defer = ill;
-    return ill ? MFast::inf() : t;
+    return t;
 }
 
 __device__ __forceinline__ float hit_mixed(int type, const HitRec &h, const Ray<float> &w, float eps,
@@ -479,7 +480,7 @@ __device__ __forceinline__ float stack_mixed(const HitRec &h, const Ray<float> &
     const float ra = MFast::rcp(A);
     const float t = stack_pick<MFast>(o, ra * (B - disc), ra * (B + disc), eps, (int)h.aux.y, ring);
     defer = ill;
-    return ill ? MFast::inf() : t;
+    return t;
 }
 
 static __device__ __noinline__ float stack_f64(const HitRec &h, const Ray<float> &w, float eps, int &ring)
@@ -581,8 +582,7 @@ static __device__ __noinline__ float2 deferred_f64(const HitRec *rec, int j, Ray
 // parameters (r[0], r[1]) of its emission point.
 __device__ __forceinline__ int ray_key(const Ray<float> &ray, const float r[4])
 {
-    return (direction_cell(ray.cx, ray.cy, ray.cz) << 4) | (min(3, (int)(r[0] * 4.0f)) << 2) |
-           min(3, (int)(r[1] * 4.0f));
+    return (direction_cell(ray.cx, ray.cy, ray.cz) << 4) | ((int)(r[0] * 4.0f) << 2) | (int)(r[1] * 4.0f);  // r < 1
 }
 
 // A planar emitter (disc, annulus, rectangle) cannot be hit by its own rays:

@@ -117,7 +117,7 @@ __device__ __forceinline__ int quick_key(const rf_primitive &e, const float4 *f,
         cy = fmaf(nz, oy, fmaf(-nx, k, ny * oz));
         cz = fmaf(nz, oz, -fmaf(nx, ox, ny * oy));
     }
-    return (direction_cell(cx, cy, cz) << 4) | (min(3, (int)(r[0] * 4.0f)) << 2) | min(3, (int)(r[1] * 4.0f));
+    return (direction_cell(cx, cy, cz) << 4) | ((int)(r[0] * 4.0f) << 2) | (int)(r[1] * 4.0f);
 }
 
 // Rotation rows of alignRayDirection (RayFactorGPU.cl:87-97) for a planar
