@@ -336,12 +336,13 @@ bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
 //     1.5e5 43 / 65, at 2e5 59 / 66, at 3e5 66 / 84; 201 at 2e5 157 / 201, at 3e5 219 / 206; 400
 //     at 1e4 35 / 230, at 1e5 160 / 304; 252 rings that the culled kernel searches as one
 //     stack at 1e4 22 / 48, at 1e5 92 / 92, at 2e5 186 / 97
-//   FAST  3 at 2.5e4 7.8 / 7.8, at 4.9e4 9.6 / 7.9; 32 at 1.5e5 19 / 26, at 2e5 28 / 26; 201 at 2e5 116 / 163, at 3e5 163 / 163
+//   FAST  3 at 2.5e4 7.8 / 7.8, at 4.9e4 9.6 / 7.9; 32 at 1.5e5 19 / 26, at 2e5 28 / 26; 201 at
+//     2e5 116 / 163, at 3e5 163 / 163
 //   MIXED  12 at 2e5 20 / 26; 32 at 2e5 36 / 39, at 3e5 41 / 39; 64 at 6e4 26 / 45, at 1.5e5
 //     47 / 49; 201 at 6e4 61 / 86, at 1.5e5 127 / 116; rings in stacks at 2e5 47 / 57; 1000 (no
 //     longer in the batched kernel's shared memory) at 2e5 854 / 1339
-//   FP64  3 at 1e4 24 / 94; 12 at 4e4 144 / 251; 32 at 4e4 297 / 359; 64 at 2e4 300 / 318, at 4e4
-//     457 / 524; 100 at 1e4 246 / 214
+//   FP64 (before either kernel kept its matrices in doubles)  3 at 1e4 24 / 94; 12 at 4e4
+//     144 / 251; 32 at 4e4 297 / 359; 64 at 2e4 300 / 318, at 4e4 457 / 524; 100 at 1e4 246 / 214
 int narrow_split(const rf_ctx *c, bool bv, const Budget &b)
 {
     const rf_config &f = c->cfg;

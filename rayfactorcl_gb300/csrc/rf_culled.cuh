@@ -26,13 +26,13 @@
 //   same radius, and a binary search finds the member.
 //
 // What bounds it: FP32 issue, like the batched mixed-precision kernel whose
-// structure it shares; in MF64 the FP64 pipe.  64 surfaces, EXACT, 1e8 rays: 5.9 ms
+// structure it shares; in MF64 the FP64 pipe.  64 surfaces, EXACT, 1e8 rays: 5.7 ms
 // (plain 18.2), of which draws, keys and sort 0.6, emission and packet bounds 1.3,
 // the spheres 2.2 (9 candidates per packet) and the tests 1.7 (5.3 per packet, of
 // which 2.4 find a hit for some ray; the plain kernel makes 64 per ray).  The
-// furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.07 ms EXACT
+// furnace (180-ring wall, two plates, bounding surfaces), 1e7 rays: 1.04 ms EXACT
 // (plain 7.9), 0.85 FAST (5.7); 1e6 rays in FP64 2.0 (35.4).  In mixed precision, 5e7
-// rays: 2.55 ms with bounding surfaces (3.36 as a variant of the batched kernel, which
+// rays: 2.48 ms with bounding surfaces (3.36 as a variant of the batched kernel, which
 // spilled 600 bytes a thread), 1.99 without (2.30); the reference's furnace model,
 // 2e7 rays, 0.96 (1.65).
 #pragma once

@@ -14,8 +14,9 @@
 // full, then issue: past 1e5 to 3e5 rays the kernels that sort do less work.
 // The arithmetic is the other kernels' own, so the results are theirs ray for ray.
 // Measured, us, the kernel used before / this one: 20 surfaces 1e4 rays EXACT 24 / 9.6,
-// FAST 14.5 / 7.7, MIXED 23 / 10, FP64 281 / 67; 400 surfaces 1e4 rays EXACT 230 / 35,
-// MIXED 135 / 36, 1e5 rays EXACT 304 / 165.  (rf_capi.cu, narrow_split, has the rule.)
+// FAST 14.5 / 7.7, MIXED 23 / 10; 48 surfaces FP64 183 / 105; 400 surfaces 1e4 rays
+// EXACT 230 / 34, MIXED 135 / 36, 1e5 rays EXACT 304 / 165.  (The rule: rf_capi.cu,
+// narrow_split.)
 #pragma once
 
 #include "rf_culled.cuh"

@@ -19,8 +19,9 @@ def rectangles():
     return sc
 
 
-SCENES = {"enclosure": lambda: generators.enclosure3(4).scene, "mixed9": lambda: mixed(9), "mixed17": lambda: mixed(17), "mixed120": lambda: mixed(120),
-          "rectangles": rectangles, "odd": odd_scene, "stress": lambda: generators.precision_stress(4).scene}
+SCENES = {"enclosure": lambda: generators.enclosure3(4).scene, "mixed9": lambda: mixed(9),
+          "mixed17": lambda: mixed(17), "mixed120": lambda: mixed(120), "rectangles": rectangles,
+          "odd": odd_scene, "stress": lambda: generators.precision_stress(4).scene}
 
 
 @pytest.mark.parametrize("compat", [0, COMPAT_SPHERE])
