@@ -117,7 +117,12 @@ def load() -> ctypes.CDLL:
 
 
 def ptr(a: np.ndarray | None):
-    return None if a is None else ctypes.c_void_p(a.__array_interface__["data"][0])
+    """Address of an array for a call; the pointer keeps the array alive."""
+    if a is None:
+        return None
+    p = ctypes.c_void_p(a.__array_interface__["data"][0])
+    p.array = a
+    return p
 
 
 def check(status: int, ctx=None):
