@@ -693,7 +693,8 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
             pk.cull = pk.cull && !odd;
 
             // candidate words of the 1024 positions from q0 on, lane w holding word w: by
-            // sphere (cmask), and frusta in whose band some ray of the packet lies (bmask)
+            // sphere (cmask), and frusta in whose band some ray of the packet lies (bmask; a
+            // packet too wide for packet_band looks at the band of every frustum)
             unsigned cmask = 0u, bmask = 0u;
             auto candidates = [&](int q0) {
                 const int nwords = min(32, (nc - q0 + 31) >> 5);
@@ -705,7 +706,7 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                         const float4 b = RESIDENT ? s_bs[q] : __ldg(p.bsph + q);
                         cand = (RESIDENT || b.w != 0.0f) && (!pk.cull || packet_reaches(pk, b));
                         if (kMixed) cand = cand && surface(q) != skip;
-                        if (!kMixed && b.w < 0.0f) banded = pk.cull && packet_band(p.cquad, surface(q), pk);
+                        if (!kMixed && b.w < 0.0f) banded = !pk.cull || packet_band(p.cquad, surface(q), pk);
                     }
                     const unsigned cm = __ballot_sync(0xffffffffu, cand);
                     unsigned bm = kMixed ? 0u : __ballot_sync(0xffffffffu, banded);
