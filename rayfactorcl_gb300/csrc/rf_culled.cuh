@@ -685,9 +685,10 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
             if (COUNT && lane == 7) ++tcount;
             const Ray<float> rf = to_f32(ray);
             const float cc = dot3(rf.cx, rf.cy, rf.cz, rf.cx, rf.cy, rf.cz);
-            // a ray the bounds do not speak for: its packet tests everything
-            const bool odd = __any_sync(0xffffffffu, !(fabsf(rf.sx) + fabsf(rf.sy) + fabsf(rf.sz) < 1e15f) ||
-                                                         !(cc > 1e-6f && cc < 1e6f));
+            // a ray the bounds do not speak for: its packet tests everything (mixed: a ray's
+            // own sphere checks always speak for it)
+            const bool odd = !kMixed && __any_sync(0xffffffffu, !(fabsf(rf.sx) + fabsf(rf.sy) + fabsf(rf.sz) < 1e15f) ||
+                                                                    !(cc > 1e-6f && cc < 1e6f));
             const float idd = MFast::rcp(cc);
             Packet pk = bounds_of(rf, idd);
             pk.cull = pk.cull && !odd;
@@ -728,7 +729,14 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                 else
                     return odd || reaches(rf, idd, b);
             };
-            auto test = [&](int j, T &tb, int &bi) {  // every lane, the same j
+            // the surface at q, every lane the same.  In mixed arithmetic a hit counts only if
+            // the lane's own gate admits the surface: the mixed spheres follow its m, its hits
+            // its invm, and a result must not depend on what else the packet tests.  (The gate is
+            // formed again for a nearer hit.  Furnace, bounding surfaces, 5e7 rays: 2.48 ms; the
+            // first one kept as a flag 2.60; the winner held against it after each search, with
+            // a search of the lane's own where it fails, 2.84.)
+            auto test = [&](int q, T &tb, int &bi) {
+                const int j = surface(q);
                 const HitRec h = RESIDENT ? s_tab[j] : load_rec(p.tab, j);
                 const int type = __float_as_int(h.aux.x);
                 if (COUNT) tcount += lane == (kMixed ? stat_type(type) : type) ? nvalid : 0;
@@ -742,7 +750,7 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                         idx = __float_as_int(q.y);
                         nref += valid;
                     }
-                    if (t < tb) {
+                    if (t < tb && gate(q, tb)) {
                         tb = t;
                         bi = idx;
                     }
@@ -797,10 +805,10 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                         if (two && (__any_sync(0xffffffffu, mb) || ((bm >> bb_) & 1u))) go |= 2u;
                         if constexpr (kMixed) {  // one copy of the tests: two spill (furnace 2.55 -> 2.60 ms)
 #pragma unroll 1
-                            for (; go; go &= go - 1) test(surface(qw + ((go & 1u) ? ba_ : bb_)), tb, bi);
+                            for (; go; go &= go - 1) test(qw + ((go & 1u) ? ba_ : bb_), tb, bi);
                         } else {  // two: no loop to step (64 surfaces FAST 5.03 -> 4.95 ms)
-                            if (go & 1u) test(surface(qw + ba_), tb, bi);
-                            if (go & 2u) test(surface(qw + bb_), tb, bi);
+                            if (go & 1u) test(qw + ba_, tb, bi);
+                            if (go & 2u) test(qw + bb_, tb, bi);
                         }
                     }
                 }
@@ -820,7 +828,7 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                                        sc, M::inf());
                     else
                         t = shell_hit<M>(s_bvtab + w, ray, eps, sc);
-                    const bool nearer = t < tbest;
+                    const bool nearer = t < tbest && (!kMixed || reaches(rf, idd, s_bvbs[w]));
                     if (!__any_sync(0xffffffffu, nearer)) continue;
                     const int4 info = s_bvinfo[w];
                     T tn = M::inf();

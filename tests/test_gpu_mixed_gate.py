@@ -1,0 +1,83 @@
+"""A ray's result in mixed precision is a function of the ray alone: of neither its packet
+nor the kernel that its trace takes.  Transforms whose invm describes a larger surface
+than m (both are the caller's) put hits outside the bounding spheres, which follow m, so
+that any kernel that keeps a hit its ray's own sphere check refuses shows up."""
+import numpy as np
+import pytest
+
+from rayfactorcl_gb300 import generators
+from rayfactorcl_gb300.scene import BV_DTYPE, SPHERE, Scene, parse_scene_xml
+from rayfactorcl_gb300.tracer import PREC_EXACT, PREC_MIXED, Tracer
+
+from test_gpu_culled import mixed
+
+pytestmark = pytest.mark.gpu
+
+
+def coaxial(x, kind, k):
+    """k rings that tile a cylinder, or k annuli that tile an annulus, on a tilted axis."""
+    rot = (-50.0, (0.6, 0.8, 0.0))
+    t = np.array([1.0, -2.0, 0.5])
+    if kind == "rings":
+        axis = _axis(rot)
+        for i in range(k):
+            x.prim("cylinderSurface", small=1.0, scale=(0.4, 0.4, 0.2), rotate=rot, translate=t + 0.2 * i * axis)
+            x.close()
+    else:
+        e = np.linspace(0.2, 1.0, k + 1)
+        for i in range(k):
+            x.prim("annulus", small=float(e[i]), large=float(e[i + 1]), rotate=rot, translate=t)
+            x.close()
+
+
+def _axis(rot):
+    x = generators._Xml("axis")
+    x.prim("cylinderSurface", small=1.0, scale=(1.0, 1.0, 1.0), rotate=rot)
+    x.close()
+    return parse_scene_xml(x.text()).primitives["m"][0].reshape(3, 4)[:, 2].astype(float)
+
+
+def scene(n, stack=None, grown=1.0):
+    """n surfaces of every type, the odd ones `grown` times as large for the tests as for
+    emission, and a stack or plate of four."""
+    sc = mixed(n, seed=29)
+    sc.primitives["invm"][1::2] /= np.float32(grown)
+    if stack:
+        x = generators._Xml("stack")
+        coaxial(x, stack, 4)
+        out = Scene()
+        out.primitives = np.concatenate([sc.primitives, parse_scene_xml(x.text()).primitives])
+        sc = out
+    return sc
+
+
+def with_shells(sc):
+    """The halves of the surfaces under two bounding spheres, one of them larger than its invm says."""
+    b = np.zeros(2, BV_DTYPE)
+    h = sc.n // 2
+    b["type"], b["util2"], b["settings"] = SPHERE, -1.0, (1, 0)
+    b["objStartIndex"], b["objEndIndex"] = (0, h), (h, sc.n)
+    for k, r in enumerate((7.0, 9.0)):
+        b["invm"][k] = (np.eye(4)[:3] / r).astype(np.float32).ravel()
+    sc.bounding_volumes = b
+    return sc
+
+
+def budgets(sc, total):
+    rng = np.random.Generator(np.random.PCG64(7))
+    return np.floor(rng.uniform(0.2, 1.8, size=sc.n) * total / sc.n).astype(np.int64) + 1
+
+
+@pytest.mark.parametrize("bv", [False, True])
+def test_packets_do_not_matter(built_lib, bv):
+    """Packets form in another order with another grid, and from run to run."""
+    sc = scene(60, "rings", grown=1.5)
+    if bv:
+        sc = with_shells(sc)
+    rays = budgets(sc, 3_000_000)
+    got = []
+    for grid in (0, 0, 37):
+        with Tracer(precision=PREC_MIXED, key1=3, batched_grid=grid) as t:
+            t.set_scene(sc)
+            got.append(t.trace(rays, use_bv=bv)[0])
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
