@@ -572,7 +572,9 @@ __global__ void __launch_bounds__(THREADS, 1) culled_kernel(const TraceParams p)
                 if (tid == 32 % THREADS) quick_frame(p.emit[sg.emitter], s_frame);
                 if (kMixed && tid < kFrameWords) s_mframe[tid] = p.frame[(int64_t)sg.emitter * kFrameWords + tid];
                 emitter = sg.emitter;
-                if (kMixed) skip = planar(p.emit[emitter].type) ? emitter : -1;
+                // (a plate's first member stands for all of it: the others are tested through it)
+                if (kMixed)
+                    skip = planar(p.emit[emitter].type) && !is_stack(__float_as_int(__ldg(&p.tab[emitter].aux.x))) ? emitter : -1;
             }
         }
         for (int i = tid; i < kCells; i += THREADS) cnt[i] = 0;

@@ -81,3 +81,16 @@ def test_packets_do_not_matter(built_lib, bv):
             t.set_scene(sc)
             got.append(t.trace(rays, use_bv=bv)[0])
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("member", [0, 2])
+def test_emitters_of_a_plate(built_lib, member):
+    """With next to no self-hit threshold a plate's emitter sees its plate's plane at
+    rounding distance: the same in every kernel."""
+    sc = scene(40, "plate")
+    e = 40 + member
+    with Tracer(precision=PREC_MIXED, eps=1e-12) as t:
+        t.set_scene(sc)
+        whole = t.trace_rays(e, 0, 300_000)
+        parts = np.concatenate([t.trace_rays(e, k, 30_000) for k in range(0, 300_000, 30_000)])
+    assert np.array_equal(whole, parts)
