@@ -246,6 +246,22 @@ __device__ __forceinline__ bool ray_may_hit(const Ray<float> &r, float idd, cons
     return fmaf(-bb * bb, idd, oc2) <= b.w;
 }
 
+__device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz)
+{
+    return fmaf(ax, bx, fmaf(ay, by, az * bz));
+}
+
+// The same for the culled kernel (rf_culled.cuh), with every product and sum fused
+// explicitly (two of its four translation units are compiled with -fmad=false); |b.w|
+// is the squared radius.
+__device__ __forceinline__ bool reaches(const Ray<float> &r, float idd, const float4 b)
+{
+    const float ox = b.x - r.sx, oy = b.y - r.sy, oz = b.z - r.sz;
+    const float oc2 = dot3(ox, oy, oz, ox, oy, oz);
+    const float bb = fmaxf(dot3(ox, oy, oz, r.cx, r.cy, r.cz), 0.0f);
+    return fmaf(-bb * bb, idd, oc2) <= fabsf(b.w);
+}
+
 // Bounds of a packet of 32 rays, the same in every lane.
 struct Packet {
     float ox, oy, oz, rho;  // origin ball
@@ -611,10 +627,11 @@ __device__ __forceinline__ unsigned keep_from(int k)
 }
 
 // Full nearest-hit search for one ray over the surfaces [0, n) its gate admits (the
-// cell mask when mcell is set, and the bounding-sphere check) but skip, with FP64 for
-// every ill-conditioned quadric: the surface, and in y the FP64 evaluations.  tab, bs: shared or global memory.  Cold path; by
+// cell mask when mcell is set, and the bounding-sphere check; FUSED: the culled kernel's
+// sphere check alone) but skip, with FP64 for every ill-conditioned quadric: the surface,
+// and in y the FP64 evaluations.  tab, bs: shared or global memory.  Cold path; by
 // value, so that the callers' ray stays in registers.
-template <bool STK>
+template <bool STK, bool FUSED = false>
 static __device__ __noinline__ int2 retrace_f64(int n, const HitRec *tab, const float4 *bs, const uint32_t *mcell,
                                                 Ray<float> ray, float idd, float eps, bool sc, int skip)
 {
@@ -622,7 +639,7 @@ static __device__ __noinline__ int2 retrace_f64(int n, const HitRec *tab, const 
     int bi = -1, nf64 = 0;
     for (int j = 0; j < n; ++j) {
         if (j == skip) continue;
-        if (!own_gate(mcell, j, ray, idd, bs[j])) continue;
+        if (!(FUSED ? reaches(ray, idd, bs[j]) : own_gate(mcell, j, ray, idd, bs[j]))) continue;
         const HitRec h = tab[j];
         const int type = __float_as_int(h.aux.x);
         bool defer = false;

@@ -1043,6 +1043,7 @@ int batched_grid(rf_ctx *c, bool rec)
 }
 
 bool mixed_culled(const rf_ctx *c, bool bv);
+bool small_trace(const rf_ctx *c, bool bv);
 
 // The narrow kernel on the scene held in the batch tables.
 rf_status run_mixed_narrow(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec, int32_t *d_rec,
@@ -1063,6 +1064,7 @@ rf_status run_mixed_narrow(rf_ctx *c, const std::vector<Segment> &seg, int64_t t
     p.total_chunks = total_chunks;
     p.rec = d_rec;
     p.rec_base = rec_base;
+    p.gate = small_trace(c, false) ? 0 : (mixed_culled(c, false) ? 1 : 2);  // larger traces': the same results
     RF_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     RF_CUDA(c, launch_mixed_narrow(p, split, rec, c->sms, c->stream));
     RF_CUDA(c, cudaEventRecord(c->ev1, c->stream));

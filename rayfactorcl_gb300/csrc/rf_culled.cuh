@@ -65,11 +65,6 @@ struct CulledLayout {
     }
 };
 
-__device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz)
-{
-    return fmaf(ax, bx, fmaf(ay, by, az * bz));
-}
-
 __device__ __forceinline__ Ray<float> to_f32(const Ray<float> &r) { return r; }
 __device__ __forceinline__ Ray<float> to_f32(const Ray<double> &r)
 {
@@ -135,18 +130,7 @@ __device__ __forceinline__ void quick_frame(const rf_primitive &e, float4 *f)
     f[2] = make_float4(-x, -y, z, 0.0f);
 }
 
-// As ray_may_hit and packet_bounds / packet_may_hit of the batched kernel, with
-// every product and sum fused explicitly (two of the three translation units
-// are compiled with -fmad=false); |b.w| is the squared radius.
-__device__ __forceinline__ bool reaches(const Ray<float> &r, float idd, const float4 b)
-{
-    const float ox = b.x - r.sx, oy = b.y - r.sy, oz = b.z - r.sz;
-    const float oc2 = dot3(ox, oy, oz, ox, oy, oz);
-    const float bb = fmaxf(dot3(ox, oy, oz, r.cx, r.cy, r.cz), 0.0f);
-    return fmaf(-bb * bb, idd, oc2) <= fabsf(b.w);
-}
-
-// The same for the ray's points up to the nearest hit so far, beyond which no hit
+// As reaches (rf_batched.cuh), for the ray's points up to the nearest hit so far, beyond which no hit
 // counts: the distance from the centre at the nearest parameter t of those, oc2 - 2 t
 // bb + t^2 cc, rounded by a few u reach^2 (the spheres allow for 64, rf_bounds.cu:
 // check_w).  For FP64, whose tests cost 70 times a gate: 1e6 rays 48 surfaces 1.37 ->
@@ -162,6 +146,7 @@ __device__ __forceinline__ bool reaches_before(const Ray<float> &r, float cc, fl
     return fmaf(t, fmaf(t, cc, -bb) - bb, oc2) <= fabsf(b.w);
 }
 
+// As packet_bounds and packet_may_hit of the batched kernel, fused like reaches.
 __device__ __forceinline__ Packet bounds_of(const Ray<float> &r, float idd)
 {
     Packet pk;

@@ -74,6 +74,8 @@ struct TraceParams {
     const double *tab64;            // culled kernel in FP64: invm of each surface, then bounding surface, 12 doubles
     int32_t chunk_draws;            // batched and culled kernels: draws of a chunk
     const int32_t *d_chunk;         // batched kernel: the same, device-resident (or null)
+    int32_t gate;                   // narrow kernel, mixed: the gate a hit must pass: 0 none, 1 the culled
+                                    // kernel's spheres, 2 the batched kernel's masks and spheres
 };
 
 // Cell masks of the batched kernel (rf_masks.cu): one bit per surface for

@@ -12,7 +12,10 @@
 // as in the single loop.  A part repeats the emission, about 16 tests' time.  What
 // bounds it is a warp's latency (n / SPLIT tests one after the other) until the GPU is
 // full, then issue: past 1e5 to 3e5 rays the kernels that sort do less work.
-// The arithmetic is the other kernels' own, so the results are theirs ray for ray.
+// The arithmetic is the other kernels' own, so the results are theirs ray for ray; in
+// mixed arithmetic, where those of larger traces count a hit only when the ray's own gate
+// admits its surface (p.gate), the winner is held against that gate, and a ray whose
+// winner fails it is traced again over the surfaces it admits.
 // Measured, us, the kernel used before / this one: 20 surfaces 1e4 rays EXACT 24 / 9.6,
 // FAST 14.5 / 7.7, MIXED 23 / 10; 48 surfaces FP64 183 / 105; 400 surfaces 1e4 rays
 // EXACT 230 / 34, MIXED 135 / 36, 1e5 rays EXACT 304 / 165.  (The rule: rf_capi.cu,
@@ -97,6 +100,9 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
         else
             ray = emit_ray<M>(s_emit, r);
         const int skip = kMixed && planar(s_emit.type) ? sg.emitter : -1;
+        int cell = 0;  // the batched kernel's sort key of the ray
+        if constexpr (kMixed)
+            if (p.gate == 2) cell = ray_key(ray, r);
         T tb = M::inf();
         int bi = -1;
 #pragma unroll 1
@@ -143,6 +149,28 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
                     if (s_t[tid + 32 * q] < tb) {  // (a tie: the earlier part's, the lower index)
                         tb = s_t[tid + 32 * q];
                         bi = s_i[tid + 32 * q];
+                    }
+                }
+            }
+        }
+        if constexpr (kMixed) {
+            if (p.gate && part == 0 && valid && bi >= 0) {
+                const float4 b = __ldg(p.bsph + bi);
+                if (p.gate == 1) {  // the culled kernel's
+                    const float idd = MFast::rcp(dot3(ray.cx, ray.cy, ray.cz, ray.cx, ray.cy, ray.cz));
+                    if (!reaches(ray, idd, b)) {
+                        const int2 q = retrace_f64<true, true>(n, s_tab, p.bsph, nullptr, ray, idd, eps, sc, skip);
+                        bi = q.x;
+                        nref += q.y;
+                    }
+                } else {  // the batched kernel's
+                    const float idd = MFast::rcp(ray.cx * ray.cx + ray.cy * ray.cy + ray.cz * ray.cz);
+                    const int64_t mo = p.mask_off ? p.mask_off[sg.emitter] : -1;
+                    const uint32_t *mcell = mo < 0 ? nullptr : p.cmask + mo + cell * ((n + 31) >> 5);
+                    if (!own_gate(mcell, bi, ray, idd, b)) {
+                        const int2 q = retrace_f64<true>(n, s_tab, p.bsph, mcell, ray, idd, eps, sc, skip);
+                        bi = q.x;
+                        nref += q.y;
                     }
                 }
             }

@@ -83,6 +83,23 @@ def test_packets_do_not_matter(built_lib, bv):
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
 
 
+@pytest.mark.parametrize("n,stack", [(14, None), (60, None), (60, "rings"), (60, "plate"), (600, None)])
+def test_split_run_is_the_whole_run(built_lib, n, stack):
+    """Ranges of few rays take another kernel than the whole run."""
+    sc = scene(n, stack, grown=1.5)
+    rays = budgets(sc, 300_000)
+    with Tracer(precision=PREC_MIXED, key1=3) as t:
+        t.set_scene(sc)
+        whole = t.trace(rays)[0]
+        first = np.zeros(sc.n, np.int64)
+        while (first < rays).any():
+            count = np.minimum(rays - first, 20_000 // sc.n + 3)
+            t.trace_range(first, count, accumulate=bool(first.any()))
+            first = first + count
+        parts = t.results()[0]
+    assert np.array_equal(whole, parts)
+
+
 @pytest.mark.parametrize("member", [0, 2])
 def test_emitters_of_a_plate(built_lib, member):
     """With next to no self-hit threshold a plate's emitter sees its plate's plane at
