@@ -329,6 +329,13 @@ float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, 
     const double cn = std::sqrt(dot(b.c, b.c));
     const double r = b.r * (1.0 + 1e-5) + 1e-6 * (cn + b.r) + 1e-7;
     if (!(r < (double)box.w)) return box;
+    // the hits follow invm: where it places the surface elsewhere than m does (half of the
+    // check's own widening is allowed for), the box's sphere as well as it can
+    double Mi[9], ti[3], d[3];
+    if (!inverse_of(e.invm, Mi, ti)) return box;
+    const Ball h = image_ball(Mi, ti, x);
+    for (int k = 0; k < 3; ++k) d[k] = h.c[k] - b.c[k];
+    if (!(std::sqrt(dot(d, d)) + h.r <= 1.005 * r)) return box;
     return make_float4((float)b.c[0], (float)b.c[1], (float)b.c[2], (float)r);
 }
 

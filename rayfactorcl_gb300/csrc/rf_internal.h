@@ -134,7 +134,8 @@ template <class M> cudaError_t launch_culled(const TraceParams &p, bool bv, bool
 // many; outer2: an annulus's, or a plate's, outer radius squared.  A frustum's rims
 // move out by what rounding can shift a root along a ray of length reach where its A
 // has lost the 12 bits that the FP32 test still accepts (kCondA).  loose_balls: keep
-// the box's sphere for spheres (RF_COMPAT_SPHERE's uncorrected discriminant).
+// the box's sphere for spheres (RF_COMPAT_SPHERE's uncorrected discriminant).  The box's
+// sphere stays also where invm, which the tests use, is not the inverse of m.
 float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, double reach, bool loose_balls);
 
 // Few rays: one ray a thread, the surfaces split over `split` warps (rf_narrow.cuh;
