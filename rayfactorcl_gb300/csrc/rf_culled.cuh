@@ -48,8 +48,8 @@ namespace rf {
 // candidates, in index order (a stack's first member stands for all), with bs in the
 // same order: a furnace's 252 surfaces are 35.
 struct CulledLayout {
-    int cnt, perm, unif, tab, bs, bvtab, bvinfo, bvbs, hist, live, bytes;
-    __host__ __device__ CulledLayout(int cd, int nres, int nhist, int nbv)
+    int cnt = 0, perm = 0, unif = 0, tab = 0, bs = 0, bvtab = 0, bvinfo = 0, bvbs = 0, hist = 0, live = 0, bytes = 0;
+    __host__ __device__ constexpr CulledLayout(int cd, int nres, int nhist, int nbv)
     {
         cnt = 0;
         perm = cnt + kCells * 4;
@@ -877,7 +877,11 @@ static cudaError_t launch_culled_k(const TraceParams &p, int blocks, cudaStream_
     constexpr int THREADS = M::kF64 ? 512 : 1024;
     auto k = culled_kernel<M, THREADS, BV, REC, RES, COUNT>;
     const int smem = CulledLayout(p.chunk_draws, RES ? p.n : 0, !REC && p.use_smem_hist ? p.n : 0, BV ? p.nbv : 0).bytes;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the largest launch's size always: the attribute is the function's on the device, and
+    // another thread's context may launch it between this call and ours
+    constexpr CulledLayout most(kChunkDraws, RES ? kBatchTile : 0, REC ? 0 : kBatchHist, BV ? kBatchMaxBV : 0);
+    static_assert(most.bytes <= 225 * 1024, "shared memory of a block, with 2 KB for the static arrays");
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most.bytes);
     if (e != cudaSuccess) return e;
     const int grid = (int)max((int64_t)1, min((int64_t)blocks, p.total_chunks));
     k<<<grid, THREADS, smem, st>>>(p);

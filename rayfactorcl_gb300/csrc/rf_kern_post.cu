@@ -432,10 +432,11 @@ __global__ void __launch_bounds__(kSmoothThreads, 1)
 
 // Workspace in bytes: two 16-byte-tagged buffers of x and of the errors, the state,
 // and, where a block's rows do not fit shared memory, G and the blocks' copies of x.
+constexpr size_t kSmoothShared = 216 * 1024;  // most that a block's rows and x take
 static bool smooth_resident(int n, int grid)
 {
     const size_t rows = (n + grid - 1) / grid;
-    return (rows + 1) * n * sizeof(double) <= 216 * 1024;
+    return (rows + 1) * n * sizeof(double) <= kSmoothShared;
 }
 size_t smooth_bytes(int n, int sms)
 {
@@ -456,7 +457,10 @@ cudaError_t launch_smooth(const double *F, const double *A, int n, int closed, i
     if (e != cudaSuccess) return e;
     const size_t rows = (n + grid - 1) / grid, smem = resident ? (rows + 1) * n * sizeof(double) : 0;
     const void *k = resident ? (const void *)smooth_kernel<true> : (const void *)smooth_kernel<false>;
-    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    // (the largest launch's size, whatever this one takes: the attribute is the function's, and
+    // another thread's context may launch it at the same time)
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, resident ? (int)kSmoothShared : 0)) != cudaSuccess)
+        return e;
     void *args[] = {&F, &A, &n, &closed, &max_iter, &tol, &G, &xg, &xbuf, &ebuf, &F_out, &ds};
     if ((e = cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kSmoothThreads), args, smem, st)) != cudaSuccess) return e;
     SmoothState h{};

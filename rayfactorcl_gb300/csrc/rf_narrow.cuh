@@ -194,10 +194,11 @@ __global__ void __launch_bounds__(kNarrowThreads, M::kF64 ? 2 : kNarrowBlocks) n
 template <class M, int SPLIT>
 static cudaError_t launch_narrow_s(const TraceParams &p, bool rec, int sms, cudaStream_t st)
 {
-    const size_t smem = (size_t)p.n * (sizeof(HitRec) + (M::kF64 ? 12 * sizeof(double) : 0));
+    constexpr size_t kRec = sizeof(HitRec) + (M::kF64 ? 12 * sizeof(double) : 0);
+    const size_t smem = p.n * kRec;
     const void *k = rec ? (const void *)narrow_kernel<M, SPLIT, true> : (const void *)narrow_kernel<M, SPLIT, false>;
-    if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 40 * 1024) {  // (the largest launch's size: see launch_culled_k)
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kNarrowMax * kRec));
         if (e != cudaSuccess) return e;
     }
     const int per_sm = M::kF64 ? 2 : kNarrowBlocks;
