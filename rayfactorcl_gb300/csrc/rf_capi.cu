@@ -141,6 +141,7 @@ struct rf_ctx {
     // 2 = batched kernel (set by rf_autotune)
     int mixed_path = 0;
     int b_stacks = 0;  // segment stacks in the mixed tables
+    int b_tests = 0;   // tests of scene 0 there: its surfaces, a stack as one
     std::vector<int> b_test_type;  // scene 0 of the mixed tables: type each surface's test counts as
                                    // (a stack: RF_CYLINDER at its first member, -1 at the others)
     bool last_small = false;                 // the last MIXED launch was the small-scene kernel
@@ -343,6 +344,8 @@ bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
 //     longer in the batched kernel's shared memory) at 2e5 854 / 1339
 //   FP64 (before either kernel kept its matrices in doubles)  3 at 1e4 24 / 94; 12 at 4e4
 //     144 / 251; 32 at 4e4 297 / 359; 64 at 2e4 300 / 318, at 4e4 457 / 524; 100 at 1e4 246 / 214
+bool mixed_culled(const rf_ctx *c, bool bv);
+
 int narrow_split(const rf_ctx *c, bool bv, const Budget &b)
 {
     const rf_config &f = c->cfg;
@@ -355,7 +358,7 @@ int narrow_split(const rf_ctx *c, bool bv, const Budget &b)
     switch (f.precision) {
     case RF_PREC_FP64: most = n <= 64 ? std::min<int64_t>(50000, 1200000 / n) : 0; break;
     case RF_PREC_FAST: most = n < 200 ? 160000 : 220000; break;
-    case RF_PREC_MIXED: most = n <= 40 || n > kBatchTile || c->b_stacks > 0 ? 200000 : 90000; break;
+    case RF_PREC_MIXED: most = n <= 40 || n > kBatchTile || mixed_culled(c, false) ? 200000 : 90000; break;
     default: most = n < 128 ? 220000 : 100000; break;
     }
     if (rays > std::min<int64_t>(most, 16000 * n)) return 0;
@@ -903,12 +906,14 @@ rf_status upload_batch(rf_ctx *c, const rf_scene_desc *scenes, int ns, bool with
                                        s == 0 ? cut0 : std::vector<char>());
         if (s == 0) {
             c->b_test_type.assign(n, 0);
+            c->b_tests = 0;
             for (int i = 0; i < n; ++i) {
                 int32_t ti, w;
                 std::memcpy(&ti, &tab[off + i].aux.x, 4);
                 std::memcpy(&w, &tab[off + i].aux.w, 4);
                 const int own = ti == kStackType ? (int)RF_CYLINDER : (ti == kPlateType ? (int)RF_ANNULUS : ti);
                 c->b_test_type[i] = (ti < kStackType || (w & 0xffff) == 0) ? own : -1;
+                c->b_tests += c->b_test_type[i] >= 0;
             }
         }
         for (int i = 0; i < n; ++i) bs[off + i] = widen_sq(bs[off + i], reach_slack(reach));
@@ -1042,7 +1047,6 @@ int batched_grid(rf_ctx *c, bool rec)
     return c->cfg.batched_grid > 0 ? std::min(wave, (int)c->cfg.batched_grid) : wave;
 }
 
-bool mixed_culled(const rf_ctx *c, bool bv);
 bool small_trace(const rf_ctx *c, bool bv);
 
 // The narrow kernel on the scene held in the batch tables.
@@ -1140,10 +1144,18 @@ int small_gpt(const rf_ctx *c, bool rec, bool bv = false)
 }
 
 // Single scenes that the culled kernel traces in MIXED precision: with bounding
-// surfaces, and with segment stacks, whose members it need not look at.
+// surfaces, and where nearly all surfaces are in segment stacks, whose members it need not
+// look at; else the batched kernel's cell masks leave more out.  Batched / culled, ms at
+// 1e7 rays, by the share of tests (a stack is one) in the surfaces, 200 surfaces far apart
+// and overlapping, 400 the same  1/2: 0.63 / 0.65, 3.19 / 3.88, 1.07 / 1.09, 6.57 / 7.90;
+// 1/4: 0.49 / 0.42, 1.84 / 2.16, 0.83 / 0.71, 3.50 / 4.06; 1/6: 0.45 / 0.37, 1.29 / 1.46,
+// 0.73 / 0.55, 2.65 / 2.95; 1/16: 0.38 / 0.28, 0.74 / 0.74, 0.65 / 0.38, 1.42 / 1.39; one ring
+// pair in 200 rectangles 4.8 / 6.8; furnaces of 35 tests in 252 surfaces 0.54 / 0.47, 18 in
+// 412 0.80 / 0.48.
 bool mixed_culled(const rf_ctx *c, bool bv)
 {
-    return c->b_single && !small_trace(c, bv) && (bv || (c->b_stacks > 0 && c->n <= kBatchTile));
+    return c->b_single && !small_trace(c, bv) &&
+           (bv || (c->b_stacks > 0 && c->n <= kBatchTile && 6 * c->b_tests <= c->n));
 }
 
 int mixed_split(const rf_ctx *c, bool bv, const Budget &b)
