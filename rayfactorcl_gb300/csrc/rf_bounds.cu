@@ -313,6 +313,20 @@ int ring_stack(const rf_primitive *prims, int n, int i, const std::vector<char> 
     return four && tiles(4) ? 4 : 1;
 }
 
+// The share of an emitter's packets that reach ball b, roughly: rays start within 0.4 of
+// the emitter's radius of each other and span 0.15 about their axis (a sort cell), which
+// points anywhere.
+double packet_share(const Ball &e, const Ball &b)
+{
+    if (!std::isfinite(b.r)) return 1.0;
+    double d[3];
+    for (int k = 0; k < 3; ++k) d[k] = b.c[k] - e.c[k];
+    const double L = std::sqrt(dot(d, d)), R = b.r + 0.4 * e.r;
+    if (!(L > R)) return 1.0;
+    const double s = R / L;
+    return 0.5 * (1.0 - (std::sqrt(1.0 - s * s) * std::cos(0.15) - s * std::sin(0.15)));
+}
+
 }  // namespace
 
 float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, double reach, bool loose_balls)
@@ -349,7 +363,7 @@ float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, 
 }
 
 bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs, int nbv, bool stacks, HitRec *tab,
-                 float4 *sph, float4 *quad, float4 *slack, float4 *bvsph)
+                 float4 *sph, float4 *quad, float4 *slack, float4 *bvsph, CullReach *reach)
 {
     // where rays start: the emitters' surfaces under m (a frustum's z from its own
     // formula, RayFactorGPU.cl:369-393, which loses digits as util1 nears 1)
@@ -394,6 +408,8 @@ bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs
         return make_float4((float)b.c[0], (float)b.c[1], (float)b.c[2], frustum ? -w : w);
     };
 
+    const int nsample = std::min(n, 16);
+    *reach = CullReach{};
     int bounded = 0;
     for (int i = 0; i < n;) {
         const rf_primitive &p = prims[i];
@@ -412,6 +428,15 @@ bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs
         quad[2 * i] = quad[2 * i + 1] = make_float4(0.f, 0.f, 0.f, INFINITY);
         const Ball b = hit_ball(p.invm, p.type, p.util1, x, from, smax, quad + 2 * i);
         const float4 s = ball_out(b, p.type == RF_FRUSTUM);
+        double share = 0.0;
+        for (int q = 0; q < nsample; ++q) share += packet_share(emit[(size_t)q * n / nsample], b) / nsample;
+        if (p.type == RF_CYLINDER || p.type == RF_SPHERE || p.type == RF_FRUSTUM) {
+            (p.type == RF_FRUSTUM ? reach->cones : reach->round) += (float)(m > 1 ? 3.0 * share : share);
+            reach->ncurved += m;
+        } else {
+            reach->planar += (float)(m > 1 ? 2.0 * share : share);
+            reach->nplanar += m;
+        }
         if (std::isfinite(s.w)) bounded += m;
         double M[9], t[3];
         if (m == 1 && std::isfinite(s.w) && inverse_of(p.invm, M, t))

@@ -107,6 +107,7 @@ struct rf_ctx {
     DevBuf d_tab, d_emit, d_bvtab, d_bvinfo;
     std::vector<rf_bounding_volume> bvs;
     int cull = 0;   // the culled kernel's tables: 0 not made yet, 1 in d_cull, -1 of no use for this scene
+    CullReach reach{};  // of those tables
     DevBuf d_cull;  // hit records (n), then float4: spheres (n), cone words (2 n), slack (n), bounding
                     // surfaces' spheres (nbv), and in FP64 each one's invm in doubles (6 (n + nbv))
     bool tuning = false;  // rf_autotune is timing the plain kernel's launch shapes
@@ -314,9 +315,13 @@ struct Plan {
 //   a few hundred rays per emitter leave most threads of a plain chunk idle: 1e4 rays,
 //     64 surfaces EXACT 0.033 / 0.056, FAST 0.029 / 0.032 (bounding surfaces only: other
 //     traces of so few rays take the narrow kernel).
-// The tables are made for the first trace that takes this kernel (about 40 us at 64
+// Those are scenes whose surfaces lie apart.  Where a packet's rays reach most of them (coaxial
+// shells, parallel baffles), the sort and the gates are for nothing: see culled_gains.
+// The tables are made for the first trace that may take this kernel (about 40 us at 64
 // surfaces), not in rf_set_scene, where a scene traced otherwise would pay for them.
-bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
+bool culled_gains(const rf_ctx *c, const Budget &b);
+
+bool culled_pays(const rf_ctx *c, bool bv, const Budget &b)
 {
     const rf_config &f = c->cfg;
     if (f.precision == RF_PREC_MIXED || c->tuning || f.block_size || f.rays_per_thread || f.tally_mode || f.table_mode ||
@@ -324,10 +329,51 @@ bool culled_pays(const rf_ctx *c, bool bv, int64_t draws)
         return false;
     if (bv && (c->n > kBatchTile || c->nbv > kBatchMaxBV)) return false;
     const int n = c->n;
-    const int64_t rays = 4 * draws;
-    if (f.precision == RF_PREC_FP64) return n >= 8 || (n >= 3 && rays >= 250000);
-    if (f.precision == RF_PREC_FAST) return n >= 256 || (n >= 24 && rays >= 1000000) || (n >= 64 && rays <= 200 * n);
-    return n >= 128 || (n >= 16 && rays >= 400000) || (n >= 24 && rays <= 400 * n);
+    const int64_t rays = 4 * b.draws;
+    bool may, sure;
+    if (f.precision == RF_PREC_FP64) {
+        may = n >= 8 || (n >= 3 && rays >= 250000);
+        sure = rays >= 150000 || rays <= 1500 * n;
+    } else if (f.precision == RF_PREC_FAST) {
+        sure = n >= 64 && rays <= 200 * n;
+        may = sure || n >= 256 || (n >= 24 && rays >= 1000000);
+    } else {
+        sure = n >= 24 && rays <= 200 * n;
+        may = sure || n >= 128 || (n >= 24 && (rays >= 400000 || rays <= 400 * n)) || (n >= 16 && rays >= 1000000);
+    }
+    return may && (sure || c->cull <= 0 || culled_gains(c, b));
+}
+
+// Does culling leave enough out: the culled kernel's tests, each about 2.5 (planar), 1.4
+// (cylinders, spheres; FAST 1.7) or 1.55 (frusta; FAST 2.4) times the plain kernel's, which
+// has four rays a thread to overlap, against the plain kernel's, every surface.  The limits
+// are where the two kernels' times met, for 16 to 400 surfaces of five kinds at seven
+// densities (packets that reach all surfaces down to a twentieth): lower for few rays, whose
+// packets are less alike and leave SMs idle.  Plain / culled, ms at 1e7 rays, 64 surfaces
+// of every type with centres in [-s, s]^3:  s = 3 EXACT 1.57 / 0.63, FAST 1.00 / 0.55; s = 1
+// 1.58 / 1.52, 1.01 / 1.30; s = 0.1 1.61 / 2.58, 1.03 / 2.15; 200 rectangles through one
+// another EXACT 3.1 / 7.7.  Over those scenes the rule's choice takes 1.01 of the better
+// kernel's time; the culled kernel alone 1.3 (EXACT) and 1.4 (FAST).
+bool culled_gains(const rf_ctx *c, const Budget &b)
+{
+    const CullReach &r = c->reach;
+    const int64_t rays = 4 * b.draws;
+    if (c->cfg.precision == RF_PREC_FP64)  // (below 1.5e5 rays the plain kernel's time is one wave's)
+        return r.planar + r.round + r.cones <= c->n * (c->n / 80.0);
+    double tests, plain, limit;
+    if (c->cfg.precision == RF_PREC_FAST) {
+        tests = 33.0 * (r.planar + r.round) + 46.0 * r.cones;
+        plain = 13.0 * r.nplanar + 19.0 * r.ncurved;
+        limit = rays < 2000000 ? 0.25 : (rays < 6000000 ? 0.36 : (rays < 20000000 ? 0.52 : 0.62));
+    } else {
+        tests = 37.0 * r.planar + 40.0 * r.round + 45.0 * r.cones;
+        plain = 15.0 * r.nplanar + 29.0 * r.ncurved;
+        limit = rays < 650000 ? (c->n >= 128 ? 0.35 : 0.15)
+                              : (rays < 2000000 ? 0.35 : (rays < 6000000 ? 0.45 : (rays < 20000000 ? 0.58 : 0.68)));
+    }
+    // rows that fill little of the plain kernel's chunks make it slower
+    if (rays >= 400000) tests *= (double)b.draws / (double)(b.chunks(kBlock) * kBlock);
+    return tests <= limit * plain;
 }
 
 // The narrow kernel (rf_narrow.cuh) takes traces of few rays, unless a launch shape of
@@ -398,7 +444,7 @@ rf_status ensure_culled(rf_ctx *c)
     }
     float4 *q = buf.data() + 4 * n;
     const bool ok = cull_tables(c->prims.data(), c->n, c->bvs.data(), c->nbv, c->cfg.split_stacks == 0, tab, q, q + n,
-                                q + 3 * n, q + 4 * n);
+                                q + 3 * n, q + 4 * n, &c->reach);
     if (ok) {
         RF_CUDA(c, cudaStreamSynchronize(c->stream));
         RF_CUDA(c, c->d_cull.ensure(words * sizeof(float4)));
@@ -419,7 +465,7 @@ Plan make_plan(const rf_ctx *c, bool bv, bool rec, const Budget &b)
 {
     Plan pl;
     pl.split = narrow_split(c, bv, b);
-    if (pl.split == 0 && c->cull > 0 && culled_pays(c, bv, b.draws)) pl.chunk_draws = culled_chunk(c, b.draws);
+    if (pl.split == 0 && c->cull > 0 && culled_pays(c, bv, b)) pl.chunk_draws = culled_chunk(c, b.draws);
     pl.lc.bv = bv;
     pl.lc.rec = rec;
     pl.lc.block = c->block > 0 ? c->block : (c->cfg.block_size > 0 ? c->cfg.block_size : kBlock);
@@ -1496,7 +1542,7 @@ rf_status rf_trace_async(rf_ctx *c, const int64_t *rays, int32_t use_bv)
         return RF_OK;
     }
     const Budget budget(rays, c->n);
-    if (c->cull == 0 && culled_pays(c, use_bv != 0, budget.draws) && (s = ensure_culled(c)) != RF_OK) return s;
+    if (c->cull == 0 && culled_pays(c, use_bv != 0, budget) && (s = ensure_culled(c)) != RF_OK) return s;
     Plan pl = make_plan(c, use_bv != 0, false, budget);
     std::vector<Segment> seg;
     int64_t chunks = 0;
@@ -1530,7 +1576,7 @@ rf_status rf_trace_range(rf_ctx *c, const int64_t *first_ray, const int64_t *cou
     int64_t chunks = 0;
     const bool mixed = c->cfg.precision == RF_PREC_MIXED;
     const Budget budget(count, c->n);
-    if (c->cull == 0 && culled_pays(c, use_bv != 0, budget.draws) && (s = ensure_culled(c)) != RF_OK) return s;
+    if (c->cull == 0 && culled_pays(c, use_bv != 0, budget) && (s = ensure_culled(c)) != RF_OK) return s;
     Plan pl = make_plan(c, use_bv != 0, false, budget);
     const int64_t chunk_gids = mixed ? mixed_chunk_draws(c, false, use_bv != 0, budget) : pl.chunk_gids();
     for (int e = 0; e < c->n; ++e) chunks = plan_segments(seg, e, 0, first_ray[e], count[e], chunk_gids, chunks);
@@ -1662,7 +1708,7 @@ rf_status rf_trace_rays(rf_ctx *c, int32_t emitter, int64_t first_ray, int64_t n
             return s;
     } else {
         const Budget budget(&n_rays, 1);
-        if (c->cull == 0 && culled_pays(c, use_bv != 0, budget.draws) && (s = ensure_culled(c)) != RF_OK) return s;
+        if (c->cull == 0 && culled_pays(c, use_bv != 0, budget) && (s = ensure_culled(c)) != RF_OK) return s;
         Plan pl = make_plan(c, use_bv != 0, true, budget);
         std::vector<Segment> seg;
         const int64_t chunks = plan_segments(seg, emitter, 0, first_ray, n_rays, pl.chunk_gids(), 0);

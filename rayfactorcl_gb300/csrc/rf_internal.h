@@ -150,8 +150,15 @@ cudaError_t launch_mixed_narrow(const TraceParams &p, int split, bool rec, int s
 // stack's later members); quad (2 n), slack (n, ring stacks), bvsph (nbv); a stack's
 // size goes into its first member's tab[].aux.w.
 // False when the bounds leave too little out.  stacks: look for ring stacks.
+//
+// reach: how many of the surfaces a packet of rays is likely to test, by what a test
+// costs (an estimate over 16 emitters), and how many there are.
+struct CullReach {
+    float planar, round, cones;  // tests of planar surfaces, of cylinders and spheres, of frusta
+    int32_t nplanar, ncurved;
+};
 bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs, int nbv, bool stacks, HitRec *tab,
-                 float4 *sph, float4 *quad, float4 *slack, float4 *bvsph);
+                 float4 *sph, float4 *quad, float4 *slack, float4 *bvsph, CullReach *reach);
 
 // Batched mixed-precision persistent kernel (rf_kern_batched.cu); count: also
 // collect the work counters (TraceParams::work); stacks: some scene's tables
