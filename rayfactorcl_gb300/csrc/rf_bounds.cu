@@ -354,12 +354,23 @@ float4 tight_sphere(const rf_primitive &e, float4 box, int rings, float outer2, 
     if (!(r < (double)box.w)) return box;
     // the hits follow invm: where it places the surface elsewhere than m does (half of the
     // check's own widening is allowed for), the box's sphere as well as it can
+    // (at once where invm m differs from 1 by so little that no point of the surface moves far)
+    const double far = 2 * std::max(x.r0, x.r1) + std::max(std::fabs(x.z0), std::fabs(x.z1)) + 1.0;
+    double moved = 0.0;
+    for (int i = 0; i < 3; ++i) {
+        const float *p = e.invm + 4 * i;
+        double off = std::fabs(p[0] * t[0] + p[1] * t[1] + p[2] * t[2] + p[3]);
+        for (int k = 0; k < 3; ++k)
+            off = std::max(off, std::fabs(p[0] * M[k] + p[1] * M[3 + k] + p[2] * M[6 + k] - (i == k ? 1.0 : 0.0)));
+        moved += off * std::sqrt(M[i] * M[i] + M[3 + i] * M[3 + i] + M[6 + i] * M[6 + i]);
+    }
+    const float4 tight = make_float4((float)b.c[0], (float)b.c[1], (float)b.c[2], (float)r);
+    if (moved * far <= 0.002 * r) return tight;
     double Mi[9], ti[3], d[3];
     if (!inverse_of(e.invm, Mi, ti)) return box;
     const Ball h = image_ball(Mi, ti, x);
     for (int k = 0; k < 3; ++k) d[k] = h.c[k] - b.c[k];
-    if (!(std::sqrt(dot(d, d)) + h.r <= 1.005 * r)) return box;
-    return make_float4((float)b.c[0], (float)b.c[1], (float)b.c[2], (float)r);
+    return std::sqrt(dot(d, d)) + h.r <= 1.005 * r ? tight : box;
 }
 
 bool cull_tables(const rf_primitive *prims, int n, const rf_bounding_volume *bvs, int nbv, bool stacks, HitRec *tab,
