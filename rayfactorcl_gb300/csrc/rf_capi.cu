@@ -310,8 +310,8 @@ struct Plan {
 //     5: 0.166 / 0.150, 8: 0.175 / 0.188 -> from 8, or from 3 at 2.5e5 rays;
 //   rays: the sort's fixed cost, EXACT at 1e5 rays  64 surfaces: 0.065 / 0.056, 201: 0.15 / 0.19;
 //     at 3e5 rays 24: 0.044 / 0.040, 64: 0.071 / 0.085, FAST 64: 0.060 / 0.060, at 1e6 rays
-//     0.099 / 0.140 -> from 4e5 rays (FAST 1e6) or 128 surfaces (FAST 256) on (FP64 64
-//     surfaces, 1e5 rays: 0.58 / 1.01);
+//     0.099 / 0.140 -> from 4e5 rays (FAST, and EXACT below 24 surfaces, 1e6) or 128 surfaces
+//     (FAST 256) on (FP64 64 surfaces, 1e5 rays: 0.58 / 1.01);
 //   a few hundred rays per emitter leave most threads of a plain chunk idle: 1e4 rays,
 //     64 surfaces EXACT 0.033 / 0.056, FAST 0.029 / 0.032 (bounding surfaces only: other
 //     traces of so few rays take the narrow kernel).
@@ -350,10 +350,11 @@ bool culled_pays(const rf_ctx *c, bool bv, const Budget &b)
 // are where the two kernels' times met, for 16 to 400 surfaces of five kinds at seven
 // densities (packets that reach all surfaces down to a twentieth): lower for few rays, whose
 // packets are less alike and leave SMs idle.  Plain / culled, ms at 1e7 rays, 64 surfaces
-// of every type with centres in [-s, s]^3:  s = 3 EXACT 1.57 / 0.63, FAST 1.00 / 0.55; s = 1
-// 1.58 / 1.52, 1.01 / 1.30; s = 0.1 1.61 / 2.58, 1.03 / 2.15; 200 rectangles through one
+// of every type with centres in [-s, s]^3:  s = 3 EXACT 1.75 / 0.70, FAST 1.10 / 0.60; s = 1
+// 1.79 / 1.72, 1.14 / 1.46; s = 0.1 1.76 / 2.83, 1.14 / 2.38; 200 rectangles through one
 // another EXACT 3.1 / 7.7.  Over those scenes the rule's choice takes 1.01 of the better
-// kernel's time; the culled kernel alone 1.3 (EXACT) and 1.4 (FAST).
+// kernel's time (geometric mean), the choice by surfaces and rays alone 1.29 (EXACT) and
+// 1.34 (FAST).  FP64 at 1e5 rays, 24 surfaces, s = 3 0.41 / 0.24, s = 0.6 0.41 / 0.57.
 bool culled_gains(const rf_ctx *c, const Budget &b)
 {
     const CullReach &r = c->reach;
@@ -376,6 +377,8 @@ bool culled_gains(const rf_ctx *c, const Budget &b)
     return tests <= limit * plain;
 }
 
+bool mixed_culled(const rf_ctx *c, bool bv);
+
 // The narrow kernel (rf_narrow.cuh) takes traces of few rays, unless a launch shape of
 // another kernel is pinned: how many warps share a ray's surfaces, 0 for the other
 // kernels.  Best split against the kernel that took the trace before, measured, us:
@@ -388,10 +391,13 @@ bool culled_gains(const rf_ctx *c, const Budget &b)
 //   MIXED  12 at 2e5 20 / 26; 32 at 2e5 36 / 39, at 3e5 41 / 39; 64 at 6e4 26 / 45, at 1.5e5
 //     47 / 49; 201 at 6e4 61 / 86, at 1.5e5 127 / 116; rings in stacks at 2e5 47 / 57; 1000 (no
 //     longer in the batched kernel's shared memory) at 2e5 854 / 1339
-//   FP64 (before either kernel kept its matrices in doubles)  3 at 1e4 24 / 94; 12 at 4e4
-//     144 / 251; 32 at 4e4 297 / 359; 64 at 2e4 300 / 318, at 4e4 457 / 524; 100 at 1e4 246 / 214
-bool mixed_culled(const rf_ctx *c, bool bv);
-
+//   FP64 (the culled kernel)  3 at 1e4 23 / 94, at 4e4 46 / 94; 12 at 1e4 42 / 95, at 4e4 117 /
+//     205; 20 at 4e4 164 / 224; 32 at 1e4 75 / 65, at 2e4 131 / 106, at 4e4 177 / 178; 48 at 1e4 102 /
+//     76, at 2e4 184 / 100 (the limit was set when the culled kernel converted its matrices ray
+//     by ray; the plain kernel, which took these before, 244 to 980)
+// Where EXACT and FAST traces have too many rays for this kernel and too few for the culled
+// one (16 to 127 surfaces, 2.2e5 to 4e5 rays; FAST to 255, 1.6e5 to 1e6) the plain kernel has
+// them: 64 surfaces EXACT at 3e5 84, 66 here, 71 culled.
 int narrow_split(const rf_ctx *c, bool bv, const Budget &b)
 {
     const rf_config &f = c->cfg;
@@ -1270,8 +1276,8 @@ rf_status run_small(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_ch
     return RF_OK;
 }
 
-// A MIXED trace of the single scene: small-scene or batched kernel; with its
-// bounding surfaces (runBVGPU semantics), the batched kernel's BV variant.
+// A MIXED trace of the single scene: narrow, small-scene, culled (always so with
+// bounding surfaces and more than a few surfaces) or batched kernel.
 rf_status run_mixed(rf_ctx *c, const std::vector<Segment> &seg, int64_t total_chunks, bool rec, int32_t *d_rec,
                     int64_t rec_base, bool zero_hits, bool bv, int64_t chunk_draws)
 {

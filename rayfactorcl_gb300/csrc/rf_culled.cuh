@@ -410,7 +410,7 @@ __device__ __forceinline__ void plate_hits(const HitRec &h, const HitRec *tab, b
 
 // The mixed-precision arithmetic (emit_mixed, test_mixed with FP64 for an
 // ill-conditioned quadric at once) over the mixed tables; used for scenes with
-// bounding surfaces.
+// bounding surfaces, and for those that are nearly all segment stacks.
 struct MMixed : MFast {};
 template <class M> constexpr bool kIsMixed = false;
 template <> constexpr bool kIsMixed<MMixed> = true;
