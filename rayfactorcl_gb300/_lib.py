@@ -116,11 +116,15 @@ def load() -> ctypes.CDLL:
     return L
 
 
+class _ArrayPtr(ctypes.c_void_p):
+    __slots__ = ("array",)
+
+
 def ptr(a: np.ndarray | None):
     """Address of an array for a call; the pointer keeps the array alive."""
     if a is None:
         return None
-    p = ctypes.c_void_p(a.__array_interface__["data"][0])
+    p = _ArrayPtr(a.__array_interface__["data"][0])
     p.array = a
     return p
 
